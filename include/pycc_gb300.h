@@ -48,6 +48,21 @@ int pcg_contract_f64(int m_n, const long long* m_ext, const long long* m_sa,
                      double alpha, const double* A, const double* B, double beta, double* C,
                      void* stream);
 
+/* The same contraction on the BF16 tensor cores in residue arithmetic (csrc/contract_rns.cu):
+ * operands scaled by row to integers of at least 54 bits, one exact BF16 GEMM per modulus,
+ * the FP64 result rebuilt from the residues.  `work` is device scratch of `work_len` bytes,
+ * 256-byte aligned, not read after the call's kernels; an operand larger than it goes through
+ * in panels.  pcg_contract_rns_f64_work gives the bytes for flat extents M, N, K within
+ * `limit` (0 when no panel fits).  An expired device-side wait makes the outputs NaN. */
+int pcg_contract_rns_f64(int m_n, const long long* m_ext, const long long* m_sa,
+                         const long long* m_sc, int n_n, const long long* n_ext,
+                         const long long* n_sb, const long long* n_sc, int k_n,
+                         const long long* k_ext, const long long* k_sa, const long long* k_sb,
+                         double alpha, const double* A, const double* B, double beta, double* C,
+                         void* work, long long work_len, void* stream);
+int pcg_contract_rns_f64_work(long long M, long long N, long long K, long long limit,
+                              long long* bytes);
+
 /* Sum of up to four FP64 contractions into one output (written once):
  *   C = beta*C + sum_t alpha[t] * A_t[m,k] B_t[n,k]
  * Common M / N extents and C strides (m_ext, m_sc, n_ext, n_sc); per term t the A strides

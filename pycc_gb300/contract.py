@@ -12,6 +12,10 @@ existing tensor and ``alpha``/``beta`` give ``out = beta*out + alpha*contract(..
 """
 from __future__ import annotations
 
+import ctypes as C
+import functools
+import math
+
 import torch
 
 from . import _lib
@@ -117,8 +121,13 @@ def contract_f64(subscripts, a, b, out=None, alpha=1.0, beta=0.0, stream=None):
             raise ValueError("contract: out has shape %s, expected %s" % (tuple(out.shape), plan.shape))
     M, N, K, batch, ast, bst, cst = plan.groups(a, b, out)
     st = _lib.stream_handle(stream)
+    work = None
+    if out.is_cuda:
+        m, n, k = (math.prod([g[0] for g in G]) for G in (M, N, K))
+        if _takes_rns(m, n, k):
+            work = _rns_scratch(m, n, k, out.device, stream)
     if not batch:
-        _launch(M, N, K, alpha, a.data_ptr(), b.data_ptr(), beta, out.data_ptr(), st)
+        _launch(M, N, K, alpha, a.data_ptr(), b.data_ptr(), beta, out.data_ptr(), st, work)
         return out
     # batch indices (present in both operands and the output): one launch per value
     import itertools
@@ -128,17 +137,66 @@ def contract_f64(subscripts, a, b, out=None, alpha=1.0, beta=0.0, stream=None):
         ob = sum(v * bst[c] for v, c in zip(vals, batch)) * 8
         oc = sum(v * cst[c] for v, c in zip(vals, batch)) * 8
         _launch(M, N, K, alpha, a.data_ptr() + oa, b.data_ptr() + ob, beta,
-                out.data_ptr() + oc, st)
+                out.data_ptr() + oc, st, work)
     return out
 
 
-def _launch(M, N, K, alpha, pa, pb, beta, pc, st):
+def _launch(M, N, K, alpha, pa, pb, beta, pc, st, work=None):
     i64 = _lib.i64s
-    _lib.call("pcg_contract_f64",
-              len(M), i64([g[0] for g in M]), i64([g[1] for g in M]), i64([g[2] for g in M]),
-              len(N), i64([g[0] for g in N]), i64([g[1] for g in N]), i64([g[2] for g in N]),
-              len(K), i64([g[0] for g in K]), i64([g[1] for g in K]), i64([g[2] for g in K]),
-              float(alpha), pa, pb, float(beta), pc, st)
+    args = (len(M), i64([g[0] for g in M]), i64([g[1] for g in M]), i64([g[2] for g in M]),
+            len(N), i64([g[0] for g in N]), i64([g[1] for g in N]), i64([g[2] for g in N]),
+            len(K), i64([g[0] for g in K]), i64([g[1] for g in K]), i64([g[2] for g in K]),
+            float(alpha), pa, pb, float(beta), pc)
+    if work is None:
+        _lib.call("pcg_contract_f64", *args, st)
+    else:
+        _lib.call("pcg_contract_rns_f64", *args, work.data_ptr(), work.numel(), st)
+
+
+RNS_WORK_LIMIT = 8 << 30     # bytes of scratch of one contraction in residue arithmetic
+
+
+@functools.lru_cache(maxsize=4096)
+def _rns_work(m, n, k, limit=RNS_WORK_LIMIT):
+    """Scratch bytes of an m x n x k contraction in residue arithmetic (0: does not fit)."""
+    out = C.c_longlong(0)
+    _lib.call("pcg_contract_rns_f64_work", m, n, k, limit, C.byref(out))
+    return out.value
+
+
+@functools.lru_cache(maxsize=4096)
+def _takes_rns(m, n, k):
+    """Whether an m x n x k contraction runs on the tensor cores in residue arithmetic rather
+    than on the FP64 pipe: where its estimated time is the shorter one.
+
+    FP64 pipe: 1.15 TFLOP/s over whole 64 x 64 tiles.  Residues: 80 us of launches, 48 bytes
+    moved per operand element at 5 TB/s, 16 BF16 products over whole 128 x 16 tiles at
+    1.1 PFLOP/s and 13 ps per output to rebuild it."""
+    if min(m, n) < 2 or m * n * k < 1 << 22:
+        return False
+    fp64 = 2.0 * -(-m // 64) * 64 * -(-n // 64) * 64 * k / 1.15e12
+    lo, hi = (m, n) if m < n else (n, m)
+    rns = (80e-6 + 48.0 * (m + n) * k / 5e12 + 32.0 * -(-lo // 128) * 128 * hi * k / 1.1e15
+           + 13e-12 * m * n)
+    return rns < fp64
+
+
+def _rns_scratch(m, n, k, device, stream):
+    """Scratch for the call on ``device``, owned by the launching stream, or None when the
+    device has no room even for small panels (the FP64 kernel needs none)."""
+    limit = RNS_WORK_LIMIT
+    while limit >= 256 << 20:
+        nbytes = _rns_work(m, n, k, limit)
+        if not nbytes:
+            return None
+        try:
+            if stream is None:
+                return torch.empty(nbytes, dtype=torch.uint8, device=device)
+            with torch.cuda.stream(stream):
+                return torch.empty(nbytes, dtype=torch.uint8, device=device)
+        except torch.cuda.OutOfMemoryError:
+            limit = min(limit, nbytes) // 4
+    return None
 
 
 class ContractionBackend:
