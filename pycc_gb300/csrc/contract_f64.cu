@@ -23,7 +23,7 @@ struct F64Args {
   const double* A;
   const double* B;
   double* C;
-  int a_kfast, b_kfast, atomic_out;
+  int atomic_out;
 };
 
 __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
@@ -32,121 +32,132 @@ __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
                : "d"(a), "d"(b));
 }
 
-__global__ void __launch_bounds__(NT) contract_f64_kernel(const F64Args p) {
-  __shared__ double As[BK][BM + 2];
-  __shared__ double Bs[BK][BN + 2];
-  __shared__ long long aoff[BM], coffm[BM], boff[BN], coffn[BN];
-  __shared__ long long akoff[BK], bkoff[BK];
-
-  const int tid = threadIdx.x;
-  const long long m0 = (long long)blockIdx.y * BM;
-  const long long n0 = (long long)blockIdx.x * BN;
-  const long long kbeg = (long long)blockIdx.z * p.k_per_split;
-  const long long kend = min(p.K, kbeg + p.k_per_split);
-
-  if (tid < BM) {
-    long long r = m0 + tid, o0 = 0, o1 = 0;
-    if (r < p.M) sub_offsets(p.m, r, o0, o1);
-    aoff[tid] = o0;
-    coffm[tid] = o1;
-  } else {
-    int t = tid - BM;
-    long long r = n0 + t, o0 = 0, o1 = 0;
-    if (r < p.N) sub_offsets(p.n, r, o0, o1);
-    boff[t] = o0;
-    coffn[t] = o1;
+// Offsets of flat index r in both tensors; I is the type of the index arithmetic (32-bit
+// division where the totals allow it, a third of the 64-bit sequence).
+template <typename I>
+__device__ __forceinline__ void sub_offsets_as(const SubIdx& d, I r, long long& o0,
+                                               long long& o1) {
+  o0 = 0;
+  o1 = 0;
+  for (int q = d.n - 1; q >= 0; --q) {
+    const I e = (I)d.ext[q];
+    const long long x = (long long)(r % e);
+    r /= e;
+    o0 += x * d.s0[q];
+    o1 += x * d.s1[q];
   }
+}
 
-  const int warp = tid >> 5, lane = tid & 31;
-  const int wm = warp >> 1, wn = warp & 1;
+// A warp computes 8 FM x 8 FN outputs over a slice of K, its DMMA fragments read straight from
+// global memory (L1 holds the rows; the 8 x 4 fragment of a lane pattern is whole sectors
+// whichever index is unit-stride).  A quarter of an SM's FP64 pipe takes about 512 clocks for one
+// m8n8k4, so loads cost little next to it; what bounds a small product is how evenly the
+// multiply-adds spread over the 608 quarters.  Blocks of 64 x 64 tiles left most of them idle.
+// Here kw of the block's 8 warps share an output tile and split K, blocks split K further (FP64
+// atomics), and a tile is 16 x 16, 8 x 32 or 32 x 8 where one side has at most 8 entries, or
+// 8 x 8 where there would be fewer 16-K steps than would keep every quarter busy.
+// Device time against 64 x 64 tiles in shared memory, us: no = 5, nv = 19 ring 138 -> 11, small
+// products 45-60 -> 6-8; no = 9, nv = 53 'nb,mnej->mbej' 41 -> 15, 'mief,maef->ia' 490 -> 59; the
+// large ladder of no = 20, nv = 180 882 -> 770 ms (1.09 TFLOP/s).
+template <int FM, int FN, typename I>
+__global__ void __launch_bounds__(256) contract_f64_kernel(const F64Args p, int kw,
+                                                           long long tiles_n, long long tiles) {
+  constexpr int NF = 2 * FM * FN;
+  __shared__ double red[8][NF][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t4 = lane & 3;
-  double acc[4][4][2];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  const int ks = warp % kw;
+  const long long tile = (long long)blockIdx.x * (8 / kw) + warp / kw;
+  const bool live = tile < tiles;
+  const long long m0 = (live ? tile / tiles_n : 0) * (8 * FM);
+  const long long n0 = (live ? tile % tiles_n : 0) * (8 * FN);
+  const long long kbeg = (long long)blockIdx.y * p.k_per_split;
+  const long long kend = live ? min(p.K, kbeg + p.k_per_split) : 0;
 
-  double ra[8], rb[8];
-  auto kofs = [&](long long kt) {
-    if (tid < BK) {
-      long long r = kt + tid, o0 = 0, o1 = 0;
-      if (r < kend) sub_offsets(p.k, r, o0, o1);
-      akoff[tid] = o0;
-      bkoff[tid] = o1;
-    }
-  };
-  auto load = [&](long long kt) {
+  long long ao[FM], bo[FN], cm[FM];
+  bool aok[FM], bok[FN];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      int e = tid + NT * i;
-      int mm, kk;
-      if (p.a_kfast) { kk = e % BK; mm = e / BK; } else { mm = e % BM; kk = e / BM; }
-      bool ok = (m0 + mm < p.M) && (kt + kk < kend);
-      ra[i] = ok ? __ldg(p.A + aoff[mm] + akoff[kk]) : 0.0;
-      int nn;
-      if (p.b_kfast) { kk = e % BK; nn = e / BK; } else { nn = e % BN; kk = e / BN; }
-      ok = (n0 + nn < p.N) && (kt + kk < kend);
-      rb[i] = ok ? __ldg(p.B + boff[nn] + bkoff[kk]) : 0.0;
-    }
-  };
-  auto store = [&]() {
+  for (int i = 0; i < FM; ++i) {
+    const long long r = m0 + 8 * i + g;
+    aok[i] = r < p.M;
+    ao[i] = cm[i] = 0;
+    if (aok[i]) sub_offsets_as<I>(p.m, (I)r, ao[i], cm[i]);
+  }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      int e = tid + NT * i;
-      int mm, kk;
-      if (p.a_kfast) { kk = e % BK; mm = e / BK; } else { mm = e % BM; kk = e / BM; }
-      As[kk][mm] = ra[i];
-      int nn;
-      if (p.b_kfast) { kk = e % BK; nn = e / BK; } else { nn = e % BN; kk = e / BN; }
-      Bs[kk][nn] = rb[i];
-    }
-  };
+  for (int j = 0; j < FN; ++j) {
+    const long long r = n0 + 8 * j + g;
+    long long unused;
+    bok[j] = r < p.N;
+    bo[j] = 0;
+    if (bok[j]) sub_offsets_as<I>(p.n, (I)r, bo[j], unused);
+  }
+  double acc[FM][FN][2];
+#pragma unroll
+  for (int i = 0; i < FM; ++i)
+#pragma unroll
+    for (int j = 0; j < FN; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
 
-  kofs(kbeg);
-  __syncthreads();
-  if (kbeg < kend) load(kbeg);
-  for (long long kt = kbeg; kt < kend; kt += BK) {
-    __syncthreads();  // previous compute done with As/Bs and akoff
-    store();
-    if (kt + BK < kend) kofs(kt + BK);
-    __syncthreads();
-    if (kt + BK < kend) load(kt + BK);  // global loads overlap the DMMAs below
+  for (long long k0 = kbeg + 16 * ks; k0 < kend; k0 += 16 * kw) {
+    double a[4][FM], b[4][FN];
 #pragma unroll
-    for (int ks = 0; ks < BK; ks += 4) {
-      double a[4], b[4];
+    for (int s = 0; s < 4; ++s) {
+      const long long k = k0 + 4 * s + t4;
+      const bool ok = k < kend;
+      long long ka = 0, kb = 0;
+      if (ok) sub_offsets_as<I>(p.k, (I)k, ka, kb);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[ks + t4][wm * 32 + i * 8 + g];
+      for (int i = 0; i < FM; ++i) a[s][i] = (ok && aok[i]) ? __ldg(p.A + ao[i] + ka) : 0.0;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[ks + t4][wn * 32 + j * 8 + g];
+      for (int j = 0; j < FN; ++j) b[s][j] = (ok && bok[j]) ? __ldg(p.B + bo[j] + kb) : 0.0;
+    }
+    if (k0 + 12 < kend) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int s = 0; s < 4; ++s)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) dmma(acc[i][j], a[i], b[j]);
+        for (int i = 0; i < FM; ++i)
+#pragma unroll
+          for (int j = 0; j < FN; ++j) dmma(acc[i][j], a[s][i], b[s][j]);
+    } else {  // the last step multiplies the K it has
+#pragma unroll
+      for (int s = 0; s < 3; ++s)
+        if (k0 + 4 * s < kend)
+#pragma unroll
+          for (int i = 0; i < FM; ++i)
+#pragma unroll
+            for (int j = 0; j < FN; ++j) dmma(acc[i][j], a[s][i], b[s][j]);
     }
   }
 
+  if (kw > 1) {  // the K slices of a tile add up in its first warp
+    if (ks > 0)
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    int row = wm * 32 + i * 8 + g;
-    if (m0 + row >= p.M) continue;
+      for (int f = 0; f < NF; ++f) red[warp][f][lane] = acc[f / (2 * FN)][(f / 2) % FN][f % 2];
+    __syncthreads();
+    if (ks > 0) return;
+    for (int w = warp + 1; w < warp + kw; ++w)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+      for (int f = 0; f < NF; ++f) acc[f / (2 * FN)][(f / 2) % FN][f % 2] += red[w][f][lane];
+  }
+  if (!live) return;
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        int col = wn * 32 + j * 8 + 2 * t4 + h;
-        if (n0 + col >= p.N) continue;
-        double* dst = p.C + coffm[row] + coffn[col];
-        double v = p.alpha * acc[i][j][h];
-        if (p.atomic_out) {
+  for (int j = 0; j < FN; ++j)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const long long c = n0 + 8 * j + 2 * t4 + h;
+      if (c >= p.N) continue;
+      long long unused, cn;
+      sub_offsets_as<I>(p.n, (I)c, unused, cn);
+#pragma unroll
+      for (int i = 0; i < FM; ++i) {
+        if (!aok[i]) continue;
+        double* dst = p.C + cm[i] + cn;
+        const double v = p.alpha * acc[i][j][h];
+        if (p.atomic_out)
           atomicAdd(dst, v);
-        } else if (p.beta == 0.0) {
-          *dst = v;
-        } else {
-          *dst = p.beta * *dst + v;
-        }
+        else
+          *dst = p.beta == 0.0 ? v : p.beta * *dst + v;
       }
     }
-  }
 }
 
 // C[m, n] *= beta over the strided M x N range (used before a split-K accumulation).
@@ -234,7 +245,9 @@ __global__ void __launch_bounds__(256) contract_gemv_thread_kernel(const F64Args
 }
 
 // K slices for a matrix-vector launch of `blocks` output blocks: enough blocks for about
-// eight per SM, each slice at least `kmin` long; beta is applied up front when split.
+// eight per SM, each slice at least `kmin` long; beta is applied up front when split.  kmin is
+// 64 for a thread per output (with 1024, 'mf,mafe->ae' at no = 9, nv = 53 ran 11 blocks for
+// 79 us; 11 us now) and 512 for a warp.
 long long gemv_splits(const F64Args& p, long long blocks, long long kmin);
 
 // Reorder sub-indices by decreasing |stride| in the operand (s0), unit stride innermost.
@@ -321,9 +334,6 @@ extern "C" int pcg_contract_f64(int m_n, const long long* m_ext, const long long
   p.A = A;
   p.B = B;
   p.C = C;
-  // Load the operand tile along whichever index is unit-stride in memory.
-  p.a_kfast = (p.k.s0[p.k.n - 1] == 1) ? 1 : 0;
-  p.b_kfast = (p.k.s1[p.k.n - 1] == 1) ? 1 : 0;
   cudaStream_t st = (cudaStream_t)stream;
   if (p.M == 1 || p.N == 1) {
     // one free side: enumerate the outputs along the big operand's unit-stride index
@@ -339,7 +349,7 @@ extern "C" int pcg_contract_f64(int m_n, const long long* m_ext, const long long
     }
     if (q.n.s0[q.n.n - 1] == 1 && q.M * q.N >= 1024) {
       const long long blocks = (q.M * q.N + 255) / 256;
-      const long long splits = gemv_splits(q, blocks, 1024);
+      const long long splits = gemv_splits(q, blocks, 64);
       q.k_per_split = (q.K + splits - 1) / splits;
       q.atomic_out = splits > 1;
       if (q.atomic_out && beta != 1.0) {
@@ -352,10 +362,10 @@ extern "C" int pcg_contract_f64(int m_n, const long long* m_ext, const long long
       return 0;
     }
   }
-  if (p.M < 8 || p.N < 8) {
+  if (p.M == 1 || p.N == 1) {
     long long warps = p.M * p.N;
     int blocks = (int)std::min<long long>((warps * 32 + 255) / 256, 152LL * 64);
-    const long long splits = gemv_splits(p, blocks, 4096);
+    const long long splits = gemv_splits(p, blocks, 512);
     p.k_per_split = (p.K + splits - 1) / splits;
     p.atomic_out = splits > 1;
     if (p.atomic_out && beta != 1.0) {
@@ -367,34 +377,47 @@ extern "C" int pcg_contract_f64(int m_n, const long long* m_ext, const long long
     PCG_CHECK_LAUNCH("pcg_contract_f64/gemv");
     return 0;
   }
-  long long mt = (p.M + BM - 1) / BM, nt = (p.N + BN - 1) / BN;
-  if (mt > 65535) {
-    set_error("pcg_contract_f64: M=%lld too large", p.M);
-    return -1;
-  }
-  long long tiles = mt * nt;
-  long long target = 2LL * num_sms();
+  // tiles of 16 x 16 outputs per warp, 8 x 32 or 32 x 8 where a side has at most 8, 8 x 8 where
+  // 16 x 16 tiles would leave fewer than two K steps for each quarter of an SM
+  const long long steps = (p.K + 15) / 16;
+  int fm = p.M <= 8 ? 1 : (p.N <= 8 ? 4 : 2), fn = 4 / fm;
+  if ((p.M + 15) / 16 * ((p.N + 15) / 16) * steps < 8LL * num_sms()) fm = fn = 1;
+  const long long nt = (p.N + 8 * fn - 1) / (8 * fn), mt = (p.M + 8 * fm - 1) / (8 * fm);
+  const long long tiles = mt * nt;
+  // warps per tile: K's 16-wide steps over up to 8 warps while that fills the chip (16 warps on
+  // each SM), then over blocks, each at least two steps a warp
+  const long long want = 16LL * num_sms();
+  int kw = 1;
+  while (kw < 8 && 2 * kw <= steps && tiles * kw < want) kw *= 2;
   long long splits = 1;
-  if (tiles < target && p.K >= 8 * BK) {
-    splits = (target + tiles - 1) / tiles;
-    long long maxs = p.K / (4 * BK);
-    if (splits > maxs) splits = maxs;
-    if (splits > 64) splits = 64;
-    if (splits < 1) splits = 1;
-  }
-  long long kps = (p.K + splits - 1) / splits;
-  kps = ((kps + BK - 1) / BK) * BK;
+  if (kw == 8 && tiles * 8 < want)
+    splits = std::max(1LL, std::min((want + tiles * 8 - 1) / (tiles * 8), steps / 16));
+  long long kps = ((p.K + splits - 1) / splits + 15) / 16 * 16;
   splits = (p.K + kps - 1) / kps;
   p.k_per_split = kps;
   p.atomic_out = splits > 1;
+  const long long blocks = (tiles + 8 / kw - 1) / (8 / kw);
+  if (blocks > 0x7fffffffLL) {
+    set_error("pcg_contract_f64: M=%lld x N=%lld too large", p.M, p.N);
+    return -1;
+  }
   if (p.atomic_out && beta != 1.0) {
-    long long total = p.M * p.N;
-    int blocks = (int)std::min<long long>((total + 255) / 256, 4096);
-    scale_strided_kernel<<<blocks, 256, 0, st>>>(p.m, p.n, p.M, p.N, beta, C);
+    const long long total = p.M * p.N;
+    scale_strided_kernel<<<(int)std::min<long long>((total + 255) / 256, 4096), 256, 0, st>>>(
+        p.m, p.n, p.M, p.N, beta, C);
     PCG_CHECK_LAUNCH("pcg_contract_f64/scale");
   }
-  dim3 grid((unsigned)nt, (unsigned)mt, (unsigned)splits);
-  contract_f64_kernel<<<grid, NT, 0, st>>>(p);
+  const dim3 grid((unsigned)blocks, (unsigned)splits);
+  const bool wide = p.M > 0x7fffffffLL || p.N > 0x7fffffffLL || p.K > 0x7fffffffLL;
+  auto go = [&](auto kernel) { kernel<<<grid, 256, 0, st>>>(p, kw, nt, tiles); };
+  if (fm == 1 && fn == 1)
+    wide ? go(contract_f64_kernel<1, 1, unsigned long long>) : go(contract_f64_kernel<1, 1, unsigned>);
+  else if (fm == 1)
+    wide ? go(contract_f64_kernel<1, 4, unsigned long long>) : go(contract_f64_kernel<1, 4, unsigned>);
+  else if (fm == 2)
+    wide ? go(contract_f64_kernel<2, 2, unsigned long long>) : go(contract_f64_kernel<2, 2, unsigned>);
+  else
+    wide ? go(contract_f64_kernel<4, 1, unsigned long long>) : go(contract_f64_kernel<4, 1, unsigned>);
   PCG_CHECK_LAUNCH("pcg_contract_f64");
   return 0;
 }
