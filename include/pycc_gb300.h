@@ -63,6 +63,19 @@ int pcg_contract_rns_f64(int m_n, const long long* m_ext, const long long* m_sa,
 int pcg_contract_rns_f64_work(long long M, long long N, long long K, long long limit,
                               long long* bytes);
 
+/* The connected triples t3c_ijk (pycc/cctriples.py:27-72) of batches of triples, FP64 in residue
+ * arithmetic (csrc/triples_rns.cu).  pcg_t3_rns_work: workspace bytes for batches of up to
+ * `batch` triples (0: sizes out of range).  pcg_t3_rns_pack: residues of V = <pq|ex> ([v][v][v][o]),
+ * O = <mp|xy> ([o][v][o][o]) and t2 ([o][o][v][v]), all contiguous FP64, into `work` (256-byte
+ * aligned).  pcg_t3_rns_partials: for the ntrip triples ijk (device int [ntrip][3]) the partial
+ * tensors of the three orientations, P[triple][orientation][z][x][y], as pcg_triples_energy reads
+ * them.  An Inf or NaN in an operand, or an expired device-side wait, makes them NaN. */
+int pcg_t3_rns_work(long long no, long long nv, int batch, long long* bytes);
+int pcg_t3_rns_pack(const double* V, const double* O, const double* t2, long long no, long long nv,
+                    void* work, long long work_len, void* stream);
+int pcg_t3_rns_partials(long long no, long long nv, const int* ijk, int ntrip, double* P, void* work,
+                        long long work_len, void* stream);
+
 /* Sum of up to four FP64 contractions into one output (written once):
  *   C = beta*C + sum_t alpha[t] * A_t[m,k] B_t[n,k]
  * Common M / N extents and C strides (m_ext, m_sc, n_ext, n_sc); per term t the A strides

@@ -1,0 +1,802 @@
+// FP64 products on the BF16 tensor cores in residue arithmetic: what contract_rns.cu (pairwise
+// contractions) and triples_rns.cu (the connected triples) share -- operands to residues, the
+// GEMM over residues, residues to FP64.  contract_rns.cu describes the method.
+#pragma once
+#include "tc_common.cuh"
+#include <cuda_bf16.h>
+#include <algorithm>
+#include <cmath>
+
+namespace pcg {
+namespace rns {
+
+using namespace pcg::tc;
+
+// Sixteen pairwise coprime moduli whose nearest residues fit a signed byte (255 would reach
+// +128).  The rounding of the scaled integers, relative to the sum, grows with sqrt(K) and with
+// the spread of a row's magnitudes; measured against 113-bit sums, 15 moduli (2^-58.5 |a| |b|)
+// fall behind the FP64 kernel at K = 50000 with magnitudes spread over e^+-4 (8.7e-16 against
+// 5.8e-16 of the sums' norm), 16 stay ahead of it everywhere.
+constexpr int NM = 16;
+constexpr int kModuli[NM] = {256, 253, 251, 247, 241, 239, 233, 229,
+                             227, 223, 217, 211, 199, 197, 193, 191};
+constexpr int kBits2 = 123;         // |a'|^2 |b'|^2 <= 2^(2 * 123.75); log2(product / 2) = 123.95
+// first bit of the four digits of a scaled integer (16, 15, 15 and 16 bits): with residues of
+// the powers of at most 127, a digit sum stays below 2^16 + 127 * 2^17 < 2^24, exact in FP32
+__host__ __device__ constexpr int digit_bit(int q) { return q == 0 ? 0 : (q == 4 ? 62 : 1 + 15 * q); }
+constexpr int kChunk = 15;          // 64-K blocks per exact FP32 accumulation: 960 K
+constexpr float kMagic = 12582912.f;  // 1.5 * 2^23: adding it rounds to an integer
+
+// Per modulus: p, 1/p and the residues of 2^16, 2^31, 2^46 (symmetric).
+struct ModTab {
+  float p[NM], inv[NM], c1[NM], c2[NM], c3[NM];
+};
+// Per modulus floor(2^96 q / p), q = ((P / p)^-1 mod p), in three 32-bit words; b: what the
+// bias of the stored bytes adds, negated; scale = P 2^-96.
+struct CrtTab {
+  unsigned c0[NM], c1[NM], c2[NM], b0, b1, b2;
+  double scale;
+};
+static_assert(NM * 8 <= 128, "the product fits a 128-bit integer");
+
+// Nearest residue of an integer-valued t, |t| < 2^24: FP32's 1/p is off by at most 2^-24.4
+// relative, so the quotient is off its nearest integer by less than 0.5 + 0.0027 and |r| <= 127
+// (128 for p = 256).
+__device__ __forceinline__ float mod_near(float t, float p, float inv) {
+  const float q = fmaf(t, inv, kMagic) - kMagic;
+  return fmaf(-p, q, t);
+}
+
+// Four residues as bytes r + 128 (modulo 256).
+__device__ __forceinline__ unsigned residue_bytes(float a, float b, float c, float d) {
+  constexpr float bias = 8388608.f + 128.f;
+  return __byte_perm(
+      __byte_perm(__float_as_uint(a + bias), __float_as_uint(b + bias), 0x0040),
+      __byte_perm(__float_as_uint(c + bias), __float_as_uint(d + bias), 0x0040), 0x5410);
+}
+
+struct Operand {
+  const double* X;
+  SubIdx r;             // rows: s0 = strides in X, s1 = strides in C
+  long long R;          // rows
+  long long* off;       // [R] element offset of each row in X
+  long long* coff;      // [R] element offset of each row (or column) in C
+  int* walk;            // [R] rows in an order whose neighbours are close in X
+  unsigned* top;        // [R] biased exponent of the row's largest |x| (2047: Inf or NaN)
+  float* norm2;         // [R] sum of the row's squares, each term truncated to 20 bits
+  const int* shift;     // one power of two for all rows, or null: each row its own
+  const long long* k;   // [K] element offset of each K index in X
+  long long kstep;      // > 0: k[i] = i * kstep
+  int wq;               // sub-index that the walk has innermost
+  int kfast;            // gathered along K (otherwise along the rows)
+};
+
+struct TableArgs {
+  Operand a, b;
+  SubIdx k;
+  long long K;
+  long long *ka, *kb;
+  int* status;
+};
+
+__device__ __forceinline__ void fill_row(const Operand& o, long long r) {
+  long long o0, o1;
+  sub_offsets(o.r, r, o0, o1);
+  o.off[r] = o0;
+  if (o.coff) o.coff[r] = o1;
+  // r as a position of the walk: the same sub-indices with wq moved innermost
+  const int n = o.r.n;
+  long long x[kMaxSub], rr = r;
+  x[o.wq] = rr % o.r.ext[o.wq];
+  rr /= o.r.ext[o.wq];
+  for (int q = n - 1; q >= 0; --q) {
+    if (q == o.wq) continue;
+    x[q] = rr % o.r.ext[q];
+    rr /= o.r.ext[q];
+  }
+  long long row = 0;
+  for (int q = 0; q < n; ++q) row = row * o.r.ext[q] + x[q];
+  o.walk[r] = (int)row;
+}
+
+static __global__ void rns_tables_kernel(const TableArgs t) {
+  const long long total = t.a.R + t.b.R + t.K;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
+       i += (long long)gridDim.x * blockDim.x) {
+    if (i == 0 && t.status) *t.status = 0;
+    if (i < t.a.R) {
+      fill_row(t.a, i);
+      t.a.top[i] = 0;
+      t.a.norm2[i] = 0.f;
+    } else if (i < t.a.R + t.b.R) {
+      fill_row(t.b, i - t.a.R);
+      t.b.top[i - t.a.R] = 0;
+      t.b.norm2[i - t.a.R] = 0.f;
+    } else if (t.ka) {
+      const long long k = i - t.a.R - t.b.R;
+      long long ka, kb;
+      sub_offsets(t.k, k, ka, kb);
+      t.ka[k] = ka;
+      t.kb[k] = kb;
+    }
+  }
+}
+
+__device__ __forceinline__ long long k_offset(const Operand& o, long long k) {
+  return o.kstep > 0 ? k * o.kstep : o.k[k];
+}
+
+// |x| as FP32 from the upper word of a double (20 mantissa bits, truncated); below FP32's
+// range 0, above it infinity.
+__device__ __forceinline__ float abs_hi_f32(unsigned h) {
+  h &= 0x7fffffffu;
+  if (h < (897u << 20)) return 0.f;
+  return h < (1151u << 20) ? __uint_as_float((h - (896u << 20)) << 3)
+                           : __uint_as_float(0x7f800000u);
+}
+
+// Largest exponent and sum of squares of each row over K indices [k0, k1): one read of the
+// operand, bound by HBM.  Gathered along K (KF: a warp per row) or along the rows (a thread
+// per row), eight loads in flight per lane; blockIdx.y cuts K.
+template <bool KF>
+__device__ __forceinline__ void norm_rows(const Operand& o, long long k0, long long k1,
+                                          long long seg, long long bx, long long by) {
+  const long long kb = k0 + by * seg, ke = min(k1, kb + seg);
+  const int lane = threadIdx.x & 31;
+  const long long w = KF ? bx * 8 + (threadIdx.x >> 5) : bx * 256 + threadIdx.x;
+  if (w >= o.R) return;
+  constexpr int STEP = KF ? 32 : 1;
+  const int row = o.walk[w];
+  const double* x = o.X + o.off[row];
+  unsigned m = 0;
+  float s = 0.f;
+  long long k = kb + (KF ? lane : 0);
+  for (; k + 7 * STEP < ke; k += 8 * STEP) {
+    unsigned h[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      h[u] = (unsigned)__double2hiint(__ldg(x + k_offset(o, k + STEP * u)));
+    float t = 0.f;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const float f = abs_hi_f32(h[u]);
+      m = max(m, h[u] & 0x7fffffffu);
+      t = fmaf(f, f, t);
+    }
+    s += t;
+  }
+  for (; k < ke; k += STEP) {
+    const unsigned h = (unsigned)__double2hiint(__ldg(x + k_offset(o, k)));
+    const float f = abs_hi_f32(h);
+    m = max(m, h & 0x7fffffffu);
+    s = fmaf(f, f, s);
+  }
+  if (KF) {
+    for (int d = 16; d > 0; d >>= 1) {
+      m = max(m, __shfl_xor_sync(0xffffffffu, m, d));
+      s += __shfl_xor_sync(0xffffffffu, s, d);
+    }
+    if (lane != 0) return;
+  }
+  atomicMax(o.top + row, m >> 20);
+  atomicAdd(o.norm2 + row, s);
+}
+
+struct NormArgs {
+  Operand o[2];
+  long long gx[2], blocks[2], seg[2];  // row blocks, blocks and K segment of each operand
+  long long k0, k1;
+};
+
+// Both operands in one launch: the first blocks take A, the others B.
+static __global__ void __launch_bounds__(256) rns_norm_kernel(const __grid_constant__ NormArgs p) {
+  const int side = blockIdx.x >= p.blocks[0];
+  const long long b = (long long)blockIdx.x - (side ? p.blocks[0] : 0);
+  const long long bx = b % p.gx[side], by = b / p.gx[side];
+  if (p.o[side].kfast)
+    norm_rows<true>(p.o[side], p.k0, p.k1, p.seg[side], bx, by);
+  else
+    norm_rows<false>(p.o[side], p.k0, p.k1, p.seg[side], bx, by);
+}
+
+// Power of two s of a row: |x| 2^s has a 2-norm of at most 2^61.9.  From the sum of squares
+// where FP32 holds it (1 + 2^-7 covers its truncation and summation), else from the largest
+// element and K.  A zero row may take any.
+__device__ __forceinline__ int row_shift(const Operand& o, long long row, int log2k) {
+  if (o.shift) return *o.shift;
+  const float n2 = o.norm2[row] * 1.0078125f;
+  if (n2 >= 0x1p-80f && n2 <= 0x1p100f) {
+    const unsigned u = __float_as_uint(n2);
+    const int e = (int)(u >> 23) - 127;
+    // log2 n2 <= e + 0.75 or e + 1.75
+    return ((u & 0x7fffffu) < 0x570000u ? kBits2 - e : kBits2 - 1 - e) >> 1;
+  }
+  return (kBits2 - log2k - 2 * (max((int)o.top[row], 1) - 1022)) >> 1;
+}
+
+// The four digits (with the sign) of x 2^s rounded to an integer of at most 62 bits.
+__device__ __forceinline__ void digits(double x, int s, unsigned flip, float (&d)[4]) {
+  const unsigned hi = (unsigned)__double2hiint(x) ^ flip, lo = (unsigned)__double2loint(x);
+  int ex = (int)((hi >> 20) & 0x7ffu);
+  unsigned long long m = ((unsigned long long)(hi & 0xfffffu) << 32) | lo;
+  if (ex)
+    m |= 1ull << 52;
+  else
+    ex = 1;
+  const int sh = ex - 1075 + s;  // at most 9, since |x| 2^s <= 2^61.9
+  if (ex == 2047)
+    m = 0;  // the row's outputs come from the FP64 dot product
+  else if (sh >= 0)
+    m <<= sh;
+  else if (sh > -55)
+    m = (m + (1ull << (-sh - 1))) >> -sh;
+  else
+    m = 0;
+  const unsigned sign = hi & 0x80000000u;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const unsigned v = (unsigned)(m >> digit_bit(q)) & ((1u << (digit_bit(q + 1) - digit_bit(q))) - 1);
+    d[q] = __uint_as_float(__float_as_uint(__uint_as_float(0x4b000000u | v) - 8388608.f) ^ sign);
+  }
+}
+
+struct PackSide {
+  Operand o;
+  long long w0, nrow;  // rows of this panel: walk positions [w0, w0 + nrow); nrow 0: none
+  __nv_bfloat16* out;  // [modulus][nrow][Kp]
+  unsigned flip;       // 0x80000000: the negated operand
+  long long blocks;
+};
+
+struct PackArgs {
+  PackSide s[2];
+  long long k0, K, Kp;  // K indices [k0, k0 + K), padded with zeros to Kp
+  int log2k;            // ceil(log2 K)
+  ModTab t;
+};
+
+// Residues of two neighbouring K entries for every modulus, one 32-bit store per modulus: an
+// integer of at most 8 bits is exact in the upper half of its FP32 word, which is BF16.
+__device__ __forceinline__ void store_residues(const PackArgs& p, const PackSide& o, double x0,
+                                               double x1, int s, long long at) {
+  float a[4], b[4];
+  digits(x0, s, o.flip, a);
+  digits(x1, s, o.flip, b);
+  unsigned* out = reinterpret_cast<unsigned*>(o.out + at);
+  const long long plane = (o.nrow * p.Kp) >> 1;
+#pragma unroll
+  for (int l = 0; l < NM; ++l) {
+    const float t0 = fmaf(a[3], p.t.c3[l], fmaf(a[2], p.t.c2[l], fmaf(a[1], p.t.c1[l], a[0])));
+    const float t1 = fmaf(b[3], p.t.c3[l], fmaf(b[2], p.t.c2[l], fmaf(b[1], p.t.c1[l], b[0])));
+    const float r0 = mod_near(t0, p.t.p[l], p.t.inv[l]), r1 = mod_near(t1, p.t.p[l], p.t.inv[l]);
+    out[l * plane] = __byte_perm(__float_as_uint(r0), __float_as_uint(r1), 0x7632);
+  }
+}
+
+// Operand -> residues: 8 bytes read and 2 NM written per element, about 7 NM FP32
+// instructions; bound by the writes (9.8 ms at 1.05e9 elements, 4.3 of 6.8 TB/s).  Gathered along K, a
+// warp takes 64 K of a row, four rows at a time, straight from global memory.  Otherwise a tile
+// of 64 walked rows x 64 K goes through shared memory, read along the rows.  One launch packs a
+// panel of each operand: the first blocks take A's, the others B's.
+static __global__ void __launch_bounds__(256, 5) rns_pack_kernel(const __grid_constant__ PackArgs p) {
+  __shared__ double tile[64][65];
+  __shared__ long long off[64], kof[64];
+  __shared__ int srow[64], ssh[64];
+  const int side = blockIdx.x >= p.s[0].blocks;
+  const PackSide& ps = p.s[side];
+  const Operand& o = ps.o;
+  const long long b = (long long)blockIdx.x - (side ? p.s[0].blocks : 0);
+  const long long nk = p.Kp >> 6;
+  const long long w = (b / nk) * (o.kfast ? 32 : 64);  // first row of the block
+  const long long kk0 = (b % nk) * 64;                 // first K, in the panel
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (o.kfast) {
+    const long long ka = kk0 + 2 * lane, kb = ka + 1;
+    const long long oa = ka < p.K ? k_offset(o, p.k0 + ka) : 0;
+    const long long ob = kb < p.K ? k_offset(o, p.k0 + kb) : 0;
+    const long long w1 = w + 4 * warp;
+    double x[4], y[4];
+    int row[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      x[u] = y[u] = 0.0;
+      row[u] = 0;
+      if (w1 + u < ps.nrow) {
+        row[u] = o.walk[ps.w0 + w1 + u];
+        const double* q = o.X + o.off[row[u]];
+        if (ka < p.K) x[u] = __ldg(q + oa);
+        if (kb < p.K) y[u] = __ldg(q + ob);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (w1 + u < ps.nrow)
+        store_residues(p, ps, x[u], y[u], row_shift(o, row[u], p.log2k),
+                       (row[u] - ps.w0) * p.Kp + kk0 + 2 * lane);
+  } else {
+    if (threadIdx.x < 64) {
+      kof[threadIdx.x] = kk0 + threadIdx.x < p.K ? k_offset(o, p.k0 + kk0 + threadIdx.x) : 0;
+      if (w + threadIdx.x < ps.nrow) {
+        const int r = o.walk[ps.w0 + w + threadIdx.x];
+        srow[threadIdx.x] = r;
+        off[threadIdx.x] = o.off[r];
+        ssh[threadIdx.x] = row_shift(o, r, p.log2k);
+      }
+    }
+    __syncthreads();
+    const int rr = threadIdx.x & 63;
+    double v[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+      const int k = (threadIdx.x >> 6) + 4 * u;
+      v[u] = (w + rr < ps.nrow && kk0 + k < p.K) ? __ldg(o.X + off[rr] + kof[k]) : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 16; ++u) tile[rr][(threadIdx.x >> 6) + 4 * u] = v[u];
+    __syncthreads();
+#pragma unroll 1
+    for (int r = warp; r < 64 && w + r < ps.nrow; r += 8)
+      store_residues(p, ps, tile[r][2 * lane], tile[r][2 * lane + 1], ssh[r],
+                     (srow[r] - ps.w0) * p.Kp + kk0 + 2 * lane);
+  }
+}
+
+// ---- GEMM over the residues -------------------------------------------------------------
+// Output tiles and K of a launch.  Plain: C[split][modulus] = A B^T over K blocks
+// [split kb_per_split, ...).  Triples (TRIP): group g = 3 t + q is orientation q of triple t,
+// the sum of four products of row blocks (pycc_gb300/triples.py, orientation_terms).
+struct GemmArgs {
+  long long M, N;    // rows of A and of B in this panel (TRIP: v^2 and v)
+  long long mt, nt;  // 128-row and bs-column tiles
+  int gm;            // M tiles per raster group
+  int bs;            // columns per N tile, a multiple of 16
+  int planes;        // splits, or groups
+  int nkb, kb_per_split;
+  long long ld;        // bytes of one output row: N rounded up to 16
+  unsigned char* out;  // [split or group][modulus][M][ld]
+  int* status;
+  unsigned long long wait_ns;
+  ModTab t;
+  // TRIP
+  const int* ijk;  // [triples][3]
+  int no, kv, ko;  // occupied orbitals, K blocks of the products over e and over m
+};
+
+struct GemmMaps {
+  CUtensorMap a[4];  // TRIP: VT, VN, TM, TMT
+  CUtensorMap b[2];  // TRIP: T2P, OB
+};
+
+constexpr int kEpiWarps = 8;
+constexpr int kGemmThreads = 64 + 32 * kEpiWarps;
+
+template <int BN>
+struct RSmem {
+  static constexpr int A_BYTES = BM * KBYTES, B_BYTES = BN * KBYTES;
+  static constexpr int STAGE = A_BYTES + B_BYTES;
+  static constexpr int TAIL = 256;
+  static constexpr int FIT = (232448 - 1024 - TAIL) / STAGE;
+  static constexpr int STAGES = FIT > 8 ? 8 : FIT;
+  static constexpr int TOTAL = 1024 + STAGES * STAGE + TAIL;
+  static constexpr unsigned TMEM_COLS = 2 * BN;
+  static_assert(BN == 64 || BN == 128 || BN == 256, "two accumulators in a power of two columns");
+};
+
+// One unit of work: an output tile of one modulus, the sum of up to four runs of K blocks.
+struct Unit {
+  int plane, mod, n0, blocks;  // plane: split or group; blocks: K blocks in all
+  long long m0;
+  int nseg, ma[4], mb[4], ya[4], yb[4], kb[4], nk[4];
+};
+
+// Unit u -> (modulus, split or group, tile): neighbouring groups share row blocks of one
+// modulus.  The tile order within a modulus is
+// tc_gemm_kernel's raster (groups of gm M tiles, M fastest), so a wave shares the row blocks of
+// both operands in L2.
+template <bool TRIP, bool SEGS>
+__device__ __forceinline__ Unit decode_unit(const GemmArgs& p, unsigned u) {
+  // 32-bit divisions: in 64 bits the chain took longer than the MMAs of a short-K unit
+  const unsigned mt = (unsigned)p.mt, nt = (unsigned)p.nt, per = mt * nt, gm = (unsigned)p.gm;
+  Unit x;
+  const unsigned g = u / per, r = u - g * per;
+  x.mod = (int)(g / (unsigned)p.planes);
+  x.plane = (int)(g - (unsigned)x.mod * (unsigned)p.planes);
+  const unsigned group = r / (gm * nt), rg = r - group * gm * nt;
+  const unsigned here = min(gm, mt - group * gm), n = rg / here;
+  x.m0 = (long long)(group * gm + (rg - n * here)) * BM;
+  x.n0 = (int)n * p.bs;
+  if (!TRIP) {
+    x.nseg = 1;
+    x.kb[0] = x.plane * p.kb_per_split;
+    x.blocks = x.nk[0] = min(p.nkb, x.kb[0] + p.kb_per_split) - x.kb[0];
+    if (SEGS) {
+      x.ma[0] = x.mb[0] = 0;
+      x.ya[0] = (int)(x.mod * p.M + x.m0);
+      x.yb[0] = (int)(x.mod * p.N + x.n0);
+    }
+    return x;
+  }
+  x.nseg = 4;
+  x.blocks = 2 * (p.kv + p.ko);
+  if (SEGS) {
+    const int q = x.plane % 3;
+    const int i = p.ijk[x.plane - q], j = p.ijk[x.plane - q + 1], k = p.ijk[x.plane - q + 2];
+    // (A map, its occupied index, the pair of B's row block) per product
+    const int s0 = q == 2 ? k : i, s1 = q == 0 ? j : (q == 1 ? k : j);
+    const int bx[4] = {q == 0 ? k : (q == 1 ? j : i), q == 0 ? k : (q == 1 ? j : i),
+                       q == 0 ? j : (q == 1 ? k : j), q == 0 ? i : (q == 1 ? i : k)};
+    const int by[4] = {q == 0 ? j : (q == 1 ? k : j), q == 0 ? i : (q == 1 ? i : k),
+                       q == 0 ? k : (q == 1 ? j : i), q == 0 ? k : (q == 1 ? j : i)};
+    const int ma[4] = {q == 2 ? 1 : 0, q == 2 ? 0 : 1, q == 2 ? 3 : 2, q == 2 ? 2 : 3};
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      x.ma[s] = ma[s];
+      x.mb[s] = s >> 1;
+      x.ya[s] = (int)(((long long)x.mod * p.no + ((s & 1) ? s1 : s0)) * p.M + x.m0);
+      x.yb[s] = (int)(((long long)x.mod * p.no * p.no + bx[s] * p.no + by[s]) * p.N + x.n0);
+      x.kb[s] = 0;
+      x.nk[s] = s < 2 ? p.kv : p.ko;
+    }
+  }
+  return x;
+}
+
+// Persistent and warp-specialised: warp 0 TMA, warp 1 MMA, warps 2-9 epilogue (a TMEM lane
+// quarter and a column half each).  The two TMEM accumulators alternate between chunks of
+// kChunk K blocks; the epilogue warps add each chunk to their running residues (BN / 2
+// registers per thread) and reduce modulo p while the other accumulator fills: four FP32
+// instructions per element and chunk.  Every wait is bounded; an expired one leaves its code in
+// *status and the caller's outputs become NaN.
+template <int BN, bool TRIP>
+static __global__ void __launch_bounds__(kGemmThreads, 1)
+    rns_gemm_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ GemmArgs p,
+                    unsigned units) {
+  using L = RSmem<BN>;
+  constexpr int S = L::STAGES;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw = smem_u32(smem_raw);
+  uint8_t* base = smem_raw + (((raw + 1023u) & ~1023u) - raw);
+  uint8_t* sA = base;
+  uint8_t* sB = base + S * L::A_BYTES;
+  uint64_t* full = reinterpret_cast<uint64_t*>(base + S * L::STAGE);
+  uint64_t* empty = full + S;
+  uint64_t* tfull = empty + S;
+  uint64_t* tempty = tfull + 2;
+  uint64_t* mdone = tempty + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mdone + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+
+  if (tid == 0) {
+    for (int s = 0; s < S; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&tfull[b], 1);
+      mbar_init(&tempty[b], kEpiWarps);
+    }
+    mbar_init(mdone, 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(tmem_slot)),
+                 "r"(L::TMEM_COLS));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int it = 0;
+      bool stop = false;
+      const uint32_t bytes = (uint32_t)(BM + p.bs) * KBYTES;
+      for (unsigned u = blockIdx.x; u < units && !stop; u += gridDim.x) {
+        const Unit x = decode_unit<TRIP, true>(p, u);
+#pragma unroll
+        for (int g = 0; g < (TRIP ? 4 : 1); ++g) {
+          const CUtensorMap* ta = &maps.a[x.ma[g]];
+          const CUtensorMap* tb = &maps.b[x.mb[g]];
+          for (int kb = x.kb[g]; kb < x.kb[g] + x.nk[g] && !stop; ++kb, ++it) {
+            const int s = it % S;
+            if (it >= S && !mbar_wait(&empty[s], ((it / S) - 1) & 1, p.wait_ns)) {
+              atomicExch(p.status, kStatusTimeoutEmpty);
+              *abort_flag = 1;
+            }
+            if (*abort_flag) {
+              stop = true;
+              break;
+            }
+            mbar_expect_tx(&full[s], bytes);
+            tma_load_2d(ta, &full[s], sA + s * L::A_BYTES, kb * 64, x.ya[g]);
+            tma_load_2d(tb, &full[s], sB + s * L::B_BYTES, kb * 64, x.yb[g]);
+          }
+        }
+      }
+      if (stop)  // copies in flight land before the CTA gives up its shared memory
+        for (int j = max(0, it - S); j < it; ++j)
+          mbar_wait(&full[j % S], (j / S) & 1, p.wait_ns);
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (lane == 0) {
+      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) |
+                             ((uint32_t)(p.bs >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+      int it = 0, c = 0;
+      bool stop = false;
+      for (unsigned u = blockIdx.x; u < units && !stop; u += gridDim.x) {
+        const int blocks = decode_unit<TRIP, false>(p, u).blocks;
+        for (int k0 = 0; k0 < blocks && !stop; k0 += kChunk, ++c) {
+          const int b = c & 1;
+          if (c >= 2 && !mbar_wait(&tempty[b], ((c >> 1) - 1) & 1, p.wait_ns)) {
+            atomicExch(p.status, kStatusTimeoutEmpty);
+            *abort_flag = 1;
+          }
+          if (*abort_flag) {
+            stop = true;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t d = tmem + (uint32_t)(b * BN);
+          uint32_t acc = 0u;
+          const int n = min(kChunk, blocks - k0);
+          for (int kb = 0; kb < n; ++kb, ++it) {
+            const int s = it % S;
+            if (!mbar_wait(&full[s], (it / S) & 1, p.wait_ns)) {
+              atomicExch(p.status, kStatusTimeoutFull);
+              *abort_flag = 1;
+            }
+            if (*abort_flag) {
+              stop = true;
+              break;
+            }
+            tc_fence_after();
+            const uint64_t da = sw128_desc(smem_u32(sA + s * L::A_BYTES));
+            const uint64_t db = sw128_desc(smem_u32(sB + s * L::B_BYTES));
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              umma_f16(d, da + 2 * k, db + 2 * k, idesc, acc);
+              acc = 1u;
+            }
+            umma_commit(&empty[s]);
+          }
+          umma_commit(&tfull[b]);
+        }
+      }
+      umma_commit(mdone);
+      mbar_wait(mdone, 0, p.wait_ns);  // every MMA retired before TMEM is released
+    }
+    __syncwarp();
+  } else {
+    const int q = warp & 3, h = (warp - 2) >> 2;
+    constexpr int HB = BN / 2;  // columns of this warp: [h HB, (h + 1) HB) of the tile
+    int c = 0;
+    bool stop = false;
+    for (unsigned u = blockIdx.x; u < units && !stop; u += gridDim.x) {
+      const Unit x = decode_unit<TRIP, false>(p, u);
+      const float pm = p.t.p[x.mod], inv = p.t.inv[x.mod];
+      float r[HB];
+#pragma unroll
+      for (int j = 0; j < HB; ++j) r[j] = 0.f;
+      for (int k0 = 0; k0 < x.blocks; k0 += kChunk, ++c) {
+        const int b = c & 1;
+        int okw = 1;
+        if (lane == 0) {
+          okw = mbar_wait_sleep(&tfull[b], (c >> 1) & 1, p.wait_ns) ? 1 : 0;
+          if (!okw) {
+            atomicExch(p.status, kStatusTimeoutDone);
+            *abort_flag = 1;
+          }
+          if (*abort_flag) okw = 0;
+        }
+        if (!__shfl_sync(0xffffffffu, okw, 0)) {  // warp-uniform: tcgen05.ld is .sync.aligned
+          stop = true;
+          break;
+        }
+        tc_fence_after();
+        const uint32_t tbase = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * BN + h * HB);
+#pragma unroll
+        for (int f = 0; f < HB / 32; ++f) {
+          if (h * HB + 32 * f >= p.bs) break;  // columns the tile does not have
+          uint32_t v[32];
+          tmem_ld32(tbase + 32 * f, v);
+#pragma unroll
+          for (int j = 0; j < 32; ++j)
+            r[32 * f + j] = mod_near(__uint_as_float(v[j]) + r[32 * f + j], pm, inv);
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&tempty[b]);
+      }
+      if (stop) break;
+      const long long row = x.m0 + q * 32 + lane;
+      if (row < p.M) {
+        unsigned char* o = p.out + (((long long)x.plane * NM + x.mod) * p.M + row) * p.ld;
+#pragma unroll
+        for (int f = 0; f < HB / 16; ++f) {
+          const int cj = h * HB + 16 * f;  // 16 columns: inside the tile and the row, or not at all
+          if (cj < p.bs && x.n0 + cj < p.ld) {
+            const float* e = r + 16 * f;
+            *reinterpret_cast<uint4*>(o + x.n0 + cj) =
+                make_uint4(residue_bytes(e[0], e[1], e[2], e[3]),
+                           residue_bytes(e[4], e[5], e[6], e[7]),
+                           residue_bytes(e[8], e[9], e[10], e[11]),
+                           residue_bytes(e[12], e[13], e[14], e[15]));
+          }
+        }
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
+                 "r"(L::TMEM_COLS));
+  }
+}
+
+// ---- residues -> FP64 ---------------------------------------------------------------------
+// Four outputs' sums of residue times floor(2^96 q / p), in three words of 64-bit accumulators.
+struct CrtSum {
+  unsigned long long s0[4], s1[4], s2[4];
+  __device__ __forceinline__ CrtSum(const CrtTab& t) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      s0[e] = t.b0;
+      s1[e] = t.b1;
+      s2[e] = t.b2;
+    }
+  }
+  // w[l]: the four outputs' bytes modulo the l-th modulus
+  __device__ __forceinline__ void add(const CrtTab& t, const unsigned (&w)[NM]) {
+#pragma unroll
+    for (int l = 0; l < NM; ++l)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const unsigned r = (w[l] >> (8 * e)) & 0xffu;
+        s0[e] += (unsigned long long)r * t.c0[l];
+        s1[e] += (unsigned long long)r * t.c1[l];
+        s2[e] += (unsigned long long)r * t.c2[l];
+      }
+  }
+  // output e: the signed fraction of P (their integer part fell out modulo 2^96) times 2^ex times
+  // t.scale, rounded to FP64 in integer arithmetic (GB300's FP64 pipe converts two values per
+  // clock and SM) and multiplied once; exponents that could make the intermediate subnormal
+  // scale last
+  __device__ __forceinline__ double value(const CrtTab& t, int e, int ex) const {
+    const unsigned long long t1 = s1[e] + (s0[e] >> 32);
+    const unsigned w2 = (unsigned)s2[e] + (unsigned)(t1 >> 32);
+    unsigned long long hi = ((unsigned long long)w2 << 32) | (unsigned)t1;
+    unsigned lo = (unsigned)s0[e];
+    const bool neg = (w2 >> 31) != 0;
+    if (neg) {  // two's complement of the 96 bits
+      lo = ~lo + 1u;
+      hi = ~hi + (lo == 0u ? 1ull : 0ull);
+    }
+    double v;
+    if (hi == 0 || ex < -800 || ex > 800) {
+      v = scalbn(fma(__ull2double_rn(hi), 4294967296.0, __uint2double_rn(lo)) * t.scale, ex);
+    } else {
+      const int lz = __clzll((long long)hi);
+      const unsigned long long top =
+          lz ? (hi << lz) | (((unsigned long long)lo << 32) >> (64 - lz)) : hi;
+      unsigned long long m = top >> 11;
+      const unsigned rest = (unsigned)top & 0x7ffu;
+      m += (rest > 0x400u || (rest == 0x400u && (m & 1ull))) ? 1ull : 0ull;
+      // top 2^(32 - lz) = m 2^(43 - lz), with m's leading bit added into the exponent field
+      v = __longlong_as_double(
+              (long long)(m + ((unsigned long long)(1023 + 94 - lz + ex) << 52))) * t.scale;
+    }
+    return neg ? -v : v;
+  }
+};
+
+// ---- host side --------------------------------------------------------------------------
+struct Tables {
+  ModTab mod;
+  CrtTab crt;
+};
+
+inline const Tables& tables() {
+  static const Tables t = [] {
+    Tables x{};
+    unsigned __int128 P = 1;
+    for (int p : kModuli) P *= (unsigned)p;
+    for (int l = 0; l < NM; ++l) {
+      const int p = kModuli[l];
+      auto sym = [p](long long r) { r %= p; return (float)(2 * r > p ? r - p : r); };
+      x.mod.p[l] = (float)p;
+      x.mod.inv[l] = 1.0f / (float)p;
+      x.mod.c1[l] = sym(1ll << digit_bit(1));
+      x.mod.c2[l] = sym(1ll << digit_bit(2));
+      x.mod.c3[l] = sym(1ll << digit_bit(3));
+      const unsigned m = (unsigned)((P / (unsigned)p) % (unsigned)p);
+      unsigned q = 1;
+      while ((q * m) % p != 1) ++q;
+      unsigned long long rem = q;
+      unsigned* w[3] = {x.crt.c2, x.crt.c1, x.crt.c0};
+      for (auto* word : w) {
+        word[l] = (unsigned)((rem << 32) / p);
+        rem = (rem << 32) % p;
+      }
+    }
+    x.crt.scale = std::ldexp((double)P, -96);
+    return x;
+  }();
+  return t;
+}
+
+// The tables of a join that adds up `planes` planes of biased bytes and scales by alpha.
+inline CrtTab crt_tab(int planes, double alpha) {
+  CrtTab t = tables().crt;
+  unsigned __int128 sum = 0;
+  for (int l = 0; l < NM; ++l)
+    sum += ((unsigned __int128)t.c2[l] << 64) | ((unsigned __int128)t.c1[l] << 32) | t.c0[l];
+  const unsigned __int128 b = -(sum * 128 * (unsigned)planes);
+  t.b0 = (unsigned)b;
+  t.b1 = (unsigned)(b >> 32);
+  t.b2 = (unsigned)(b >> 64);
+  t.scale *= alpha;
+  return t;
+}
+
+inline long long up(long long x, long long m) { return (x + m - 1) / m * m; }
+
+inline int blocks_for(long long n, int per) {
+  return (int)std::max(1LL, std::min((n + per - 1) / per, 16LL * num_sms()));
+}
+
+inline int run_norm(const Operand& a, const Operand& b, long long k0, long long k1, cudaStream_t st) {
+  NormArgs p{};
+  p.o[0] = a;
+  p.o[1] = b;
+  p.k0 = k0;
+  p.k1 = k1;
+  const long long K = k1 - k0;
+  for (int s = 0; s < 2; ++s) {
+    const Operand& o = p.o[s];
+    p.gx[s] = o.kfast ? (o.R + 7) / 8 : (o.R + 255) / 256;
+    const long long most = std::max(1LL, K / (o.kfast ? 512 : 32));
+    const long long segs = std::max(1LL, std::min((8LL * num_sms() + p.gx[s] - 1) / p.gx[s], most));
+    p.seg[s] = (K + segs - 1) / segs;
+    p.blocks[s] = p.gx[s] * ((K + p.seg[s] - 1) / p.seg[s]);
+  }
+  rns_norm_kernel<<<(unsigned)(p.blocks[0] + p.blocks[1]), 256, 0, st>>>(p);
+  PCG_CHECK_LAUNCH("rns norm");
+  return 0;
+}
+
+inline int run_pack(PackArgs& p, cudaStream_t st) {
+  for (PackSide& s : p.s) {
+    const int rows = s.o.kfast ? 32 : 64;
+    s.blocks = (p.Kp >> 6) * ((s.nrow + rows - 1) / rows);
+  }
+  rns_pack_kernel<<<(unsigned)(p.s[0].blocks + p.s[1].blocks), 256, 0, st>>>(p);
+  PCG_CHECK_LAUNCH("rns pack");
+  return 0;
+}
+
+template <int BN, bool TRIP>
+inline int run_gemm(const GemmMaps& maps, const GemmArgs& a, cudaStream_t st) {
+  const int smem = RSmem<BN>::TOTAL;
+  cudaFuncSetAttribute(rns_gemm_kernel<BN, TRIP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       smem);
+  const long long units = a.mt * a.nt * NM * a.planes;
+  if (units > 0x7fffffffLL) {
+    set_error("rns gemm: %lld units of work", units);
+    return -1;
+  }
+  rns_gemm_kernel<BN, TRIP>
+      <<<(unsigned)std::min<long long>(units, num_sms()), kGemmThreads, smem, st>>>(maps, a, (unsigned)units);
+  PCG_CHECK_LAUNCH("rns gemm");
+  return 0;
+}
+
+}  // namespace rns
+}  // namespace pcg

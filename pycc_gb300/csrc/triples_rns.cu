@@ -1,0 +1,288 @@
+// The connected triples t3c_ijk (pycc/cctriples.py:27-72) in FP64 on the BF16 tensor cores, by
+// the residue arithmetic of contract_rns.cu.
+//
+// The twelve terms of a triple are products of six operand matrices, turned into residues once
+// for one set of amplitudes:
+//   A side (rows (x, p, q)):  VT = <qp|ex>,  VN = <pq|ex>  (K = e);  TM = t2_xmpq,
+//                             TMT = t2_xmqp  (K = m)
+//   B side (rows (x, y, p)):  T2P = t2_xype  (K = e);  OB = -<mp|xy>  (K = m)
+// One GEMM launch computes the three orientations of a batch of triples, each the sum of four
+// products (pycc_gb300/triples.py, orientation_terms) in one accumulator: a sum of residues is
+// the residue of the sum when all four products carry the same scale, so a matrix has one power
+// of two for all its rows, chosen from its largest row norm so that the sum of the four stays
+// below half the product of the moduli.  A second kernel rebuilds the partials in FP64, in the
+// layout the energy kernel reads.  E(T) at no = 7, nv = 45: 63.4 ms with one FP64 launch per
+// triple and orientation (46.6 ms on a few SMs' FP64 pipes, a host synchronisation per triple),
+// 1.9 ms here (GEMM 0.73, rebuild 0.19, energy 0.44).
+#include "rns.cuh"
+
+namespace pcg {
+namespace rns {
+namespace {
+
+struct T3Shift {
+  int sh[4];  // V, T2P, t2 (rows of TM), OB
+  int total;  // sh[0] + sh[1] = sh[2] + sh[3]
+  int bad;    // an operand holds an Inf or a NaN
+};
+
+struct T3MaxArgs {
+  const float* norm2[4];
+  const unsigned* top[4];
+  long long R[4];
+  unsigned* out;  // [4] largest squared row norm (float bits), [4] largest exponent
+};
+
+__global__ void __launch_bounds__(256) t3_max_kernel(const T3MaxArgs p) {
+  const int q = blockIdx.y;
+  unsigned m = 0, t = 0;
+  for (long long r = (long long)blockIdx.x * 256 + threadIdx.x; r < p.R[q];
+       r += (long long)gridDim.x * 256) {
+    m = max(m, __float_as_uint(p.norm2[q][r]));  // non-negative: bits are ordered as values
+    t = max(t, p.top[q][r]);
+  }
+  for (int s = 16; s > 0; s >>= 1) {
+    m = max(m, __shfl_xor_sync(0xffffffffu, m, s));
+    t = max(t, __shfl_xor_sync(0xffffffffu, t, s));
+  }
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(p.out + q, m);
+    atomicMax(p.out + 4 + q, t);
+  }
+}
+
+// Powers of two with every product of rows at most 2^122 in norm: four of them sum to less than
+// half the product of the moduli (2^123.95).
+__global__ void t3_shift_kernel(const unsigned* mx, int log2v, int log2o, T3Shift* out) {
+  int e[4];  // row norms are at most 2^e
+  bool bad = false;
+  for (int q = 0; q < 4; ++q) {
+    const float n2 = __uint_as_float(mx[q]) * 1.0078125f;
+    const int top = (int)mx[4 + q];
+    bad = bad || top == 2047;
+    const int l2 = (n2 >= 0x1p-80f && n2 <= 0x1p100f)
+                       ? (int)(__float_as_uint(n2) >> 23) - 126
+                       : 2 * (max(top, 1) - 1022) + (q < 2 ? log2v : log2o);
+    e[q] = (l2 + 1) >> 1;
+  }
+  const int s1 = 122 - e[0] - e[1], s2 = 122 - e[2] - e[3], s = min(s1, s2);
+  out->sh[0] = 61 - e[0] - ((s1 - s) >> 1);
+  out->sh[1] = s - out->sh[0];
+  out->sh[2] = 61 - e[2] - ((s2 - s) >> 1);
+  out->sh[3] = s - out->sh[2];
+  out->total = s;
+  out->bad = bad;
+}
+
+struct T3JoinArgs {
+  const unsigned char* res;  // [group][modulus][v^2][ld]
+  long long ld;
+  int nv, groups;
+  double* P;  // [group][z][x][y]
+  const T3Shift* shift;
+  const int* status;
+  CrtTab t;
+};
+
+// Lanes along the rows (x, y), which are P's unit stride; four columns z per thread.
+__global__ void __launch_bounds__(256) t3_join_kernel(const __grid_constant__ T3JoinArgs p) {
+  const long long M = (long long)p.nv * p.nv;
+  const long long row = (long long)blockIdx.x * 32 + threadIdx.x;
+  const int col = 4 * (int)(blockIdx.y * 8 + threadIdx.y);
+  if (row >= M || col >= p.nv) return;
+  const bool bad = *p.status != 0 || p.shift->bad;
+  const int ex = -p.shift->total;
+  for (int g = blockIdx.z; g < p.groups; g += gridDim.z) {
+    const unsigned char* src = p.res + ((long long)g * NM * M + row) * p.ld + col;
+    unsigned w[NM];
+#pragma unroll
+    for (int l = 0; l < NM; ++l)
+      w[l] = __ldg(reinterpret_cast<const unsigned*>(src + (long long)l * M * p.ld));
+    CrtSum sum(p.t);
+    sum.add(p.t, w);
+    double* out = p.P + ((long long)g * p.nv + col) * M + row;
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (col + e < p.nv)
+        out[e * M] = bad ? __longlong_as_double(0x7ff8000000000000ll) : sum.value(p.t, e, ex);
+  }
+}
+
+// Workspace of a wave function: status and shifts, the residues of the six matrices, then each
+// batch's products (during packing the rows' tables lie there instead).
+struct T3Plan {
+  long long no, nv, rows_a, rows_b, kv, ko, ld;  // kv, ko: K padded to whole 64-K blocks
+  long long vt, vn, tm, tmt, t2p, ob, fixed;     // byte offsets; fixed: the end of the residues
+  long long tables, per_triple;
+};
+
+bool t3_plan(T3Plan& p, long long no, long long nv) {
+  if (no < 1 || nv < 1 || no > 2048 || nv > 8192) return false;
+  p.no = no;
+  p.nv = nv;
+  p.rows_a = no * nv * nv;
+  p.rows_b = no * no * nv;
+  p.kv = up(nv, 64);
+  p.ko = up(no, 64);
+  p.ld = up(nv, 16);
+  const long long av = up(NM * p.rows_a * p.kv * 2, 256), ao = up(NM * p.rows_a * p.ko * 2, 256);
+  p.vt = 256;
+  p.vn = p.vt + av;
+  p.tm = p.vn + av;
+  p.tmt = p.tm + ao;
+  p.t2p = p.tmt + ao;
+  p.ob = p.t2p + up(NM * p.rows_b * p.kv * 2, 256);
+  p.fixed = p.ob + up(NM * p.rows_b * p.ko * 2, 256);
+  p.tables = (4 * p.rows_a + 2 * p.rows_b) * (8 + 4 + 4 + 4) + 6 * 4 * 16;
+  p.per_triple = 3 * NM * nv * nv * p.ld;
+  return NM * p.rows_a < 0x7fffffffLL - BM && NM * p.rows_b < 0x7fffffffLL - 256 &&
+         (p.rows_a / 64 + p.rows_b / 32 + 4) * (p.kv / 64) < 0x7fffffffLL;
+}
+
+}  // namespace
+}  // namespace rns
+}  // namespace pcg
+
+using namespace pcg;
+using namespace pcg::rns;
+
+extern "C" int pcg_t3_rns_work(long long no, long long nv, int batch, long long* bytes) {
+  T3Plan p;
+  if (!bytes || batch < 1) {
+    set_error("pcg_t3_rns_work: bad arguments");
+    return -1;
+  }
+  *bytes = t3_plan(p, no, nv) ? p.fixed + std::max(p.tables, batch * p.per_triple) : 0;
+  return 0;
+}
+
+extern "C" int pcg_t3_rns_pack(const double* V, const double* O, const double* t2, long long no,
+                               long long nv, void* work, long long work_len, void* stream) {
+  T3Plan p;
+  if (!V || !O || !t2 || !work || ((uintptr_t)work & 255u) || !t3_plan(p, no, nv) ||
+      work_len < p.fixed + p.tables) {
+    set_error("pcg_t3_rns_pack: bad arguments, or too little workspace");
+    return -1;
+  }
+  cudaStream_t st = (cudaStream_t)stream;
+  unsigned char* w = (unsigned char*)work;
+  unsigned* mx = (unsigned*)(w + 64);
+  T3Shift* shift = (T3Shift*)(w + 128);
+  unsigned char* tb = w + p.fixed;
+  auto take = [&](long long bytes) {  // every array 16-byte aligned
+    unsigned char* r = tb;
+    tb += up(bytes, 16);
+    return r;
+  };
+  const long long o = no, v = nv;
+  auto operand = [&](const double* X, long long e0, long long s0, long long e1, long long s1,
+                     long long e2, long long s2, long long kstep, int near, int which) {
+    Operand x{};
+    x.X = X;
+    x.r.n = 3;
+    x.r.ext[0] = e0;
+    x.r.ext[1] = e1;
+    x.r.ext[2] = e2;
+    x.r.s0[0] = s0;
+    x.r.s0[1] = s1;
+    x.r.s0[2] = s2;
+    x.R = e0 * e1 * e2;
+    x.off = (long long*)take(8 * x.R);
+    x.walk = (int*)take(4 * x.R);
+    x.top = (unsigned*)take(4 * x.R);
+    x.norm2 = (float*)take(4 * x.R);
+    x.kstep = kstep;
+    x.kfast = kstep == 1;
+    x.wq = near;
+    x.shift = &shift->sh[which];
+    return x;
+  };
+  const Operand vt = operand(V, o, 1, v, v * o, v, v * v * o, o, 0, 0);
+  const Operand vn = operand(V, o, 1, v, v * v * o, v, v * o, o, 0, 0);
+  const Operand tm = operand(t2, o, o * v * v, v, v, v, 1, v * v, 2, 2);
+  const Operand tmt = operand(t2, o, o * v * v, v, 1, v, v, v * v, 1, 2);
+  const Operand t2p = operand(t2, o, o * v * v, o, v * v, v, v, 1, 2, 1);
+  const Operand ob = operand(O, o, o, o, 1, v, o * o, v * o * o, 1, 3);
+  const Operand none{};
+  struct {
+    Operand a, b;
+    long long K, Kp, pa, pb;
+  } pass[4] = {{vt, t2p, v, p.kv, p.vt, p.t2p}, {tm, ob, o, p.ko, p.tm, p.ob},
+               {vn, none, v, p.kv, p.vn, 0}, {tmt, none, o, p.ko, p.tmt, 0}};
+  cudaMemsetAsync(w, 0, 256, st);
+  for (auto& x : pass) {
+    TableArgs t{x.a, x.b, SubIdx{}, 0, nullptr, nullptr, nullptr};
+    rns_tables_kernel<<<blocks_for(x.a.R + x.b.R, 256), 256, 0, st>>>(t);
+    PCG_CHECK_LAUNCH("pcg_t3_rns_pack/tables");
+  }
+  for (int q = 0; q < 2; ++q)
+    if (run_norm(pass[q].a, pass[q].b, 0, pass[q].K, st)) return -2;
+  T3MaxArgs m{{vt.norm2, t2p.norm2, tm.norm2, ob.norm2}, {vt.top, t2p.top, tm.top, ob.top},
+              {vt.R, t2p.R, tm.R, ob.R}, mx};
+  t3_max_kernel<<<dim3(num_sms(), 4), 256, 0, st>>>(m);
+  PCG_CHECK_LAUNCH("pcg_t3_rns_pack/max");
+  auto log2up = [](long long x) {
+    int l = 0;
+    while ((1LL << l) < x) ++l;
+    return l;
+  };
+  t3_shift_kernel<<<1, 1, 0, st>>>(mx, log2up(v), log2up(o), shift);
+  PCG_CHECK_LAUNCH("pcg_t3_rns_pack/shift");
+  for (auto& x : pass) {
+    PackArgs a{{{x.a, 0, x.a.R, (__nv_bfloat16*)(w + x.pa), 0, 0},
+                {x.b, 0, x.b.R, (__nv_bfloat16*)(w + x.pb), x.b.X == O ? 0x80000000u : 0u, 0}},
+               0, x.K, x.Kp, 0, tables().mod};
+    if (run_pack(a, st)) return -2;
+  }
+  return 0;
+}
+
+extern "C" int pcg_t3_rns_partials(long long no, long long nv, const int* ijk, int ntrip, double* P,
+                                   void* work, long long work_len, void* stream) {
+  T3Plan p;
+  if (!ijk || ntrip < 1 || ntrip > 21845 || !P || !work || ((uintptr_t)work & 255u) ||
+      !t3_plan(p, no, nv) || work_len < p.fixed + ntrip * p.per_triple) {
+    set_error("pcg_t3_rns_partials: bad arguments, or too little workspace");
+    return -1;
+  }
+  cudaStream_t st = (cudaStream_t)stream;
+  unsigned char* w = (unsigned char*)work;
+  GemmArgs g{};
+  g.M = nv * nv;
+  g.N = nv;
+  g.mt = (g.M + BM - 1) / BM;
+  const int BN = nv > 128 ? 256 : (nv > 64 ? 128 : 64);
+  g.nt = (nv + BN - 1) / BN;
+  g.bs = (int)(16 * (((nv + 15) / 16 + g.nt - 1) / g.nt));
+  g.gm = 1;
+  g.planes = 3 * ntrip;
+  g.ld = p.ld;
+  g.out = w + p.fixed;
+  g.status = (int*)w;
+  g.wait_ns = wait_limit_ns();
+  g.t = tables().mod;
+  g.ijk = ijk;
+  g.no = (int)no;
+  g.kv = (int)(p.kv / 64);
+  g.ko = (int)(p.ko / 64);
+  GemmMaps maps{};
+  const long long a_off[4] = {p.vt, p.vn, p.tm, p.tmt}, b_off[2] = {p.t2p, p.ob};
+  for (int q = 0; q < 4; ++q) {
+    const long long kb = 2 * (q < 2 ? p.kv : p.ko);
+    if (!make_map(&maps.a[q], w + a_off[q], NM * p.rows_a, kb, kb, 2, BM)) return -1;
+  }
+  for (int q = 0; q < 2; ++q) {
+    const long long kb = 2 * (q == 0 ? p.kv : p.ko);
+    if (!make_map(&maps.b[q], w + b_off[q], NM * p.rows_b, kb, kb, 2, g.bs)) return -1;
+  }
+  const int rc = BN == 256   ? run_gemm<256, true>(maps, g, st)
+                 : BN == 128 ? run_gemm<128, true>(maps, g, st)
+                             : run_gemm<64, true>(maps, g, st);
+  if (rc) return rc;
+  T3JoinArgs j{w + p.fixed, p.ld, (int)nv, g.planes, P, (const T3Shift*)(w + 128),
+               (const int*)w, crt_tab(1, 1.0)};
+  const dim3 grid((unsigned)((g.M + 31) / 32), (unsigned)((nv + 31) / 32), (unsigned)g.planes);
+  t3_join_kernel<<<grid, dim3(32, 8), 0, st>>>(j);
+  PCG_CHECK_LAUNCH("pcg_t3_rns_partials");
+  return 0;
+}

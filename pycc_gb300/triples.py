@@ -18,9 +18,9 @@ Lee-Rendell weights, and accumulates E(T) in FP64.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 
-import numpy as np
 import torch
 
 from . import _lib
@@ -90,19 +90,37 @@ def triples_list(no):
     return [(i, j, k) for i in range(no) for j in range(i + 1) for k in range(j + 1)]
 
 
-def _energy(fp32, P1, P2, P3, pstride, ijk_dev, ntrip, w, t1, t2, part, stream):
-    H = w.H
-    o, v = w.o, w.v
-    fov = H.F[o, v].contiguous()
-    fov_ptr = fov.data_ptr() if bool(fov.abs().max() > 0) else None
-    _lib.call("pcg_triples_energy", int(fp32), P1.data_ptr(), P2.data_ptr(), P3.data_ptr(),
-              int(pstride), ijk_dev.data_ptr(), int(ntrip), H.eps.data_ptr(),
-              H.ERI[o, o, v, v].data_ptr(), t1.data_ptr(), t2.data_ptr(), fov_ptr, w.no, w.nv,
-              part.data_ptr(), _lib.stream_handle(stream))
+T3_WORK_LIMIT = 8 << 30      # bytes of scratch (residues, products and partials) of one E(T)
+
+
+def _t3_scratch(no, nv, ntrip, device, stream):
+    """(work, partials, batch) for the residue path on ``device``, owned by the launching stream,
+    or None when the device has no room for it.  The residues of the operands are one block for
+    all triples; the batch takes what the limit leaves, at least one triple."""
+    def bytes_of(batch):
+        out = C.c_longlong(0)
+        _lib.call("pcg_t3_rns_work", no, nv, batch, C.byref(out))
+        return out.value
+    if not bytes_of(1):
+        return None
+    each = bytes_of(1 << 20) - bytes_of((1 << 20) - 1) + 24 * nv ** 3
+    batch = max(1, min(ntrip, 4096, (T3_WORK_LIMIT - bytes_of(1)) // each))
+    with torch.cuda.stream(stream) if stream is not None else contextlib.nullcontext():
+        for b in sorted({batch, min(batch, 4), 1}, reverse=True):
+            try:
+                return (torch.empty(bytes_of(b), dtype=torch.uint8, device=device),
+                        torch.empty((b, 3, nv, nv, nv), dtype=torch.float64, device=device), b)
+            except torch.cuda.OutOfMemoryError:
+                pass
+    return None
 
 
 def t_energy_fp64(w, t1=None, t2=None):
-    """E(T) with FP64 partials (DMMA) and FP64 energy arithmetic."""
+    """E(T) with FP64 partials and FP64 energy arithmetic.
+
+    The partials of a batch of triples come from one launch of the residue GEMM on the tensor
+    cores (``csrc/triples_rns.cu``); without room for its scratch, from the FP64 multi-term
+    contraction, one triple and orientation at a time."""
     t1 = (w.t1 if t1 is None else t1).contiguous()
     t2 = (w.t2 if t2 is None else t2).contiguous()
     no, nv = w.no, w.nv
@@ -110,17 +128,39 @@ def t_energy_fp64(w, t1=None, t2=None):
     V = w.H.ERI[v, v, v, o]
     O = w.H.ERI[o, v, o, o]
     dev = t2.device
-    P = torch.empty((3, nv, nv, nv), dtype=torch.float64, device=dev)
+    st = _lib.stream_handle(w.stream)
     trips = triples_list(no)
+    scratch = _t3_scratch(no, nv, len(trips), dev, w.stream) if t2.is_cuda else None
     part = torch.empty((len(trips), nv), dtype=torch.float64, device=dev)
     ijk = torch.tensor(trips, dtype=torch.int32, device=dev)
-    for t, (i, j, k) in enumerate(trips):
-        for q, (lab, terms) in enumerate(orientation_terms(i, j, k, t2, V, O)):
-            contract_multi(P[q].permute(1, 2, 0), lab, terms, stream=w.stream)
-        _energy(False, P[0], P[1], P[2], 0, ijk[t:t + 1], 1, w, t1, t2, part[t:t + 1], w.stream)
+    fov = w.H.F[o, v].contiguous()
+    fov_ptr = fov.data_ptr() if bool(fov.abs().max() > 0) else None
+    eoovv = w.H.ERI[o, o, v, v].contiguous()
+
+    def energy(t0, n, P):
+        _lib.call("pcg_triples_energy", 0, P[0, 0].data_ptr(), P[0, 1].data_ptr(),
+                  P[0, 2].data_ptr(), 3 * nv ** 3, ijk[t0:].data_ptr(), n, w.H.eps.data_ptr(),
+                  eoovv.data_ptr(), t1.data_ptr(), t2.data_ptr(), fov_ptr, no, nv,
+                  part[t0:].data_ptr(), st)
+
+    if scratch is None:
+        P = torch.empty((1, 3, nv, nv, nv), dtype=torch.float64, device=dev)
+        for t, (i, j, k) in enumerate(trips):
+            for q, (lab, terms) in enumerate(orientation_terms(i, j, k, t2, V, O)):
+                contract_multi(P[0, q].permute(1, 2, 0), lab, terms, stream=w.stream)
+            energy(t, 1, P)
+    else:
+        work, P, batch = scratch
+        V, O = V.contiguous(), O.contiguous()
+        _lib.call("pcg_t3_rns_pack", V.data_ptr(), O.data_ptr(), t2.data_ptr(), no, nv,
+                  work.data_ptr(), work.numel(), st)
+        for t0 in range(0, len(trips), batch):
+            n = min(batch, len(trips) - t0)
+            _lib.call("pcg_t3_rns_partials", no, nv, ijk[t0:].data_ptr(), n, P.data_ptr(),
+                      work.data_ptr(), work.numel(), st)
+            energy(t0, n, P)
     out = torch.zeros((), dtype=torch.float64, device=dev)
-    _lib.call("pcg_reduce_sum_f64", part.data_ptr(), part.numel(), out.data_ptr(),
-              _lib.stream_handle(w.stream))
+    _lib.call("pcg_reduce_sum_f64", part.data_ptr(), part.numel(), out.data_ptr(), st)
     return float(out)
 
 

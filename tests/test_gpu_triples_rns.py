@@ -1,0 +1,60 @@
+"""The connected triples in residue arithmetic (csrc/triples_rns.cu) against the FP64 multi-term
+contraction, at the edges of tiles and K blocks, and what non-finite operands give.
+
+Tolerance: a partial sums four products of rows of length K = nv or no; the FP64 side rounds each
+of its multiply-adds by 2^-53 of a partial sum of at most sum |a||b|, the residue side its scaled
+operands by less than 2^-56 of the largest row norms' products.
+"""
+import ctypes as C
+
+import pytest
+import torch
+
+from pycc_gb300 import _lib
+from pycc_gb300.triples import contract_multi, orientation_terms
+
+pytestmark = pytest.mark.gpu
+
+
+def partials(V, O, t2, trips, batch):
+    no, nv = t2.shape[0], t2.shape[2]
+    nbytes = C.c_longlong(0)
+    _lib.call("pcg_t3_rns_work", no, nv, batch, C.byref(nbytes))
+    work = torch.empty(nbytes.value, dtype=torch.uint8, device=t2.device)
+    _lib.call("pcg_t3_rns_pack", V.data_ptr(), O.data_ptr(), t2.data_ptr(), no, nv,
+              work.data_ptr(), work.numel(), _lib.stream_handle())
+    ijk = torch.tensor(trips, dtype=torch.int32, device=t2.device)
+    out = torch.full((len(trips), 3, nv, nv, nv), float("nan"), dtype=torch.float64,
+                     device=t2.device)
+    for t0 in range(0, len(trips), batch):
+        n = min(batch, len(trips) - t0)
+        _lib.call("pcg_t3_rns_partials", no, nv, ijk[t0:].data_ptr(), n, out[t0].data_ptr(),
+                  work.data_ptr(), work.numel(), _lib.stream_handle())
+    return out
+
+
+@pytest.mark.parametrize("no,nv", [(1, 1), (2, 3), (3, 19), (2, 64), (65, 5), (3, 65), (2, 130),
+                                   (1, 257)])
+def test_partials(cuda, no, nv):
+    gen = torch.Generator(device=cuda).manual_seed(no + nv)
+    rand = lambda *s: torch.randn(s, dtype=torch.float64, device=cuda, generator=gen)
+    V, O, t2 = rand(nv, nv, nv, no), rand(no, nv, no, no), 0.1 * rand(no, no, nv, nv)
+    trips = [(no - 1, no // 2, 0), (no - 1, no - 1, no // 3), (0, 0, 0)]
+    got = partials(V, O, t2, trips, 2)
+    for t, (i, j, k) in enumerate(trips):
+        for q, (lab, terms) in enumerate(orientation_terms(i, j, k, t2, V, O)):
+            ref, mag = torch.empty_like(got[t, q]), torch.empty_like(got[t, q])
+            contract_multi(ref.permute(1, 2, 0), lab, terms)
+            contract_multi(mag.permute(1, 2, 0), lab,
+                           [(1.0, A.abs(), la, B.abs(), lb) for _, A, la, B, lb in terms])
+            top = float(mag.max())
+            tol = 2.0 ** -53 * (2 * (nv + no) + 8) * mag + 2.0 ** -56 * top
+            assert bool(((got[t, q] - ref).abs() <= tol).all())
+
+
+def test_not_finite(cuda):
+    gen = torch.Generator(device=cuda).manual_seed(1)
+    rand = lambda *s: torch.randn(s, dtype=torch.float64, device=cuda, generator=gen)
+    V, O, t2 = rand(7, 7, 7, 3), rand(3, 7, 3, 3), rand(3, 3, 7, 7)
+    t2[1, 2, 3, 4] = float("inf")
+    assert bool(partials(V, O, t2, [(2, 1, 0)], 1).isnan().all())
