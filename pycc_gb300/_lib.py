@@ -7,7 +7,10 @@ element strides and sizes; streams as ``cudaStream_t`` handles.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import os
+
+import torch
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libpycc_gb300.so")
@@ -102,16 +105,20 @@ def exported_symbols():
     return list(SIGNATURES)
 
 
+@functools.lru_cache(maxsize=8192)
+def _i64_array(vals):
+    return (C.c_longlong * max(1, len(vals)))(*[int(x) for x in vals])
+
+
 def i64s(vals):
-    vals = [int(x) for x in vals]
-    return (C.c_longlong * max(1, len(vals)))(*vals)
+    """A C array of long long for the library to read (shared between equal calls)."""
+    return _i64_array(tuple(vals))
 
 
 def call(name, *args):
-    lib = load()
-    rc = getattr(lib, name)(*args)
+    rc = getattr(_lib or load(), name)(*args)
     if rc != 0:
-        msg = lib.pcg_last_error().decode(errors="replace")
+        msg = _lib.pcg_last_error().decode(errors="replace")
         raise EngineError("%s failed (%d): %s" % (name, rc, msg))
     return rc
 
@@ -129,6 +136,16 @@ def launch_count() -> int:
 
 def stream_handle(stream=None):
     """cudaStream_t of a torch stream (default: the current stream)."""
-    import torch
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return C.c_void_p(s.cuda_stream)
+    if stream is not None:
+        return C.c_void_p(stream.cuda_stream)
+    # the raw handle of the current device's current stream, without building a Stream object
+    return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
+
+
+def remember(cache, key, value, most=4096):
+    """Store a plan in a module's bounded cache (emptied when full).  Plans depend on the labels,
+    extents and strides in their key alone, and are not changed once stored."""
+    if len(cache) >= most:
+        cache.clear()
+    cache[key] = value
+    return value

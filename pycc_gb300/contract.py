@@ -14,6 +14,7 @@ from __future__ import annotations
 
 import ctypes as C
 import functools
+import itertools
 import math
 
 import torch
@@ -107,50 +108,74 @@ def _check(t, name):
         raise TypeError("contract: %s must be float64, got %s" % (name, t.dtype))
 
 
+class _Call:
+    """The launch arguments of one contraction that its labels, extents and strides fix: the
+    sub-index groups as C arrays, the offsets of its batch indices, the output shape and whether
+    it goes to the residue path."""
+
+    def __init__(self, subscripts, a, b, out):
+        plan = ContractPlan(subscripts, a, b)
+        self.shape = plan.shape
+        if out is None:
+            out = torch.empty(plan.shape, dtype=torch.float64, device="meta")
+        elif tuple(out.shape) != plan.shape:
+            raise ValueError("contract: out has shape %s, expected %s"
+                             % (tuple(out.shape), plan.shape))
+        M, N, K, batch, ast, bst, cst = plan.groups(a, b, out)
+        self.groups = _group_args(M, N, K)
+        self.mnk = tuple(math.prod([g[0] for g in G]) for G in (M, N, K))
+        self.rns = _takes_rns(*self.mnk)
+        # batch indices (present in both operands and the output): one launch per value
+        self.batch = [tuple(8 * sum(v * st[c] for v, c in zip(vals, batch))
+                            for st in (ast, bst, cst))
+                      for vals in itertools.product(*[range(plan.ext[c]) for c in batch])]
+
+
+_CALLS = {}
+
+
 def contract_f64(subscripts, a, b, out=None, alpha=1.0, beta=0.0, stream=None):
-    """``out = beta*out + alpha * einsum(subscripts, a, b)`` on the FP64 DMMA kernel."""
+    """``out = beta*out + alpha * einsum(subscripts, a, b)`` in FP64: on the FP64 DMMA kernel, or,
+    where that is the shorter (``_takes_rns``), on the tensor cores in residue arithmetic."""
     _check(a, "operand 0")
     _check(b, "operand 1")
-    plan = ContractPlan(subscripts, a, b)
-    if out is None:
-        out = torch.empty(plan.shape, dtype=torch.float64, device=a.device)
-        beta = 0.0
-    else:
+    if out is not None:
         _check(out, "out")
-        if tuple(out.shape) != plan.shape:
-            raise ValueError("contract: out has shape %s, expected %s" % (tuple(out.shape), plan.shape))
-    M, N, K, batch, ast, bst, cst = plan.groups(a, b, out)
+    key = (subscripts, a.shape, a.stride(), b.shape, b.stride(),
+           None if out is None else (out.shape, out.stride()))
+    call = _CALLS.get(key)
+    if call is None:
+        call = _lib.remember(_CALLS, key, _Call(subscripts, a, b, out))
+    if out is None:
+        out = torch.empty(call.shape, dtype=torch.float64, device=a.device)
+        beta = 0.0
+    work = _rns_scratch(*call.mnk, out.device, stream) if call.rns and out.is_cuda else None
     st = _lib.stream_handle(stream)
-    work = None
-    if out.is_cuda:
-        m, n, k = (math.prod([g[0] for g in G]) for G in (M, N, K))
-        if _takes_rns(m, n, k):
-            work = _rns_scratch(m, n, k, out.device, stream)
-    if not batch:
-        _launch(M, N, K, alpha, a.data_ptr(), b.data_ptr(), beta, out.data_ptr(), st, work)
-        return out
-    # batch indices (present in both operands and the output): one launch per value
-    import itertools
-    rngs = [range(plan.ext[c]) for c in batch]
-    for vals in itertools.product(*rngs):
-        oa = sum(v * ast[c] for v, c in zip(vals, batch)) * 8
-        ob = sum(v * bst[c] for v, c in zip(vals, batch)) * 8
-        oc = sum(v * cst[c] for v, c in zip(vals, batch)) * 8
-        _launch(M, N, K, alpha, a.data_ptr() + oa, b.data_ptr() + ob, beta,
-                out.data_ptr() + oc, st, work)
+    pa, pb, pc = a.data_ptr(), b.data_ptr(), out.data_ptr()
+    for oa, ob, oc in call.batch:
+        _launch_groups(call.groups, alpha, pa + oa, pb + ob, beta, pc + oc, st, work)
     return out
 
 
-def _launch(M, N, K, alpha, pa, pb, beta, pc, st, work=None):
+def _group_args(M, N, K):
+    """The three sub-index groups as the library takes them."""
     i64 = _lib.i64s
-    args = (len(M), i64([g[0] for g in M]), i64([g[1] for g in M]), i64([g[2] for g in M]),
-            len(N), i64([g[0] for g in N]), i64([g[1] for g in N]), i64([g[2] for g in N]),
-            len(K), i64([g[0] for g in K]), i64([g[1] for g in K]), i64([g[2] for g in K]),
-            float(alpha), pa, pb, float(beta), pc)
+    out = ()
+    for G in (M, N, K):
+        out += (len(G), i64([g[0] for g in G]), i64([g[1] for g in G]), i64([g[2] for g in G]))
+    return out
+
+
+def _launch_groups(groups, alpha, pa, pb, beta, pc, st, work=None):
     if work is None:
-        _lib.call("pcg_contract_f64", *args, st)
+        _lib.call("pcg_contract_f64", *groups, float(alpha), pa, pb, float(beta), pc, st)
     else:
-        _lib.call("pcg_contract_rns_f64", *args, work.data_ptr(), work.numel(), st)
+        _lib.call("pcg_contract_rns_f64", *groups, float(alpha), pa, pb, float(beta), pc,
+                  work.data_ptr(), work.numel(), st)
+
+
+def _launch(M, N, K, alpha, pa, pb, beta, pc, st, work=None):
+    _launch_groups(_group_args(M, N, K), alpha, pa, pb, beta, pc, st, work)
 
 
 RNS_WORK_LIMIT = 8 << 30     # bytes of scratch of one contraction in residue arithmetic

@@ -55,6 +55,7 @@ class Operand:
         self.a, self.b, self.c, self.d = a, b, c, d
         self.X, self.Y, self.P, self.Q, self.R, self.S = X, Y, P, Q, R, S
         self.key = key            # cache key for static operands (None = dynamic)
+        self._geometry = None
 
     @staticmethod
     def of(labels, t, key=None):
@@ -83,6 +84,13 @@ class Operand:
             t, lab = s
             out.append(t.stride(lab.index(label)) if label in lab else 0)
         return out
+
+    def geometry(self):
+        """What fixes this operand's gather besides its data: labels, extents and strides."""
+        if self._geometry is None:
+            self._geometry = tuple([None if s is None else (s[1], s[0].shape, s[0].stride())
+                                    for s in self.sources()])
+        return self._geometry
 
     def device(self):
         return next(s for s in self.sources() if s is not None)[0].device
@@ -125,6 +133,46 @@ def kblock(fmt):
 NSRC = 6   # sources of a packed operand: X, Y, P, Q, R, S
 
 
+class PackPlan:
+    """The gather of one operand as the library takes it: row and K sub-indices with their
+    per-source strides, and the gather's identity (``geo``: extents and strides whatever the
+    labels), for operands reached through differently named labels."""
+
+    def __init__(self, op, row_labels, k_labels, R, K):
+        ext = op.extents()
+        rows = [(ext[c], op.strides(c)) for c in row_labels]
+        ks = [(ext[c], op.strides(c)) for c in k_labels]
+        self.geo = tuple(tuple((n, tuple(st)) for n, st in g) for g in (rows, ks))
+        self.R = math.prod(ext[c] for c in row_labels) if R is None else R
+        self.K = math.prod(ext[c] for c in k_labels) if K is None else K
+        rows, ks = _merge_multi(rows), _merge_multi(ks)
+        if len(rows) > MAX_SUB or len(ks) > MAX_SUB:
+            raise ValueError("pack: more than %d sub-indices" % MAX_SUB)
+        self.args = self.flat(rows) + self.flat(ks)
+
+    @staticmethod
+    def flat(groups):
+        e = [g[0] for g in groups]
+        st = [0] * (NSRC * MAX_SUB)
+        for q, (_, s) in enumerate(groups):
+            for src in range(NSRC):
+                st[src * MAX_SUB + q] = s[src]
+        return len(groups), _lib.i64s(e), _lib.i64s(st)
+
+
+_PACK_PLANS = {}
+
+
+def pack_plan(op, row_labels, k_labels, row_tab=None, k_tab=None):
+    key = (op.geometry(), tuple(row_labels), tuple(k_labels),
+           None if row_tab is None else int(row_tab.shape[1]),
+           None if k_tab is None else int(k_tab.shape[1]))
+    plan = _PACK_PLANS.get(key)
+    if plan is None:
+        plan = _lib.remember(_PACK_PLANS, key, PackPlan(op, row_labels, k_labels, *key[3:]))
+    return plan
+
+
 def pack(op: Operand, row_labels, k_labels, fmt, stream=None, row_tab=None, k_tab=None,
          k_w=None) -> Packed:
     """Pack ``op`` with rows over ``row_labels`` (or the explicit per-source row offsets
@@ -132,14 +180,8 @@ def pack(op: Operand, row_labels, k_labels, fmt, stream=None, row_tab=None, k_ta
     offsets ``k_tab``, int64 [6, K], with optional float32 K multipliers ``k_w``).  With a
     table the labels' strides still tell the kernel which side is unit-stride."""
     fmt = pack_format(fmt)
-    ext = op.extents()
-    rows = [(ext[c], op.strides(c)) for c in row_labels]
-    ks = [(ext[c], op.strides(c)) for c in k_labels]
-    R = math.prod(ext[c] for c in row_labels) if row_tab is None else int(row_tab.shape[1])
-    K = math.prod(ext[c] for c in k_labels) if k_tab is None else int(k_tab.shape[1])
-    rows, ks = _merge_multi(rows), _merge_multi(ks)
-    if len(rows) > MAX_SUB or len(ks) > MAX_SUB:
-        raise ValueError("pack: more than %d sub-indices" % MAX_SUB)
+    plan = pack_plan(op, row_labels, k_labels, row_tab, k_tab)
+    R, K = plan.R, plan.K
     for tab in (row_tab, k_tab):
         if tab is not None and (tab.dtype != torch.int64 or tab.shape[0] != NSRC
                                 or not tab.is_contiguous()):
@@ -161,25 +203,36 @@ def pack(op: Operand, row_labels, k_labels, fmt, stream=None, row_tab=None, k_ta
         mid = torch.empty_like(hi) if fmt == FMT_BF16X6 else None
         scale = None
 
-    def flat(groups):
-        e = [g[0] for g in groups]
-        st = [0] * (NSRC * MAX_SUB)
-        for q, (_, s) in enumerate(groups):
-            for src in range(NSRC):
-                st[src * MAX_SUB + q] = s[src]
-        return len(groups), _lib.i64s(e), _lib.i64s(st)
-
     def ptr(t):
         return t.data_ptr() if t is not None else None
 
-    rn, re_, rs = flat(rows)
-    kn, ke, kst = flat(ks)
-    _lib.call("pcg_pack_operand", int(fmt), rn, re_, rs, kn, ke, kst, Kp,
+    _lib.call("pcg_pack_operand", int(fmt), *plan.args, Kp,
               float(op.a), _ptr(op.X), float(op.b), _ptr(op.Y), float(op.c), _ptr(op.P),
               _ptr(op.Q), float(op.d), _ptr(op.R), _ptr(op.S), hi.data_ptr(), ptr(mid), ptr(lo),
               ptr(scale), ptr(row_tab), R if row_tab is not None else 0, ptr(k_tab), ptr(k_w),
               K if k_tab is not None else 0, _lib.stream_handle(stream))
     return Packed(fmt, R, Kp, hi, lo, scale, mid)
+
+
+_MAP_PLANS = {}
+
+
+def _output_map(out, row_labels, col_labels, out_labels, with_cols):
+    """The output's row and column sub-indices as the library takes them."""
+    key = (out.shape, out.stride(), tuple(row_labels), tuple(col_labels), out_labels, with_cols)
+    got = _MAP_PLANS.get(key)
+    if got is None:
+        ost = dict(zip(out_labels, out.stride()))
+        oext = dict(zip(out_labels, out.shape))
+        mg = _merge_multi([(oext[c], [ost[c]]) for c in row_labels])
+        ng = _merge_multi([(oext[c], [ost[c]]) for c in col_labels]) if with_cols else []
+        if len(mg) > MAX_SUB or len(ng) > MAX_SUB:
+            raise ValueError("gemm: more than %d output sub-indices" % MAX_SUB)
+        args = ()
+        for g in (mg, ng):
+            args += (len(g), _lib.i64s([x[0] for x in g]), _lib.i64s([x[1][0] for x in g]))
+        got = _lib.remember(_MAP_PLANS, key, args)
+    return got
 
 
 def gemm(fmt, A: Packed, B: Packed, out, row_labels, col_labels, out_labels, alpha=1.0,
@@ -188,25 +241,57 @@ def gemm(fmt, A: Packed, B: Packed, out, row_labels, col_labels, out_labels, alp
     (or, for the columns, the explicit offsets ``col_map`` and multipliers ``col_scale``)."""
     if A.Kp != B.Kp:
         raise ValueError("gemm: K mismatch %d vs %d" % (A.Kp, B.Kp))
-    ost = dict(zip(out_labels, out.stride()))
-    oext = dict(zip(out_labels, out.shape))
-    mg = _merge_multi([(oext[c], [ost[c]]) for c in row_labels])
-    ng = _merge_multi([(oext[c], [ost[c]]) for c in col_labels]) if col_map is None else []
-    if len(mg) > MAX_SUB or len(ng) > MAX_SUB:
-        raise ValueError("gemm: more than %d output sub-indices" % MAX_SUB)
-    i64 = _lib.i64s
+    maps = _output_map(out, row_labels, col_labels, out_labels, col_map is None)
+
     def p(t):
         return t.data_ptr() if t is not None else None
     _lib.call("pcg_tc_gemm", int(fmt), p(A.hi), p(A.mid), p(A.lo), A.rows, A.Kp,
-              p(B.hi), p(B.mid), p(B.lo), B.rows, B.Kp, A.Kp,
-              A.scale.data_ptr() if A.scale is not None else None,
-              B.scale.data_ptr() if B.scale is not None else None,
-              len(mg), i64([g[0] for g in mg]), i64([g[1][0] for g in mg]),
-              len(ng), i64([g[0] for g in ng]), i64([g[1][0] for g in ng]),
-              col_map.data_ptr() if col_map is not None else None,
-              col_scale.data_ptr() if col_scale is not None else None,
-              float(alpha), float(beta), out.data_ptr(), status.data_ptr(),
-              _lib.stream_handle(stream))
+              p(B.hi), p(B.mid), p(B.lo), B.rows, B.Kp, A.Kp, p(A.scale), p(B.scale), *maps,
+              p(col_map), p(col_scale), float(alpha), float(beta), out.data_ptr(),
+              status.data_ptr(), _lib.stream_handle(stream))
+
+
+_CONTRACT_PLANS = {}
+
+
+def _contract_plan(subscripts, A, B, out):
+    """(swap, rows, columns, K labels) of one contraction: which operand takes the 128-row tile
+    side and in which order its indices run."""
+    key = (subscripts, A.labels, B.labels, A.geometry(), B.geometry(), A.key is None, out.shape,
+           out.stride())
+    got = _CONTRACT_PLANS.get(key)
+    if got is not None:
+        return got
+    lhs, rhs = subscripts.replace(" ", "").split("->")
+    la, lb = lhs.split(",")
+    if la != A.labels or lb != B.labels:
+        raise ValueError("contract: operand labels %s,%s do not match %s" % (A.labels, B.labels, lhs))
+    ost = dict(zip(rhs, out.stride()))
+    ea, eb = A.extents(), B.extents()
+    ma = [c for c in rhs if c in la and c not in lb]
+    nb = [c for c in rhs if c in lb and c not in la]
+    kk = [c for c in la if c in lb and c not in rhs]
+    if len(ma) + len(nb) != len(rhs):
+        raise ValueError("contract: batch indices are not supported (%s)" % subscripts)
+    # rows / cols in output-stride order (innermost last); K by the dynamic operand
+    ma.sort(key=lambda c: -ost[c])
+    nb.sort(key=lambda c: -ost[c])
+    dyn = A if A.key is None else B
+    dst = {c: max(abs(s) for s in dyn.strides(c)) for c in kk}
+    kk.sort(key=lambda c: -dst[c])
+    mA = math.prod(ea[c] for c in ma) if ma else 1
+    nB = math.prod(eb[c] for c in nb) if nb else 1
+    # The 128-row tile side: the side holding the output's unit-stride index (so a warp's
+    # 32 consecutive rows store to consecutive addresses), unless it is too short.
+    inner = min(rhs, key=lambda c: abs(ost[c]))
+    if inner in nb and nB >= 128:
+        swap = True
+    elif inner in ma and mA >= 128:
+        swap = False
+    else:
+        swap = nB > mA
+    rows, cols = (nb, ma) if swap else (ma, nb)
+    return _lib.remember(_CONTRACT_PLANS, key, (swap, rows, cols, kk, rhs))
 
 
 class TCEngine:
@@ -221,39 +306,12 @@ class TCEngine:
         self.dyn_cache = None     # per-residual cache of packed dynamic operands
 
     def contract(self, subscripts, A: Operand, B: Operand, out, alpha=1.0, beta=1.0, fmt=FMT_BF16):
-        lhs, rhs = subscripts.replace(" ", "").split("->")
-        la, lb = lhs.split(",")
-        if la != A.labels or lb != B.labels:
-            raise ValueError("contract: operand labels %s,%s do not match %s" % (A.labels, B.labels, lhs))
-        ost = dict(zip(rhs, out.stride()))
-        ea, eb = A.extents(), B.extents()
-        ma = [c for c in rhs if c in la and c not in lb]
-        nb = [c for c in rhs if c in lb and c not in la]
-        kk = [c for c in la if c in lb and c not in rhs]
-        if len(ma) + len(nb) != len(rhs):
-            raise ValueError("contract: batch indices are not supported (%s)" % subscripts)
-        # rows / cols in output-stride order (innermost last); K by the dynamic operand
-        ma.sort(key=lambda c: -ost[c])
-        nb.sort(key=lambda c: -ost[c])
-        dyn = A if A.key is None else B
-        dst = {c: max(abs(s) for s in dyn.strides(c)) for c in kk}
-        kk.sort(key=lambda c: -dst[c])
-        mA = math.prod(ea[c] for c in ma) if ma else 1
-        nB = math.prod(eb[c] for c in nb) if nb else 1
-        # The 128-row tile side: the side holding the output's unit-stride index (so a warp's
-        # 32 consecutive rows store to consecutive addresses), unless it is too short.
-        inner = min(rhs, key=lambda c: abs(ost[c]))
-        if inner in nb and nB >= 128:
-            swap = True
-        elif inner in ma and mA >= 128:
-            swap = False
-        else:
-            swap = nB > mA
+        swap, rows, cols, kk, rhs = _contract_plan(subscripts, A, B, out)
         if swap:
-            A, B, ma, nb = B, A, nb, ma
-        pa = self._pack(A, ma, kk, fmt, "A")
-        pb = self._pack(B, nb, kk, fmt, "B")
-        self.run_gemm(subscripts, fmt, pa, pb, out, ma, nb, rhs, alpha, beta)
+            A, B = B, A
+        pa = self._pack(A, rows, kk, fmt, "A")
+        pb = self._pack(B, cols, kk, fmt, "B")
+        self.run_gemm(subscripts, fmt, pa, pb, out, rows, cols, rhs, alpha, beta)
         return out
 
     def run_gemm(self, subscripts, fmt, pa, pb, out, rows, cols, rhs, alpha, beta,
@@ -272,18 +330,16 @@ class TCEngine:
                                 "Kp": pa.Kp, "start": ev[0], "end": ev[1]})
 
     def _pack(self, op, rows, ks, fmt, side, row_tab=None, k_tab=None, k_w=None):
-        tabs = tuple(t.data_ptr() if t is not None else None for t in (row_tab, k_tab, k_w))
         if op.key is None:
             if self.dyn_cache is None:
                 return pack(op, rows, ks, fmt, self.stream, row_tab, k_tab, k_w)
             # the key is the gather itself: each source's address, and the extent and
             # per-source strides of every row and K index, so one matrix reached through
             # differently named labels is packed once
-            ext = op.extents()
-            src = tuple(s[0].data_ptr() if s is not None else None for s in op.sources())
-            geo = tuple((ext[c], tuple(op.strides(c))) for c in rows)
-            kgeo = tuple((ext[c], tuple(op.strides(c))) for c in ks)
-            dkey = (src, op.a, op.b, op.c, op.d, geo, kgeo, tabs, pack_format(fmt))
+            src = tuple([None if s is None else s[0].data_ptr() for s in op.sources()])
+            plan = pack_plan(op, rows, ks, row_tab, k_tab)
+            tabs = tuple([None if t is None else t.data_ptr() for t in (row_tab, k_tab, k_w)])
+            dkey = (src, op.a, op.b, op.c, op.d, plan.geo, tabs, pack_format(fmt))
             hit = self.dyn_cache.get(dkey)
             if hit is None:
                 # the entry holds its source tensors and tables, so no later tensor can reuse
