@@ -23,8 +23,8 @@
 // dot product in step 4, so non-finite inputs give what FP64 arithmetic gives.
 //
 // Measured on GB300 against the FP64 kernel (contract_f64.cu), no = 20, nv = 180: the ladder
-// 'ijef,abef->ijab' 882 -> 22.9 ms (GEMM 11.7, residues 9.8), a ring 'imae,mbej->ijab' 90.8 ->
-// 1.50 ms; at no = 9, nv = 53 3.2 -> 0.18 ms and 0.46 -> 0.09 ms.
+// 'ijef,abef->ijab' 882 -> 21.1 ms (GEMM 11.5, residues 8.1), a ring 'imae,mbej->ijab' 90.8 ->
+// 1.41 ms; at no = 9, nv = 53 3.2 -> 0.18 ms and 0.46 -> 0.09 ms.
 //
 // The offsets of strided rows, columns and K indices are expanded into tables once per call;
 // operands larger than the workspace go through in panels of rows, columns or K.
@@ -38,7 +38,8 @@ struct JoinArgs {
   Operand a, b;
   long long m0, n0, M, N;  // this panel's rows and columns
   long long k0, K;
-  int splits, log2k;
+  int splits;
+  int beta_zero, beta_one;
   long long ld;
   const unsigned char* res;  // [split][modulus][M][ld]
   double alpha, beta;
@@ -59,9 +60,10 @@ __device__ __noinline__ double plain_dot(const JoinArgs& p, long long row, long 
 
 // Four columns of one row per thread: for every modulus the residues times the three words of
 // floor(2^96 q / p) are summed in 64-bit accumulators (their integer part falls out modulo
-// 2^96), the signed fraction is rounded to FP64 and scaled.  Bound by the 64-bit multiply-adds
-// (3 NM per element) and, for short K, by the residues' and C's bytes.
-__global__ void __launch_bounds__(256) rns_join_kernel(const __grid_constant__ JoinArgs p) {
+// 2^96), the signed fraction is rounded to FP64 and scaled.  About 200 integer instructions and
+// two FP64 ones per output; four resident blocks hide the loads' latency.  At 13.0e6 outputs
+// 134 us, against 175 at 66 registers with each column's scale computed where it is read.
+__global__ void __launch_bounds__(256, 4) rns_join_kernel(const __grid_constant__ JoinArgs p) {
   const unsigned nc = (unsigned)((p.N + 3) >> 2);
   const unsigned total = (unsigned)(p.M * nc);  // below 2^31 (host check)
   const bool failed = *p.status != 0;
@@ -76,19 +78,23 @@ __global__ void __launch_bounds__(256) rns_join_kernel(const __grid_constant__ J
         w[l] = __ldg(reinterpret_cast<const unsigned*>(src + (long long)l * p.M * p.ld));
       sum.add(p.t, w);
     }
-    const long long grow = p.m0 + row;
-    const bool bad_row = p.a.top[grow] == 2047u;
-    const int sa = row_shift(p.a, grow, p.log2k);
+    const long long grow = p.m0 + row, gcol = p.n0 + col;  // gcol: a multiple of four
+    const int sa = p.a.sh[grow];
+    const int4 sb = *reinterpret_cast<const int4*>(p.b.sh + gcol);
+    const longlong2 o0 = *reinterpret_cast<const longlong2*>(p.b.coff + gcol);
+    const longlong2 o1 = *reinterpret_cast<const longlong2*>(p.b.coff + gcol + 2);
     double* crow = p.C + p.a.coff[grow];
+    const int sbe[4] = {sb.x, sb.y, sb.z, sb.w};
+    const long long off[4] = {o0.x, o0.y, o1.x, o1.y};
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       if (col + e >= p.N) break;
-      const long long gcol = p.n0 + col + e;
-      double v = sum.value(p.t, e, -sa - row_shift(p.b, gcol, p.log2k));
-      if (bad_row || p.b.top[gcol] == 2047u) v = p.alpha * plain_dot(p, grow, gcol);
+      double v = sum.value(p.t, e, -sa - sbe[e]);
+      if (sa == kNotFinite || sbe[e] == kNotFinite) v = p.alpha * plain_dot(p, grow, gcol + e);
       if (failed) v = __longlong_as_double(0x7ff8000000000000ll);
-      double* dst = crow + p.b.coff[gcol];
-      *dst = p.beta == 0.0 ? v : p.beta * *dst + v;
+      double* dst = crow + off[e];
+      if (!p.beta_zero) v = p.beta_one ? *dst + v : fma(p.beta, *dst, v);
+      *dst = v;
     }
   }
 }
@@ -120,7 +126,7 @@ bool size_plan(Plan& p, long long M, long long N, long long K) {
   splits = std::min(splits, 8);
   p.kb_per_split = (int)((nkb + splits - 1) / splits);
   p.splits = (int)((nkb + p.kb_per_split - 1) / p.kb_per_split);
-  p.tables = up((M + N) * (8 + 8 + 4 + 4 + 4) + 16 * K + 256, 256);
+  p.tables = up((M + N) * (8 + 8 + 4 + 4 + 4 + 4) + 16 * K + 256 + 14 * 16, 256);
   p.panel_a = up(p.PM * p.Kp * 2 * NM, 256);
   p.panel_b = up(p.PN * p.Kp * 2 * NM, 256);
   p.res = up((long long)p.splits * NM * p.PM * p.ld, 256);
@@ -244,9 +250,9 @@ extern "C" int pcg_contract_rns_f64(int m_n, const long long* m_ext, const long 
   // workspace: tables, panels of A and B, residues of the products
   unsigned char* w = (unsigned char*)work;
   unsigned char* tb = w;
-  auto take = [&](long long bytes) {
+  auto take = [&](long long bytes) {  // every array 16-byte aligned
     unsigned char* r = tb;
-    tb += bytes;
+    tb += up(bytes, 16);
     return r;
   };
   Operand a{}, b{};
@@ -263,6 +269,8 @@ extern "C" int pcg_contract_rns_f64(int m_n, const long long* m_ext, const long 
   b.top = (unsigned*)take(4 * N);
   a.norm2 = (float*)take(4 * M);
   b.norm2 = (float*)take(4 * N);
+  a.sh = (int*)take(4 * M);
+  b.sh = (int*)take(4 * N);
   __nv_bfloat16* pa = (__nv_bfloat16*)(w + p.tables);
   __nv_bfloat16* pb = (__nv_bfloat16*)(w + p.tables + p.panel_a);
   unsigned char* res = w + p.tables + p.panel_a + p.panel_b;
@@ -332,8 +340,9 @@ extern "C" int pcg_contract_rns_f64(int m_n, const long long* m_ext, const long 
                        : p.BN == 128 ? run_gemm<128, false>(maps, g, st)
                                      : run_gemm<64, false>(maps, g, st);
         if (rc) return rc;
-        JoinArgs j{a, b, m0, n0, mm, nn, k0, kn, p.splits, log2k, g.ld, res, alpha,
-                   k0 > 0 ? 1.0 : beta, C, status, crt_tab(p.splits, alpha)};
+        const double bt = k0 > 0 ? 1.0 : beta;
+        JoinArgs j{a, b, m0, n0, mm, nn, k0, kn, p.splits, bt == 0.0, bt == 1.0, g.ld, res, alpha,
+                   bt, C, status, crt_tab(p.splits, alpha)};
         rns_join_kernel<<<blocks_for(mm * ((nn + 3) / 4), 256), 256, 0, st>>>(j);
         PCG_CHECK_LAUNCH("pcg_contract_rns_f64/join");
       }

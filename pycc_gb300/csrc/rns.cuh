@@ -65,6 +65,8 @@ struct Operand {
   unsigned* top;        // [R] biased exponent of the row's largest |x| (2047: Inf or NaN)
   float* norm2;         // [R] sum of the row's squares, each term truncated to 20 bits
   const int* shift;     // one power of two for all rows, or null: each row its own
+  int* sh;              // [R] the rows' powers of two as the pack used them (kNotFinite: the row
+                        // holds an Inf or a NaN), or null
   const long long* k;   // [K] element offset of each K index in X
   long long kstep;      // > 0: k[i] = i * kstep
   int wq;               // sub-index that the walk has innermost
@@ -199,6 +201,8 @@ static __global__ void __launch_bounds__(256) rns_norm_kernel(const __grid_const
     norm_rows<false>(p.o[side], p.k0, p.k1, p.seg[side], bx, by);
 }
 
+constexpr int kNotFinite = 1 << 20;
+
 // Power of two s of a row: |x| 2^s has a 2-norm of at most 2^61.9.  From the sum of squares
 // where FP32 holds it (1 + 2^-7 covers its truncation and summation), else from the largest
 // element and K.  A zero row may take any.
@@ -217,26 +221,19 @@ __device__ __forceinline__ int row_shift(const Operand& o, long long row, int lo
 // The four digits (with the sign) of x 2^s rounded to an integer of at most 62 bits.
 __device__ __forceinline__ void digits(double x, int s, unsigned flip, float (&d)[4]) {
   const unsigned hi = (unsigned)__double2hiint(x) ^ flip, lo = (unsigned)__double2loint(x);
-  int ex = (int)((hi >> 20) & 0x7ffu);
-  unsigned long long m = ((unsigned long long)(hi & 0xfffffu) << 32) | lo;
-  if (ex)
-    m |= 1ull << 52;
-  else
-    ex = 1;
-  const int sh = ex - 1075 + s;  // at most 9, since |x| 2^s <= 2^61.9
-  if (ex == 2047)
-    m = 0;  // the row's outputs come from the FP64 dot product
-  else if (sh >= 0)
-    m <<= sh;
-  else if (sh > -55)
-    m = (m + (1ull << (-sh - 1))) >> -sh;
-  else
-    m = 0;
-  const unsigned sign = hi & 0x80000000u;
+  const unsigned ex = (hi >> 20) & 0x7ffu;
+  const unsigned mh = (hi & 0xfffffu) | (ex ? 1u << 20 : 0u);
+  // |x| 2^s = m 2^sh, sh = max(ex, 1) - 1075 + s at most 9 since |x| 2^s <= 2^61.9: shifted left
+  // by 9 - sh from 10 bits up, then rounded off by the last.  A shift past 63 leaves 0, as does
+  // the exponent of an infinity or a NaN, whose row takes its outputs from the FP64 dot product.
+  const unsigned r = min((unsigned)(9 + 1075 - s - (int)max(ex, 1u)), 63u);
+  unsigned long long m = (((unsigned long long)mh << 32) | lo) << 10;
+  m = ((m >> r) + 1ull) >> 1;
+  const float sign = __uint_as_float(0x3f800000u | (hi & 0x80000000u));
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     const unsigned v = (unsigned)(m >> digit_bit(q)) & ((1u << (digit_bit(q + 1) - digit_bit(q))) - 1);
-    d[q] = __uint_as_float(__float_as_uint(__uint_as_float(0x4b000000u | v) - 8388608.f) ^ sign);
+    d[q] = fmaf(__uint_as_float(0x4b000000u | v), sign, -8388608.f * sign);
   }
 }
 
@@ -255,64 +252,69 @@ struct PackArgs {
   ModTab t;
 };
 
-// Residues of two neighbouring K entries for every modulus, one 32-bit store per modulus: an
+// Residues of four neighbouring K entries for every modulus, one 64-bit store per modulus: an
 // integer of at most 8 bits is exact in the upper half of its FP32 word, which is BF16.
-__device__ __forceinline__ void store_residues(const PackArgs& p, const PackSide& o, double x0,
-                                               double x1, int s, long long at) {
-  float a[4], b[4];
-  digits(x0, s, o.flip, a);
-  digits(x1, s, o.flip, b);
-  unsigned* out = reinterpret_cast<unsigned*>(o.out + at);
-  const long long plane = (o.nrow * p.Kp) >> 1;
+__device__ __forceinline__ void store_residues(const PackArgs& p, const PackSide& o,
+                                               const double (&x)[4], int s, long long at) {
+  float d[4][4];
 #pragma unroll
-  for (int l = 0; l < NM; ++l) {
-    const float t0 = fmaf(a[3], p.t.c3[l], fmaf(a[2], p.t.c2[l], fmaf(a[1], p.t.c1[l], a[0])));
-    const float t1 = fmaf(b[3], p.t.c3[l], fmaf(b[2], p.t.c2[l], fmaf(b[1], p.t.c1[l], b[0])));
-    const float r0 = mod_near(t0, p.t.p[l], p.t.inv[l]), r1 = mod_near(t1, p.t.p[l], p.t.inv[l]);
-    out[l * plane] = __byte_perm(__float_as_uint(r0), __float_as_uint(r1), 0x7632);
+  for (int e = 0; e < 4; ++e) digits(x[e], s, o.flip, d[e]);
+  uint2* out = reinterpret_cast<uint2*>(o.out + at);
+  const long long plane = (o.nrow * p.Kp) >> 2;
+#pragma unroll
+  for (int l = 0; l < NM; ++l, out += plane) {
+    unsigned r[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float t = fmaf(d[e][3], p.t.c3[l],
+                           fmaf(d[e][2], p.t.c2[l], fmaf(d[e][1], p.t.c1[l], d[e][0])));
+      r[e] = __float_as_uint(mod_near(t, p.t.p[l], p.t.inv[l]));
+    }
+    *out = make_uint2(__byte_perm(r[0], r[1], 0x7632), __byte_perm(r[2], r[3], 0x7632));
   }
 }
 
-// Operand -> residues: 8 bytes read and 2 NM written per element, about 7 NM FP32
-// instructions; bound by the writes (9.8 ms at 1.05e9 elements, 4.3 of 6.8 TB/s).  Gathered along K, a
-// warp takes 64 K of a row, four rows at a time, straight from global memory.  Otherwise a tile
-// of 64 walked rows x 64 K goes through shared memory, read along the rows.  One launch packs a
-// panel of each operand: the first blocks take A's, the others B's.
-static __global__ void __launch_bounds__(256, 5) rns_pack_kernel(const __grid_constant__ PackArgs p) {
+// Operand -> residues: 8 bytes read and 2 NM written per element, about 150 instructions; bound
+// by the writes and, not far behind, by instruction issue.  A half warp takes 64 K of a row, four
+// neighbouring K a lane.  Gathered along K it loads them straight from global memory, two rows a
+// half warp; otherwise a tile of 64 walked rows x 64 K goes through shared memory, read along the
+// rows.  One launch packs a panel of each operand: the first blocks take A's, the others B's.
+// 8.1 ms at 1.05e9 elements (5.2 TB/s) against 9.5 with 250 instructions an element (two K a
+// lane, 64-bit tile indices, branches on the shift's sign).
+static __global__ void __launch_bounds__(256, 5)
+    rns_pack_kernel(const __grid_constant__ PackArgs p) {
   __shared__ double tile[64][65];
   __shared__ long long off[64], kof[64];
   __shared__ int srow[64], ssh[64];
   const int side = blockIdx.x >= p.s[0].blocks;
   const PackSide& ps = p.s[side];
   const Operand& o = ps.o;
-  const long long b = (long long)blockIdx.x - (side ? p.s[0].blocks : 0);
-  const long long nk = p.Kp >> 6;
-  const long long w = (b / nk) * (o.kfast ? 32 : 64);  // first row of the block
-  const long long kk0 = (b % nk) * 64;                 // first K, in the panel
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned b = blockIdx.x - (side ? (unsigned)p.s[0].blocks : 0u);
+  const unsigned nk = (unsigned)(p.Kp >> 6), bw = b / nk;
+  const long long w = (long long)bw * (o.kfast ? 32 : 64);  // first row of the block
+  const long long kk0 = (long long)(b - bw * nk) * 64;      // first K, in the panel
+  const int half = threadIdx.x >> 4, kk = 4 * (threadIdx.x & 15);
   if (o.kfast) {
-    const long long ka = kk0 + 2 * lane, kb = ka + 1;
-    const long long oa = ka < p.K ? k_offset(o, p.k0 + ka) : 0;
-    const long long ob = kb < p.K ? k_offset(o, p.k0 + kb) : 0;
-    const long long w1 = w + 4 * warp;
-    double x[4], y[4];
-    int row[4];
+    const long long w1 = w + 2 * half;
+    double x[2][4];
+    int row[2];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      x[u] = y[u] = 0.0;
-      row[u] = 0;
-      if (w1 + u < ps.nrow) {
-        row[u] = o.walk[ps.w0 + w1 + u];
-        const double* q = o.X + o.off[row[u]];
-        if (ka < p.K) x[u] = __ldg(q + oa);
-        if (kb < p.K) y[u] = __ldg(q + ob);
+    for (int u = 0; u < 2; ++u) {
+      row[u] = w1 + u < ps.nrow ? o.walk[ps.w0 + w1 + u] : -1;
+      const double* q = o.X + (row[u] >= 0 ? o.off[row[u]] : 0);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const long long k = kk0 + kk + e;
+        x[u][e] = row[u] >= 0 && k < p.K ? __ldg(q + k_offset(o, p.k0 + k)) : 0.0;
       }
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
-      if (w1 + u < ps.nrow)
-        store_residues(p, ps, x[u], y[u], row_shift(o, row[u], p.log2k),
-                       (row[u] - ps.w0) * p.Kp + kk0 + 2 * lane);
+    for (int u = 0; u < 2; ++u)
+      if (row[u] >= 0) {
+        const int sh = row_shift(o, row[u], p.log2k);
+        if (o.sh && kk0 + kk == 0) o.sh[row[u]] = o.top[row[u]] == 2047u ? kNotFinite : sh;
+        store_residues(p, ps, x[u], sh, (row[u] - ps.w0) * p.Kp + kk0 + kk);
+      }
   } else {
     if (threadIdx.x < 64) {
       kof[threadIdx.x] = kk0 + threadIdx.x < p.K ? k_offset(o, p.k0 + kk0 + threadIdx.x) : 0;
@@ -320,7 +322,9 @@ static __global__ void __launch_bounds__(256, 5) rns_pack_kernel(const __grid_co
         const int r = o.walk[ps.w0 + w + threadIdx.x];
         srow[threadIdx.x] = r;
         off[threadIdx.x] = o.off[r];
-        ssh[threadIdx.x] = row_shift(o, r, p.log2k);
+        const int sh = row_shift(o, r, p.log2k);
+        ssh[threadIdx.x] = sh;
+        if (o.sh && kk0 == 0) o.sh[r] = o.top[r] == 2047u ? kNotFinite : sh;
       }
     }
     __syncthreads();
@@ -335,9 +339,10 @@ static __global__ void __launch_bounds__(256, 5) rns_pack_kernel(const __grid_co
     for (int u = 0; u < 16; ++u) tile[rr][(threadIdx.x >> 6) + 4 * u] = v[u];
     __syncthreads();
 #pragma unroll 1
-    for (int r = warp; r < 64 && w + r < ps.nrow; r += 8)
-      store_residues(p, ps, tile[r][2 * lane], tile[r][2 * lane + 1], ssh[r],
-                     (srow[r] - ps.w0) * p.Kp + kk0 + 2 * lane);
+    for (int r = half; r < 64 && w + r < ps.nrow; r += 16) {
+      const double x[4] = {tile[r][kk], tile[r][kk + 1], tile[r][kk + 2], tile[r][kk + 3]};
+      store_residues(p, ps, x, ssh[r], (srow[r] - ps.w0) * p.Kp + kk0 + kk);
+    }
   }
 }
 
@@ -659,7 +664,7 @@ struct CrtSum {
     for (int l = 0; l < NM; ++l)
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const unsigned r = (w[l] >> (8 * e)) & 0xffu;
+        const unsigned r = __byte_perm(w[l], 0u, 0x4440u + e);
         s0[e] += (unsigned long long)r * t.c0[l];
         s1[e] += (unsigned long long)r * t.c1[l];
         s2[e] += (unsigned long long)r * t.c2[l];
@@ -693,7 +698,8 @@ struct CrtSum {
       v = __longlong_as_double(
               (long long)(m + ((unsigned long long)(1023 + 94 - lz + ex) << 52))) * t.scale;
     }
-    return neg ? -v : v;
+    return __longlong_as_double(__double_as_longlong(v) ^
+                                (neg ? (long long)0x8000000000000000ull : 0ll));
   }
 };
 
