@@ -187,6 +187,13 @@ int pcg_triples_energy(int fp32, const void* P1, const void* P2, const void* P3,
                        const void* eoovv, const double* t1, const void* t2,
                        const double* fov, long long no, long long nv, double* part,
                        void* stream);
+/* pcg_triples_energy(fp32 = 1) for partials P[ntrip][3][nv][nv][pitch] and eoovv, t2 of
+ * [no][no][nv][pitch], the pitch a multiple of four floats (16-byte aligned bases): tiles by TMA.  An expired device-side wait sets
+ * *status (device int) and makes its partial NaN. */
+int pcg_triples_energy_pitched(const float* P, long long pitch, const int* ijk, int ntrip,
+                               const double* eps, const float* eoovv, const double* t1,
+                               const float* t2, const double* fov, long long no, long long nv,
+                               double* part, int* status, void* stream);
 /* FP64 partials per triple written by pcg_triples_energy: nv (FP64), or the number of
  * 8^3 tile triples A >= B >= C of the virtual range (FP32).  (Sizing helper, no reference
  * counterpart.) */
@@ -298,6 +305,13 @@ int pcg_tc_grouped_gemm(int na, const void* const* a_ptr, const long long* a_row
                         const long long* b_rows, const long long* b_ld, const void* groups,
                         int ngroups, long long M, long long N, float* C, long long ldm,
                         long long ldn, int* status, void* stream);
+/* The same with row m of a group's output at (m / inner) * outer + m % inner: runs of `inner` rows
+ * with a pitch. */
+int pcg_tc_grouped_gemm_pitched(int na, const void* const* a_ptr, const long long* a_rows,
+                                const long long* a_ld, int nb, const void* const* b_ptr,
+                                const long long* b_rows, const long long* b_ld, const void* groups,
+                                int ngroups, long long M, long long N, float* C, long long inner,
+                                long long outer, long long ldn, int* status, void* stream);
 int pcg_tc_group_desc_size(void);
 
 #ifdef __cplusplus

@@ -76,6 +76,14 @@ __device__ __forceinline__ void tma_load_2d(const CUtensorMap* tm, uint64_t* bar
       "l"((unsigned long long)tm), "r"(smem_u32(bar)), "r"(x), "r"(y)
       : "memory");
 }
+__device__ __forceinline__ void tma_load_4d(const CUtensorMap* tm, uint64_t* bar, void* dst, int x,
+                                            int y, int z, int w) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, "
+      "%4, %5, %6}], [%2];" ::"r"(smem_u32(dst)),
+      "l"((unsigned long long)tm), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z), "r"(w)
+      : "memory");
+}
 // K-major operand tile, 128-byte swizzle, 8-row groups 1024 B apart (sm_100 descriptor).
 __device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr) {
   uint64_t d = 0;
@@ -164,6 +172,9 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
 // host helpers (tc_gemm.cu)
 bool make_map(CUtensorMap* m, const void* base, long long rows, long long ld_bytes,
               long long k_bytes, int elem_bytes, int box_rows);
+// boxes of 8 x 8 x 8 floats of [slabs][n][n][pitch] FP32, n valid columns, zeros beyond n
+bool make_map_cube8(CUtensorMap* m, const float* base, long long n, long long pitch,
+                    long long slabs);
 int num_sms();
 
 }  // namespace tc

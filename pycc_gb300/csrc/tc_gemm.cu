@@ -852,6 +852,27 @@ bool make_map(CUtensorMap* m, const void* base, long long rows, long long ld_byt
   return true;
 }
 
+bool make_map_cube8(CUtensorMap* m, const float* base, long long n, long long pitch,
+                    long long slabs) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) {
+    set_error("cuTensorMapEncodeTiled unavailable");
+    return false;
+  }
+  cuuint64_t dims[4] = {(cuuint64_t)n, (cuuint64_t)n, (cuuint64_t)n, (cuuint64_t)slabs};
+  cuuint64_t strides[3] = {(cuuint64_t)(4 * pitch), (cuuint64_t)(4 * pitch * n),
+                           (cuuint64_t)(4 * pitch * n * n)};
+  cuuint32_t box[4] = {8, 8, 8, 1}, estr[4] = {1, 1, 1, 1};
+  CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float*>(base), dims, strides,
+                  box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                  CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    set_error("cuTensorMapEncodeTiled failed (%d)", (int)r);
+    return false;
+  }
+  return true;
+}
+
 int num_sms() {
   static int sms = 0;
   if (!sms) {

@@ -38,11 +38,35 @@ struct GArgs {
   const GroupDesc* groups;
   int ngroups;
   long long M, N, ldm, ldn;
+  unsigned inner;   // row m goes to (m / inner) * outer + (m % inner) * ldm
+  long long outer;
   long long mt, nt;
   float* C;
   int* status;
   unsigned long long wait_ns;  // bound on any single device-side wait
 };
+
+// Unit u -> group and tile, and the group's descriptor.  Each role loads the descriptor of its
+// next unit before it works on the present one, and the division is a 32-bit one: a unit is six
+// K blocks at K = 121 + 15 twice (0.8 us of MMA), and with its descriptor's loads and a 64-bit
+// division in the producing thread it took 3.9 us, 3.1 now (bound by the epilogue's stores, 3.1
+// TB/s).
+struct GUnit {
+  GroupDesc g;
+  unsigned group, m, n;
+};
+
+__device__ __forceinline__ GUnit load_unit(const GArgs& p, unsigned u, unsigned nunits) {
+  GUnit x;
+  const unsigned nt = (unsigned)p.nt, per = (unsigned)p.mt * nt;
+  if (u >= nunits) u = nunits - 1;
+  x.group = u / per;
+  const unsigned r = u - x.group * per;
+  x.m = r / nt;
+  x.n = r - x.m * nt;
+  x.g = p.groups[x.group];
+  return x;
+}
 
 template <int BN>
 struct GSmem {
@@ -77,8 +101,7 @@ __global__ void __launch_bounds__(GROUPED_THREADS, 1)
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const long long per = p.mt * p.nt;
-  const long long nunits = per * p.ngroups;
+  const unsigned nunits = (unsigned)(p.mt * p.nt * p.ngroups);  // below 2^31 (host check)
 
   if (tid == 0) {
     for (int s = 0; s < S; ++s) {
@@ -108,11 +131,15 @@ __global__ void __launch_bounds__(GROUPED_THREADS, 1)
     if (lane == 0) {
       int it = 0;
       bool stop = false;
-      for (long long u = blockIdx.x; u < nunits && !stop; u += gridDim.x) {
-        const GroupDesc& g = p.groups[u / per];
-        const long long r = u % per;
-        const int m0 = (int)((r / p.nt) * BM), n0 = (int)((r % p.nt) * BN);
-        for (int s = 0; s < g.nseg && !stop; ++s) {
+      GUnit next = load_unit(p, blockIdx.x, nunits);
+      for (unsigned u = blockIdx.x; u < nunits && !stop; u += gridDim.x) {
+        const GUnit x = next;
+        const GroupDesc& g = x.g;
+        next = load_unit(p, u + gridDim.x, nunits);
+        const int m0 = (int)(x.m * BM), n0 = (int)(x.n * BN);
+#pragma unroll
+        for (int s = 0; s < kMaxSeg; ++s) {
+          if (s >= g.nseg || stop) break;
           const CUtensorMap* ta = &maps.a[g.amap[s]];
           const CUtensorMap* tb = &maps.b[g.bmap[s]];
           for (int kb = 0; kb < g.nkb[s]; ++kb, ++it) {
@@ -142,8 +169,11 @@ __global__ void __launch_bounds__(GROUPED_THREADS, 1)
                              ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
       int it = 0, ui = 0;
       bool stop = false;
-      for (long long u = blockIdx.x; u < nunits && !stop; u += gridDim.x, ++ui) {
-        const GroupDesc& g = p.groups[u / per];
+      GUnit next = load_unit(p, blockIdx.x, nunits);
+      for (unsigned u = blockIdx.x; u < nunits && !stop; u += gridDim.x, ++ui) {
+        const GUnit x = next;
+        const GroupDesc& g = x.g;
+        next = load_unit(p, u + gridDim.x, nunits);
         const int b = ui & 1;
         if (ui >= 2 && !mbar_wait(&tempty[b], ((ui >> 1) - 1) & 1, p.wait_ns)) {
           atomicExch(p.status, kStatusTimeoutEmpty);
@@ -153,7 +183,9 @@ __global__ void __launch_bounds__(GROUPED_THREADS, 1)
         tc_fence_after();
         const uint32_t d = tmem + (uint32_t)(b * BN);
         uint32_t acc = 0u;
-        for (int s = 0; s < g.nseg && !stop; ++s) {
+#pragma unroll
+        for (int s = 0; s < kMaxSeg; ++s) {
+          if (s >= g.nseg || stop) break;
           for (int kb = 0; kb < g.nkb[s]; ++kb, ++it) {
             const int st = it % S;
             if (!mbar_wait(&full[st], (it / S) & 1, p.wait_ns)) {
@@ -187,10 +219,11 @@ __global__ void __launch_bounds__(GROUPED_THREADS, 1)
                                     // block split 16 / 16 (loads start at their width)
     constexpr int NFULL = BN / 64;
     int ui = 0;
-    for (long long u = blockIdx.x; u < nunits; u += gridDim.x, ++ui) {
-      const GroupDesc& g = p.groups[u / per];
-      const long long r = u % per;
-      const long long m0 = (r / p.nt) * BM, n0 = (r % p.nt) * BN;
+    GUnit next = load_unit(p, blockIdx.x, nunits);
+    for (unsigned u = blockIdx.x; u < nunits; u += gridDim.x, ++ui) {
+      const GUnit x = next;
+      next = load_unit(p, u + gridDim.x, nunits);
+      const long long m0 = (long long)x.m * BM, n0 = (long long)x.n * BN;
       const int b = ui & 1;
       int okw = 1;
       if (lane == 0) {
@@ -205,17 +238,25 @@ __global__ void __launch_bounds__(GROUPED_THREADS, 1)
       tc_fence_after();
       const long long row = m0 + q * 32 + lane;
       const bool row_ok = row < p.M;
-      float* crow = p.C + g.out + row * p.ldm;
+      const unsigned ro = (unsigned)row / p.inner;
+      float* crow = p.C + x.g.out + ro * p.outer + ((unsigned)row - ro * p.inner) * p.ldm;
       const uint32_t tb = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * BN);
 #pragma unroll 1
       for (int fb = 0; fb < NFULL; ++fb) {
         const int c0 = 32 * (2 * fb + h);
+        const int left = (int)min(32LL, p.N - n0 - c0);  // columns of the output in this block
+        if (left <= 0) break;
         uint32_t v[32];
         tmem_ld32(tb + c0, v);
-        if (row_ok)
+        float* c = crow + (n0 + c0) * p.ldn;
+        if (row_ok && left == 32) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j)
-            if (n0 + c0 + j < p.N) crow[(n0 + c0 + j) * p.ldn] = __uint_as_float(v[j]);
+          for (int j = 0; j < 32; ++j, c += p.ldn) *c = __uint_as_float(v[j]);
+        } else if (row_ok) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j, c += p.ldn)
+            if (j < left) *c = __uint_as_float(v[j]);
+        }
       }
       if constexpr (BN % 64 != 0) {
         const int c0 = BN - 32 + 16 * h;
@@ -262,31 +303,30 @@ int glaunch(const GMaps& maps, GArgs a, cudaStream_t st) {
 using namespace pcg;
 using namespace pcg::tc;
 
-// Grouped segmented BF16 GEMM, FP32 output (see the top of this file).  a_ptr / b_ptr: up
-// to four BF16 operand matrices each ([a_rows[q]][a_ld[q]] K-major, 16-byte aligned rows,
-// K a multiple of 64); groups: device array of ngroups GroupDesc records (nseg, amap[4],
-// arow[4], bmap[4], brow[4], nkb[4], out) as laid out in this file; element (m, n) of group
-// g goes to C[out_g + m*ldm + n*ldn].
-extern "C" int pcg_tc_grouped_gemm(int na, const void* const* a_ptr, const long long* a_rows,
-                                   const long long* a_ld, int nb, const void* const* b_ptr,
-                                   const long long* b_rows, const long long* b_ld,
-                                   const void* groups, int ngroups, long long M, long long N,
-                                   float* C, long long ldm, long long ldn, int* status,
-                                   void* stream) {
+namespace {
+int grouped_gemm(int na, const void* const* a_ptr, const long long* a_rows, const long long* a_ld,
+                 int nb, const void* const* b_ptr, const long long* b_rows, const long long* b_ld,
+                 const void* groups, int ngroups, long long M, long long N, float* C, long long ldm,
+                 long long inner, long long outer, long long ldn, int* status, void* stream,
+                 const char* who) {
   if (na < 1 || na > 4 || nb < 1 || nb > 4 || !groups || ngroups < 1 || M < 1 || N < 1 || !C ||
       !status || ldm < 1 || ldn < 1 || M > 0x7fffffffLL || N > 0x7fffffffLL || !a_ptr ||
       !a_rows || !a_ld || !b_ptr || !b_rows || !b_ld) {
-    set_error("pcg_tc_grouped_gemm: bad arguments");
+    set_error("%s: bad arguments", who);
     return -1;
   }
   GMaps maps;
   for (int q = 0; q < 4; ++q) {
     const int qa = q < na ? q : 0, qb = q < nb ? q : 0;
     if (!a_ptr[qa] || !b_ptr[qb] || (a_ld[qa] * 2) % 16 || (b_ld[qb] * 2) % 16) {
-      set_error("pcg_tc_grouped_gemm: operand %d not 16-byte aligned", q);
+      set_error("%s: operand %d not 16-byte aligned", who, q);
       return -1;
     }
     if (!make_map(&maps.a[q], a_ptr[qa], a_rows[qa], a_ld[qa] * 2, a_ld[qa] * 2, 2, BM)) return -1;
+  }
+  if ((M + BM - 1) / BM * ((N + 63) / 64) > 0x7fffffffLL / ngroups) {
+    set_error("%s: too many tiles", who);
+    return -1;
   }
   const int BN = (N <= 64) ? 64 : (N <= 128 ? 128 : (N <= 160 ? 160 : 256));
   for (int q = 0; q < 4; ++q) {
@@ -300,6 +340,8 @@ extern "C" int pcg_tc_grouped_gemm(int na, const void* const* a_ptr, const long 
   a.N = N;
   a.ldm = ldm;
   a.ldn = ldn;
+  a.inner = (unsigned)inner;
+  a.outer = outer;
   a.mt = (M + BM - 1) / BM;
   a.C = C;
   a.status = status;
@@ -311,6 +353,40 @@ extern "C" int pcg_tc_grouped_gemm(int na, const void* const* a_ptr, const long 
     case 160: return glaunch<160>(maps, a, st);
     default: return glaunch<256>(maps, a, st);
   }
+}
+
+}  // namespace
+
+// Grouped segmented BF16 GEMM, FP32 output (see the top of this file).  a_ptr / b_ptr: up
+// to four BF16 operand matrices each ([a_rows[q]][a_ld[q]] K-major, 16-byte aligned rows,
+// K a multiple of 64); groups: device array of ngroups GroupDesc records (nseg, amap[4],
+// arow[4], bmap[4], brow[4], nkb[4], out) as laid out in this file; element (m, n) of group
+// g goes to C[out_g + m*ldm + n*ldn].
+extern "C" int pcg_tc_grouped_gemm(int na, const void* const* a_ptr, const long long* a_rows,
+                                   const long long* a_ld, int nb, const void* const* b_ptr,
+                                   const long long* b_rows, const long long* b_ld,
+                                   const void* groups, int ngroups, long long M, long long N,
+                                   float* C, long long ldm, long long ldn, int* status,
+                                   void* stream) {
+  return grouped_gemm(na, a_ptr, a_rows, a_ld, nb, b_ptr, b_rows, b_ld, groups, ngroups, M, N, C,
+                      ldm, M, 0, ldn, status, stream, "pcg_tc_grouped_gemm");
+}
+
+// The same with rows in runs: row m goes to (m / inner) * outer + m % inner, so that the rows
+// (x, y) of a partial tensor can have a pitch of their own.
+extern "C" int pcg_tc_grouped_gemm_pitched(int na, const void* const* a_ptr,
+                                           const long long* a_rows, const long long* a_ld, int nb,
+                                           const void* const* b_ptr, const long long* b_rows,
+                                           const long long* b_ld, const void* groups, int ngroups,
+                                           long long M, long long N, float* C, long long inner,
+                                           long long outer, long long ldn, int* status,
+                                           void* stream) {
+  if (inner < 1 || inner > 0x7fffffffLL || outer < inner) {
+    set_error("pcg_tc_grouped_gemm_pitched: bad row runs (%lld, %lld)", inner, outer);
+    return -1;
+  }
+  return grouped_gemm(na, a_ptr, a_rows, a_ld, nb, b_ptr, b_rows, b_ld, groups, ngroups, M, N, C,
+                      1, inner, outer, ldn, status, stream, "pcg_tc_grouped_gemm_pitched");
 }
 
 // Size of one GroupDesc record in bytes (for hosts that build the table).

@@ -11,7 +11,7 @@
 // The Lee-Rendell energy of the reference (pycc/cctriples.py:177-240) is then evaluated
 // for a >= b >= c with the same weights; one block per (triple, a), one FP64 partial per
 // block (deterministic reduction by pcg_reduce_sum_f64).
-#include "common.cuh"
+#include "tc_common.cuh"
 #include <algorithm>
 
 namespace pcg {
@@ -350,6 +350,186 @@ long long tile_triples(long long nv) {
   return nt * (nt + 1) * (nt + 2) / 6;
 }
 
+// ---- FP32 path, partials with a 16-byte pitch: tiles by TMA ------------------------------
+// One block per (triple, tile triple A >= B >= C) as above, but the six orderings of the tile
+// sets of each partial arrive as 8 x 8 x 8 boxes by TMA (18 boxes of 2 KB, zeros beyond nv) and W is
+// summed where it is used.  The 8 x 8 blocks of integrals and amplitudes are the threads' own loads:
+// 36 more small copies by TMA, which takes 2.6 clocks for a 32-byte row, made the kernel 15 % slower.  The staging of the kernel above cost about 500 instructions a thread
+// and, at a pitch that is no multiple of 32 bytes, two sectors for each 32-byte run; what bounds
+// this one is shared-memory reads, so a warp takes 2 x 4 x 4 elements (a, b, c), which keeps the
+// boxes' 256-byte slices at two to four reads to a bank.
+// At nv = 121, 32 triples: 260 us against 400.
+struct CubeArgs {
+  const int* ijk;      // [ntrip][3]
+  const double* eps;   // [nmo]
+  const float *eoovv, *t2;  // <ij|ab> and t2, [o][o][v][pitch]
+  long long pitch;
+  const double* t1;    // [o][v]
+  const double* fov;   // [o][v] or null (canonical)
+  int no, nv;
+  unsigned ntt;
+  double* part;        // [ntrip][ntt]
+  int* status;
+  unsigned long long wait_ns;
+};
+
+// ordered pairs of the tile sets A, B, C (0, 1, 2): AB, AC, BA, BC, CA, CB
+__host__ __device__ constexpr int pair_first(int q) { return q >> 1; }
+__host__ __device__ constexpr int pair_second(int q) { return (q >> 1) == 0 ? 1 + (q & 1) : ((q & 1) ? 3 - (q >> 1) : 0); }
+
+template <bool FOV>
+struct CubeStage {
+  float box[3][6][TT * TT * TT];      // partial, ordering of (slow, middle, fast) as kord
+  float e[3][6][TT][TT];              // <ij|..>, <ik|..>, <jk|..> over the ordered pairs
+  float d2[FOV ? 3 : 1][FOV ? 6 : 1][TT][TT];
+  float t1r[3][TT3], fr[3][TT3];      // t1 and f_ov of i, j, k over the union
+  float ev[TT3];
+  double red[TE2_THREADS / 32];
+  uint64_t bar;
+  int ok;
+};
+
+template <bool FOV>
+__global__ void __launch_bounds__(TE2_THREADS, 4)
+    triples_energy_cube_kernel(const __grid_constant__ CUtensorMap map, const CubeArgs p) {
+  __shared__ __align__(128) CubeStage<FOV> s;
+  const int t = blockIdx.y, tid = threadIdx.x;
+  const int v = p.nv;
+  const int i = p.ijk[3 * t], j = p.ijk[3 * t + 1], k = p.ijk[3 * t + 2];
+  int org[3];
+  {  // tile triple blockIdx.x -> A >= B >= C, 32-bit (nv^3 < 2^31)
+    const unsigned u = blockIdx.x;
+    auto tet = [](unsigned a) { return a * (a + 1) * (a + 2) / 6; };
+    auto tri = [](unsigned b) { return b * (b + 1) / 2; };
+    unsigned a = (unsigned)cbrtf(6.0f * (float)u);
+    while (a > 0 && tet(a) > u) --a;
+    while (tet(a + 1) <= u) ++a;
+    const unsigned r = u - tet(a);
+    unsigned b = (unsigned)((sqrtf(8.0f * (float)r + 1.0f) - 1.0f) * 0.5f);
+    while (b > 0 && tri(b) > r) --b;
+    while (tri(b + 1) <= r) ++b;
+    org[0] = (int)a * TT;
+    org[1] = (int)b * TT;
+    org[2] = (int)(r - tri(b)) * TT;
+  }
+  if (tid == 0) {
+    tc::mbar_init(&s.bar, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    tc::mbar_expect_tx(&s.bar, 18 * TT * TT * TT * 4);
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+#pragma unroll
+      for (int o = 0; o < 6; ++o)
+        tc::tma_load_4d(&map, &s.bar, s.box[q][o], org[kord(o, 2)], org[kord(o, 1)],
+                        org[kord(o, 0)], 3 * t + q);
+  }
+  {
+    // the 3 x 6 blocks of 8 x 8, a 64-thread group each: of the ordered pair sp of tile sets in
+    // matrix pr (ij, ik, jk)
+    const int r = (tid / TT) % TT, c = tid % TT, grp = tid / (TT * TT);
+#pragma unroll
+    for (int rep = 0; rep < 5; ++rep) {
+      const int x = 4 * rep + grp;
+      if (x < 18) {
+        const int pr = x / 6, sp = x - 6 * pr, f = sp >> 1, g = pair_second(sp);
+        const int row = (f == 0 ? org[0] : (f == 1 ? org[1] : org[2])) + r;
+        const int col = (g == 0 ? org[0] : (g == 1 ? org[1] : org[2])) + c;
+        const unsigned slab = (unsigned)((pr == 2 ? j : i) * p.no + (pr == 0 ? j : k));
+        const bool in = row < v && col < v;
+        const long long at = (long long)(slab * (unsigned)v + row) * p.pitch + col;
+        s.e[pr][sp][r][c] = in ? __ldg(p.eoovv + at) : 0.f;
+        if (FOV) s.d2[pr][sp][r][c] = in ? __ldg(p.t2 + at) : 0.f;
+      }
+    }
+  }
+  if (tid < 3 * TT3) {
+    const int q = tid / TT3, l = tid % TT3;
+    const int x = (l < TT ? org[0] : (l < 2 * TT ? org[1] : org[2])) + l % TT;
+    const int occ = q == 0 ? i : (q == 1 ? j : k);
+    s.t1r[q][l] = x < v ? f64_to_f32(p.t1[(long long)occ * v + x]) : 0.f;
+    if (FOV) s.fr[q][l] = x < v ? f64_to_f32(p.fov[(long long)occ * v + x]) : 0.f;
+    if (q == 0) s.ev[l] = x < v ? f64_to_f32(p.eps[p.no + x]) : 0.f;
+  }
+  if (tid == 0) {
+    const bool ok = tc::mbar_wait(&s.bar, 0, p.wait_ns);
+    if (!ok) {
+      atomicExch(p.status, kStatusTimeoutFull);
+      tc::mbar_wait(&s.bar, 0, p.wait_ns);  // the copies in flight, again with a limit
+    }
+    s.ok = ok;
+  }
+  __syncthreads();
+  if (!s.ok) {
+    if (tid == 0) p.part[(long long)t * p.ntt + blockIdx.x] = __longlong_as_double(0x7ff8000000000000ll);
+    return;
+  }
+  // the TMA's writes: every thread observes the completed phase itself
+  tc::mbar_wait(&s.bar, 0, p.wait_ns);
+  const int lane = tid & 31, warp = tid >> 5;
+  const int bl = ((lane >> 2) & 3) | (((warp >> 1) & 1) << 2), cl = (lane & 3) | ((warp >> 2) << 2);
+  const int b = org[1] + bl, c = org[2] + cl;
+  // of (b, c), shared by the thread's elements: <..|bc>, <..|cb>, t1, f and their products
+  float acc = 0.f;
+  const float eo = f64_to_f32(p.eps[i] + p.eps[j] + p.eps[k]);
+  auto lin = [](int o, int la, int lb, int lc) {  // place of (la, lb, lc) in a box of ordering o
+    const int st[3] = {TT * TT, TT, 1};
+    int at = 0;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      const int set = kord(o, q);
+      at += st[q] * (set == 0 ? la : (set == 1 ? lb : lc));
+    }
+    return at;
+  };
+#pragma unroll
+  for (int rep = 0; rep < 2; ++rep) {
+    const int al = (lane >> 4) | (rep << 1) | ((warp & 1) << 2);
+    const int a = org[0] + al;
+    if (a >= v || b > a || c > b) continue;
+    int at[6];
+#pragma unroll
+    for (int o = 0; o < 6; ++o) at[o] = lin(o, al, bl, cl);
+    // W[x, y, z] = P3[x][y][z] + P2[y][x][z] + P1[z][x][y] for the orderings of (a, b, c); the
+    // orderings of the boxes' (slow, middle, fast) per ordering of W
+    constexpr int o2[6] = {2, 4, 0, 5, 1, 3}, o1[6] = {4, 2, 5, 0, 3, 1};
+    const int loc[3] = {al, bl, cl};
+    float W[6], V[6];
+    const float wt = (float)(1 + (a == b) + (a == c) + (b == c));
+    const float rw = 1.f / wt;
+#pragma unroll
+    for (int o = 0; o < 6; ++o) {
+      W[o] = s.box[2][o][at[o]] + s.box[1][o2[o]][at[o2[o]]] + s.box[0][o1[o]][at[o1[o]]];
+      const int X = kord(o, 0), Y = kord(o, 1), Z = kord(o, 2);
+      auto pr = [](int f, int g) { return 2 * f + (f == 0 ? g - 1 : (f == 1 ? (g == 2) : g)); };
+      const int lx = loc[X], ly = loc[Y], lz = loc[Z];
+      const int ux = X * TT + lx, uy = Y * TT + ly, uz = Z * TT + lz;
+      float d = s.e[0][pr(X, Y)][lx][ly] * s.t1r[2][uz] + s.e[1][pr(X, Z)][lx][lz] * s.t1r[1][uy] +
+                s.e[2][pr(Y, Z)][ly][lz] * s.t1r[0][ux];
+      if (FOV)
+        d += s.d2[0][pr(X, Y)][lx][ly] * s.fr[2][uz] + s.d2[1][pr(X, Z)][lx][lz] * s.fr[1][uy] +
+             s.d2[2][pr(Y, Z)][ly][lz] * s.fr[0][ux];
+      V[o] = (W[o] + d) * rw;
+    }
+    float X = 0.f;
+#pragma unroll
+    for (int q = 0; q < 6; ++q) X += W[q] * V[q];
+    const float Y = V[0] + V[3] + V[4], Z = V[1] + V[2] + V[5];
+    const float Wc = W[0] + W[3] + W[4], Wa = W[1] + W[2] + W[5];
+    const float S = (Y - 2.f * Z) * Wc + (Z - 2.f * Y) * Wa + 3.f * X;
+    const float D = eo - s.ev[al] - s.ev[TT + bl] - s.ev[2 * TT + cl];
+    acc += S / D;
+  }
+  for (int sh = 16; sh > 0; sh >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, sh);
+  if (lane == 0) s.red[warp] = f32_to_f64(acc);
+  __syncthreads();
+  if (tid == 0) {
+    double r = 0.0;
+    for (int q = 0; q < TE2_THREADS / 32; ++q) r += s.red[q];
+    const double fac = 2.0 - ((i == j) + (i == k) + (j == k));
+    p.part[(long long)t * p.ntt + blockIdx.x] = fac * r;
+  }
+}
+
 __global__ void reduce_sum_kernel(const double* x, long long n, double* out) {
   __shared__ double red[TE_THREADS / 32];
   double acc = 0.0;
@@ -406,6 +586,37 @@ extern "C" int pcg_triples_energy(int fp32, const void* P1, const void* P2, cons
     triples_energy_kernel<double><<<grid, TE_THREADS, 0, st>>>(a);
   }
   PCG_CHECK_LAUNCH("pcg_triples_energy");
+  return 0;
+}
+
+// The FP32 path with the partials P[triple][orientation][nv][nv][pitch] and eoovv, t2 of
+// [o][o][nv][pitch], pitch a multiple of four floats (16 bytes): the partials' tiles come by TMA.  *status: a device word that an expired wait sets (the
+// partial is NaN then).  Partials as pcg_triples_energy(fp32 = 1) writes them.
+extern "C" int pcg_triples_energy_pitched(const float* P, long long pitch, const int* ijk, int ntrip,
+                                          const double* eps, const float* eoovv, const double* t1,
+                                          const float* t2, const double* fov, long long no,
+                                          long long nv, double* part, int* status, void* stream) {
+  if (!P || !ijk || !eps || !eoovv || !t1 || !t2 || !part || !status || ntrip < 1 || ntrip > 65535 ||
+      no < 1 || nv < 1 || pitch < nv || pitch % 4 != 0 ||
+      (((uintptr_t)P | (uintptr_t)eoovv | (uintptr_t)t2) & 15u)) {
+    set_error("pcg_triples_energy_pitched: bad arguments (ntrip=%d, pitch=%lld)", ntrip, pitch);
+    return -1;
+  }
+  const long long ntt = tile_triples(nv);
+  if (ntt > 0x7fffffffLL || nv * nv * nv > 0x7fffffffLL) {
+    set_error("pcg_triples_energy_pitched: nv=%lld too large", nv);
+    return -1;
+  }
+  CUtensorMap map;
+  if (!tc::make_map_cube8(&map, P, nv, pitch, 3LL * ntrip)) return -1;
+  CubeArgs a{ijk, eps, eoovv, t2, pitch, t1, fov, (int)no, (int)nv, (unsigned)ntt, part, status,
+             wait_limit_ns()};
+  const dim3 grid((unsigned)ntt, (unsigned)ntrip);
+  if (fov)
+    triples_energy_cube_kernel<true><<<grid, TE2_THREADS, 0, (cudaStream_t)stream>>>(map, a);
+  else
+    triples_energy_cube_kernel<false><<<grid, TE2_THREADS, 0, (cudaStream_t)stream>>>(map, a);
+  PCG_CHECK_LAUNCH("pcg_triples_energy_pitched");
   return 0;
 }
 

@@ -38,12 +38,17 @@ T2P, OB = 0, 1
 class TriplesTC:
     """Packed (T) operands for one set of amplitudes, and the batched driver."""
 
+    pitch = None      # elements between the partials' rows (None: nv)
+
     def __init__(self, w, t1, t2, batch=32):
         self.w = w
         no, nv = w.no, w.nv
         o, v = w.o, w.v
         self.no, self.nv = no, nv
         self.batch = batch
+        if t2.is_cuda:
+            # whole 32-byte sectors: the energy kernel takes its tiles by TMA, in rows of eight
+            self.pitch = -(-nv // 8) * 8
         self.t1 = t1.contiguous()
         self.t2 = t2.contiguous()
         V = w.H.ERI[v, v, v, o]          # <pq|ex>
@@ -69,7 +74,7 @@ class TriplesTC:
     def groups(self, trips):
         """GroupDesc records of the three orientations of every triple (numpy, vectorised)."""
         no, nv = self.no, self.nv
-        v2, v3 = nv * nv, nv ** 3
+        v2, pitch = nv * nv, self.pitch or nv
         kv, ko = self.nkb_v, self.nkb_o
         tr = np.asarray(trips, dtype=np.int64).reshape(-1, 3)
         i, j, k = tr[:, 0], tr[:, 1], tr[:, 2]
@@ -98,7 +103,7 @@ class TriplesTC:
                 r["bmap"][:, s] = bm
                 r["brow"][:, s] = brow
                 r["nkb"][:, s] = nk
-            r["out"] = (3 * (t % self.batch) + q) * v3
+            r["out"] = (3 * (t % self.batch) + q) * v2 * pitch
         return g
 
     def energy(self):
@@ -106,7 +111,8 @@ class TriplesTC:
         dev = self.t2.device
         trips = triples_list(no)
         nb = self.batch
-        P = torch.empty((nb, 3, nv, nv, nv), dtype=torch.float32, device=dev)
+        pitch = self.pitch or nv
+        P = torch.empty((nb, 3, nv, nv, pitch), dtype=torch.float32, device=dev)
         plen = int(_lib.load().pcg_triples_part_len(1, nv))
         part = torch.empty((nb, plen), dtype=torch.float64, device=dev)   # one batch
         out = torch.zeros((), dtype=torch.float64, device=dev)
@@ -123,20 +129,31 @@ class TriplesTC:
         o, v = w.o, w.v
         fov = H.F[o, v].contiguous()
         fov_ptr = fov.data_ptr() if bool(fov.abs().max() > 0) else None
-        eoovv = H.ERI[o, o, v, v].float()          # the FP32 energy kernel's copies
-        t2f = self.t2.float()
+        # the FP32 energy kernel's copies, at the partials' pitch
+        eoovv, t2f = (torch.empty((no, no, nv, pitch), dtype=torch.float32, device=dev)
+                      for _ in range(2))
+        eoovv[..., :nv].copy_(H.ERI[o, o, v, v])
+        t2f[..., :nv].copy_(self.t2)
         # every batch's group records, uploaded once; a batch's partials start at P[0]
         gall = torch.from_numpy(self.groups(trips).view(np.uint8)).to(dev)
         gsz = GROUP_DTYPE.itemsize
         for b0 in range(0, len(trips), nb):
             chunk = trips[b0:b0 + nb]
-            _lib.call("pcg_tc_grouped_gemm", 4, a_ptr, a_rows, a_ld, 2, b_ptr, b_rows, b_ld,
-                      gall.data_ptr() + 3 * b0 * gsz, 3 * len(chunk), nv * nv, nv,
-                      P.data_ptr(), 1, nv * nv, self.status.data_ptr(), st)
-            _lib.call("pcg_triples_energy", 1, P.data_ptr(), P[:, 1].data_ptr(),
-                      P[:, 2].data_ptr(), 3 * nv ** 3, ijk_all[b0:].data_ptr(), len(chunk),
-                      H.eps.data_ptr(), eoovv.data_ptr(), self.t1.data_ptr(), t2f.data_ptr(),
-                      fov_ptr, no, nv, part.data_ptr(), st)
+            gemm = (4, a_ptr, a_rows, a_ld, 2, b_ptr, b_rows, b_ld,
+                    gall.data_ptr() + 3 * b0 * gsz, 3 * len(chunk), nv * nv, nv, P.data_ptr())
+            if P.is_cuda:
+                _lib.call("pcg_tc_grouped_gemm_pitched", *gemm, nv, pitch, nv * pitch,
+                          self.status.data_ptr(), st)
+                _lib.call("pcg_triples_energy_pitched", P.data_ptr(), pitch,
+                          ijk_all[b0:].data_ptr(), len(chunk), H.eps.data_ptr(),
+                          eoovv.data_ptr(), self.t1.data_ptr(), t2f.data_ptr(), fov_ptr, no, nv,
+                          part.data_ptr(), self.status.data_ptr(), st)
+            else:
+                _lib.call("pcg_tc_grouped_gemm", *gemm, 1, nv * nv, self.status.data_ptr(), st)
+                _lib.call("pcg_triples_energy", 1, P.data_ptr(), P[:, 1].data_ptr(),
+                          P[:, 2].data_ptr(), 3 * nv ** 3, ijk_all[b0:].data_ptr(), len(chunk),
+                          H.eps.data_ptr(), eoovv.data_ptr(), self.t1.data_ptr(),
+                          t2f.data_ptr(), fov_ptr, no, nv, part.data_ptr(), st)
             _lib.call("pcg_reduce_sum_f64", part.data_ptr(), len(chunk) * plen, out.data_ptr(),
                       st)
         s = self.status.cpu()
