@@ -79,6 +79,28 @@ inline long long sub_total(const SubIdx& d) {
   return t;
 }
 
+// Whether an output's row and column sub-indices (extents and strides) cover one contiguous run
+// of elements from its base pointer on.
+inline bool dense_output(int mn, const long long* me, const long long* ms, int nn,
+                         const long long* ne, const long long* ns) {
+  long long e[2 * kMaxSub], s[2 * kMaxSub];
+  int k = 0;
+  for (int q = 0; q < mn; ++q)
+    if (me[q] > 1) e[k] = me[q], s[k++] = ms[q];
+  for (int q = 0; q < nn; ++q)
+    if (ne[q] > 1) e[k] = ne[q], s[k++] = ns[q];
+  long long run = 1;
+  for (int left = k; left > 0; --left) {  // take the sub-index whose stride continues the run
+    int at = -1;
+    for (int q = 0; q < k; ++q)
+      if (e[q] > 0 && s[q] == run) at = q;
+    if (at < 0) return false;
+    run *= e[at];
+    e[at] = 0;
+  }
+  return true;
+}
+
 // Status word for device-side bounded waits (0 = fine).
 enum DeviceStatus : int {
   kStatusOk = 0,

@@ -187,8 +187,11 @@ __device__ __forceinline__ void gemv_store(const F64Args& p, double* dst, double
 
 // Outputs with a degenerate free dimension (matrix-vector shapes such as 'nf,mnef->me', and
 // full dot products): one warp per output element and K slice (blockIdx.y), a warp-wide FP64
-// dot over the slice.  HBM-bound.
-__global__ void contract_gemv_kernel(const F64Args p) {
+// dot over the slice, four products a lane in flight and (I) 32-bit index arithmetic where the
+// totals allow it.  'ijab,jb->ia' at no = 11, nv = 83: 17 us against 24 with one product in
+// flight and 64-bit divisions.
+template <typename I>
+__global__ void __launch_bounds__(256) contract_gemv_kernel(const F64Args p) {
   const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
   const int lane = threadIdx.x & 31;
   const long long total = p.M * p.N;
@@ -196,23 +199,35 @@ __global__ void contract_gemv_kernel(const F64Args p) {
   const long long kend = min(p.K, kbeg + p.k_per_split);
   for (long long o = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; o < total;
        o += warps) {
-    const long long m = o / p.N, n = o % p.N;
+    const long long m = (long long)((I)o / (I)p.N), n = o - m * p.N;
     long long am, cm, bn, cn;
-    sub_offsets(p.m, m, am, cm);
-    sub_offsets(p.n, n, bn, cn);
-    double acc = 0.0;
-    if (p.k.n == 1) {
-      const long long sa = p.k.s0[0], sb = p.k.s1[0];
-      for (long long k = kbeg + lane; k < kend; k += 32) acc += p.A[am + k * sa] * p.B[bn + k * sb];
-    } else {
-      for (long long k = kbeg + lane; k < kend; k += 32) {
-        long long ka, kb;
-        sub_offsets(p.k, k, ka, kb);
-        acc += p.A[am + ka] * p.B[bn + kb];
+    sub_offsets_as<I>(p.m, (I)m, am, cm);
+    sub_offsets_as<I>(p.n, (I)n, bn, cn);
+    const double *A = p.A + am, *B = p.B + bn;
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    for (long long k = kbeg + lane; k < kend; k += 128) {
+      double a[4], b[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        a[u] = b[u] = 0.0;
+        if (k + 32 * u < kend) {
+          long long ka, kb;
+          if (p.k.n == 1) {
+            ka = (k + 32 * u) * p.k.s0[0];
+            kb = (k + 32 * u) * p.k.s1[0];
+          } else {
+            sub_offsets_as<I>(p.k, (I)(k + 32 * u), ka, kb);
+          }
+          a[u] = __ldg(A + ka);
+          b[u] = __ldg(B + kb);
+        }
       }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) acc[u] = fma(a[u], b[u], acc[u]);
     }
-    for (int s = 16; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
-    if (lane == 0) gemv_store(p, p.C + cm + cn, acc);
+    double sum = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+    for (int s = 16; s > 0; s >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, s);
+    if (lane == 0) gemv_store(p, p.C + cm + cn, sum);
   }
 }
 
@@ -259,6 +274,21 @@ void sort_by_operand_stride(SubIdx& d) {
         std::swap(d.s0[i], d.s0[j]);
         std::swap(d.s1[i], d.s1[j]);
       }
+}
+
+// C[m, n] *= beta ahead of a split K.  A zero fill of a C without gaps is a memset.
+int scale_output(const F64Args& p, const SubIdx& m, const SubIdx& n, long long M, long long N,
+                 double beta, cudaStream_t st) {
+  if (beta == 1.0) return 0;
+  if (beta == 0.0 && dense_output(m.n, m.ext, m.s1, n.n, n.ext, n.s1)) {
+    if (cudaMemsetAsync(p.C, 0, (size_t)(8 * M * N), st) == cudaSuccess) return 0;
+    set_error("pcg_contract_f64: clearing the output failed");
+    return -2;
+  }
+  scale_strided_kernel<<<(int)std::min<long long>((M * N + 255) / 256, 4096), 256, 0, st>>>(
+      m, n, M, N, beta, p.C);
+  PCG_CHECK_LAUNCH("pcg_contract_f64/scale");
+  return 0;
 }
 
 bool fill_sub(SubIdx& d, int n, const long long* ext, const long long* s0, const long long* s1,
@@ -352,11 +382,8 @@ extern "C" int pcg_contract_f64(int m_n, const long long* m_ext, const long long
       const long long splits = gemv_splits(q, blocks, 64);
       q.k_per_split = (q.K + splits - 1) / splits;
       q.atomic_out = splits > 1;
-      if (q.atomic_out && beta != 1.0) {
-        scale_strided_kernel<<<(int)std::min<long long>((q.M * q.N + 255) / 256, 4096), 256, 0,
-                               st>>>(q.m, q.n, q.M, q.N, beta, C);
-        PCG_CHECK_LAUNCH("pcg_contract_f64/gemv_scale");
-      }
+      if (q.atomic_out)
+        if (const int rc = scale_output(q, q.m, q.n, q.M, q.N, beta, st)) return rc;
       contract_gemv_thread_kernel<<<dim3((unsigned)blocks, (unsigned)splits), 256, 0, st>>>(q);
       PCG_CHECK_LAUNCH("pcg_contract_f64/gemv_thread");
       return 0;
@@ -368,12 +395,13 @@ extern "C" int pcg_contract_f64(int m_n, const long long* m_ext, const long long
     const long long splits = gemv_splits(p, blocks, 512);
     p.k_per_split = (p.K + splits - 1) / splits;
     p.atomic_out = splits > 1;
-    if (p.atomic_out && beta != 1.0) {
-      scale_strided_kernel<<<(int)std::min<long long>((p.M * p.N + 255) / 256, 4096), 256, 0,
-                             st>>>(p.m, p.n, p.M, p.N, beta, C);
-      PCG_CHECK_LAUNCH("pcg_contract_f64/gemv_scale");
-    }
-    contract_gemv_kernel<<<dim3((unsigned)blocks, (unsigned)splits), 256, 0, st>>>(p);
+    if (p.atomic_out)
+      if (const int rc = scale_output(p, p.m, p.n, p.M, p.N, beta, st)) return rc;
+    const dim3 grid((unsigned)blocks, (unsigned)splits);
+    if (p.M * p.N > 0x7fffffffLL || p.K > 0x7fffffffLL - 128)
+      contract_gemv_kernel<unsigned long long><<<grid, 256, 0, st>>>(p);
+    else
+      contract_gemv_kernel<unsigned><<<grid, 256, 0, st>>>(p);
     PCG_CHECK_LAUNCH("pcg_contract_f64/gemv");
     return 0;
   }
@@ -401,12 +429,8 @@ extern "C" int pcg_contract_f64(int m_n, const long long* m_ext, const long long
     set_error("pcg_contract_f64: M=%lld x N=%lld too large", p.M, p.N);
     return -1;
   }
-  if (p.atomic_out && beta != 1.0) {
-    const long long total = p.M * p.N;
-    scale_strided_kernel<<<(int)std::min<long long>((total + 255) / 256, 4096), 256, 0, st>>>(
-        p.m, p.n, p.M, p.N, beta, C);
-    PCG_CHECK_LAUNCH("pcg_contract_f64/scale");
-  }
+  if (p.atomic_out)
+    if (const int rc = scale_output(p, p.m, p.n, p.M, p.N, beta, st)) return rc;
   const dim3 grid((unsigned)blocks, (unsigned)splits);
   const bool wide = p.M > 0x7fffffffLL || p.N > 0x7fffffffLL || p.K > 0x7fffffffLL;
   auto go = [&](auto kernel) { kernel<<<grid, 256, 0, st>>>(p, kw, nt, tiles); };
