@@ -801,12 +801,15 @@ __global__ void __launch_bounds__(PACK_THREADS) pack_fp8_kernel(const PackArgs p
   }
 }
 
+// C *= beta ahead of a split K (beta neither 0 over a C without gaps, which is a memset, nor 1).
+template <typename I>
 __global__ void scale_epi_kernel(EpiIdx em, EpiIdx en, long long M, long long N, double beta,
                                  double* C) {
-  long long total = M * N;
+  const long long total = M * N;
   for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x) {
-    double* dst = C + epi_offset(em, idx / N) + epi_offset(en, idx % N);
+    const I r = (I)idx / (I)N;
+    double* dst = C + epi_offset(em, (long long)r) + epi_offset(en, (long long)((I)idx - r * (I)N));
     *dst = (beta == 0.0) ? 0.0 : beta * *dst;
   }
 }
@@ -1260,15 +1263,26 @@ extern "C" int pcg_tc_gemm(int fmt, const void* A_hi, const void* A_mid, const v
   // (the short-K terms are bound by that wait)
   a.red_out = (splits == 1 && nkb <= a.kb_chunk) ? 1 : 0;
   cudaStream_t st = (cudaStream_t)stream;
-  if (a.atomic_out && beta != 1.0) {
+  if (a.atomic_out && beta == 0.0 &&
+      dense_output(a.em.n, a.em.ext, a.em.s, a.en.n, a.en.ext, a.en.s) && !col_map) {
+    if (cudaMemsetAsync(C, 0, (size_t)(8 * M * N), st) != cudaSuccess) {
+      set_error("pcg_tc_gemm: clearing the output failed");
+      return -2;
+    }
+  } else if (a.atomic_out && beta != 1.0) {
     int blocks = (int)std::min<long long>((M * N + 255) / 256, 4096);
-    scale_epi_kernel<<<blocks, 256, 0, st>>>(a.em, a.en, M, N, beta, C);
+    if (M * N <= 0x7fffffffLL)
+      scale_epi_kernel<unsigned><<<blocks, 256, 0, st>>>(a.em, a.en, M, N, beta, C);
+    else
+      scale_epi_kernel<unsigned long long><<<blocks, 256, 0, st>>>(a.em, a.en, M, N, beta, C);
     PCG_CHECK_LAUNCH("pcg_tc_gemm/scale");
   }
-  Maps maps;
+  Maps maps{};
   const void* pa[3] = {A_hi, fmt == kBF16x6 ? A_mid : A_lo, A_lo};
   const void* pb[3] = {B_hi, fmt == kBF16x6 ? B_mid : B_lo, B_lo};
-  for (int q = 0; q < 3; ++q) {
+  // the pieces that the format's products read: one, two (hi, lo) or three
+  const int pieces = need_lo ? (fmt == kBF16x6 ? 3 : 2) : 1;
+  for (int q = 0; q < pieces; ++q) {
     if (!make_map(&maps.a[q], pa[q] ? pa[q] : A_hi, M, lda * eb, Kp * eb, eb, BM)) return -1;
     if (!make_map(&maps.b[q], pb[q] ? pb[q] : B_hi, N, ldb * eb, Kp * eb, eb, a.bs)) return -1;
   }
