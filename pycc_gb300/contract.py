@@ -194,20 +194,21 @@ def _takes_rns(m, n, k):
     """Whether an m x n x k contraction runs on the tensor cores in residue arithmetic rather
     than on the FP64 pipe: where its estimated time is the shorter one.
 
-    FP64 pipe: 15 us and 1 TFLOP/s over whole 16 x 16 x 4 tiles.  Residues: 65 us of launches,
-    48 bytes moved per operand element at 5 TB/s, 16 BF16 products over whole 128 x 16 x 64
-    tiles at 1.1 PFLOP/s and at least 2.5 us for 128 x 256 of them on an SM, and 13 ps per output
-    to rebuild it.  Measured on both sides of the line (us, FP64 pipe / residues): 477 x 477 x
-    477 223 / 69, 53 x 25281 x 9 66 / 89, 81 x 2809 x 81 91 / 71, 110 x 21560 x 14 101 / 105,
-    180 x 72000 x 20 911 / 443."""
+    FP64 pipe: 6 us and 1.05 TFLOP/s.  Residues: 42 us of launches, 48 bytes moved per operand
+    element at 5 TB/s, 0.3 ns per step of K (a row's norm), 16 BF16 products over whole 128 x 16 x
+    64 tiles at 1.1 PFLOP/s and at least 2.5 us for 128 x 256 of them on an SM, and 13 ps per
+    output to rebuild it.  Measured on both sides of the line (us, FP64 pipe / residues): 2809 x 81
+    x 81 48 / 46, 53 x 53 x 4293 42 / 44, 60 x 60 x 8640 73 / 53, 110 x 21560 x 14 88 / 92, 11 x
+    75779 x 83 146 / 183, 14 x 169400 x 110 567 / 387, 20 x 20 x 648000 482 / 676, 180 x 72000 x
+    20 511 / 356, 477 x 477 x 477 205 / 52."""
     if min(m, n) < 2 or m * n * k < 1 << 22:
         return False
     up = lambda x, t: -(-x // t) * t
-    fp64 = 15e-6 + 2.0 * up(m, 16) * up(n, 16) * up(k, 4) / 1e12
+    fp64 = 6e-6 + 2.0 * m * n * k / 1.05e12
     lo, hi = (m, n) if m < n else (n, m)
     gemm = max(32.0 * up(lo, 128) * hi * up(k, 64) / 1.1e15,
                16 * up(lo, 128) // 128 * up(hi, 256) // 256 * 2.5e-6 / 152)
-    rns = 65e-6 + 48.0 * (m + n) * k / 5e12 + gemm + 13e-12 * m * n
+    rns = 42e-6 + 48.0 * (m + n) * k / 5e12 + 0.3e-9 * k + gemm + 13e-12 * m * n
     return rns < fp64
 
 

@@ -1,4 +1,4 @@
-// FP64 strided tensor contraction on the FP64 tensor pipe (DMMA, mma.sync m8n8k4 f64).
+// FP64 strided tensor contraction on the FP64 pipe.
 //
 //   C[m, n] = beta * C[m, n] + alpha * sum_k A[m, k] * B[n, k]
 //
@@ -48,116 +48,134 @@ __device__ __forceinline__ void sub_offsets_as(const SubIdx& d, I r, long long& 
   }
 }
 
-// A warp computes 8 FM x 8 FN outputs over a slice of K, its DMMA fragments read straight from
-// global memory (L1 holds the rows; the 8 x 4 fragment of a lane pattern is whole sectors
-// whichever index is unit-stride).  A quarter of an SM's FP64 pipe takes about 512 clocks for one
-// m8n8k4, so loads cost little next to it; what bounds a small product is how evenly the
-// multiply-adds spread over the 608 quarters.  Blocks of 64 x 64 tiles left most of them idle.
-// Here kw of the block's 8 warps share an output tile and split K, blocks split K further (FP64
-// atomics), and a tile is 16 x 16, 8 x 32 or 32 x 8 where one side has at most 8 entries, or
-// 8 x 8 where there would be fewer 16-K steps than would keep every quarter busy.
-// Device time against 64 x 64 tiles in shared memory, us: no = 5, nv = 19 ring 138 -> 11, small
-// products 45-60 -> 6-8; no = 9, nv = 53 'nb,mnej->mbej' 41 -> 15, 'mief,maef->ia' 490 -> 59; the
-// large ladder of no = 20, nv = 180 882 -> 770 ms (1.09 TFLOP/s).
-template <int FM, int FN, typename I>
-__global__ void __launch_bounds__(256) contract_f64_kernel(const F64Args p, int kw,
+// Stores one partial (or the whole) sum of products of an output element: with K split across
+// blocks (blockIdx.y) the partials are atomic FP64 adds onto C, which the host scaled by
+// beta first.
+__device__ __forceinline__ void store_sum(const F64Args& p, double* dst, double acc) {
+  const double v = p.alpha * acc;
+  if (p.atomic_out)
+    atomicAdd(dst, v);
+  else
+    *dst = (p.beta == 0.0) ? v : p.beta * *dst + v;
+}
+
+// Clusters of `cy` blocks along K: the first block's first warp adds up what the others' first
+// warps left in their shared memory (`mine` there, one value per lane and entry).  All threads of
+// all blocks come here.
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ double cluster_load(const double* p, int rank) {
+  unsigned a = (unsigned)__cvta_generic_to_shared(p);
+  double v;
+  asm volatile("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(a) : "r"(rank));
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
+  return v;
+}
+template <int N>
+__device__ __forceinline__ void cluster_sums(double (&x)[N], double* mine, int stride, int cy,
+                                             bool first_warp) {
+  if (first_warp)
+#pragma unroll
+    for (int i = 0; i < N; ++i) mine[i * stride] = x[i];
+  cluster_barrier();
+  if (first_warp && blockIdx.y % cy == 0)
+    for (int c = 1; c < cy; ++c)
+#pragma unroll
+      for (int i = 0; i < N; ++i) x[i] += cluster_load(mine + i * stride, c);
+  cluster_barrier();  // no block leaves before its sums are read
+}
+
+// A warp computes 32 x R outputs over a slice of K: a lane per index of the long side (m), R
+// entries of the other side (n), FP64 multiply-adds with all operands straight from global
+// memory.  An SM quarter takes 64 clocks for a warp's FP64 multiply-add, so a step's R + 1 loads
+// (the R ones are broadcasts) cost little next to it; what bounds a product is how evenly the
+// multiply-adds spread over the 608 quarters and how many of them are padding.  Neither side is
+// padded to 8 x 8 fragments as mma.m8n8k4 needs, which has the same FP64 rate.  kw warps of a
+// block share a tile and split K, clusters of cy blocks split it further, and clusters beyond that
+// (FP64 atomics, each a rounding of the output: without the clusters they were most of the
+// rounding error of the singles' residual).
+// Device time against 16 x 16 mma tiles, us: no = 9, nv = 53 'ijae,be->ijab' 45 -> 29, 'ie,abej->
+// ijab' 62 -> 29, no = 11, nv = 83 'nb,mnej->mbej' 40 -> 26, 'ie,abej->ijab' 215 -> 143, no = 20,
+// nv = 180 'mi,mjab->ijab' 959 -> 512 (1.0 TFLOP/s); no = 5, nv = 19 6 -> 4.6-6.
+template <int R, typename I>
+__global__ void __launch_bounds__(256) contract_f64_kernel(const F64Args p, int kw, int cy,
                                                            long long tiles_n, long long tiles) {
-  constexpr int NF = 2 * FM * FN;
-  __shared__ double red[8][NF][32];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int g = lane >> 2, t4 = lane & 3;
-  const int ks = warp % kw;
-  const long long tile = (long long)blockIdx.x * (8 / kw) + warp / kw;
+  constexpr int U = 4;  // K steps whose loads are in flight
+  __shared__ double red[8][R][32];
+  __shared__ longlong2 koff[8][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ks = warp % kw;
+  const long long tile = (long long)blockIdx.x * ((int)(blockDim.x >> 5) / kw) + warp / kw;
   const bool live = tile < tiles;
-  const long long m0 = (live ? tile / tiles_n : 0) * (8 * FM);
-  const long long n0 = (live ? tile % tiles_n : 0) * (8 * FN);
-  const long long kbeg = (long long)blockIdx.y * p.k_per_split;
-  const long long kend = live ? min(p.K, kbeg + p.k_per_split) : 0;
+  const long long tm = live ? tile / tiles_n : 0, n0 = (live ? tile % tiles_n : 0) * R;
+  const long long row = tm * 32 + lane;
+  const long long bbeg = (long long)blockIdx.y * p.k_per_split;
+  const long long bend = live ? min(p.K, bbeg + p.k_per_split) : 0;
+  const long long slice = (p.k_per_split + kw - 1) / kw;
+  const long long kbeg = min(bend, bbeg + ks * slice), kend = min(bend, kbeg + slice);
 
-  long long ao[FM], bo[FN], cm[FM];
-  bool aok[FM], bok[FN];
+  // entries past the end repeat the last one; only the store leaves them out
+  long long ao, cm, cn[R];
+  sub_offsets_as<I>(p.m, (I)min(row, p.M - 1), ao, cm);
+  const double *A = p.A + ao, *B[R];
 #pragma unroll
-  for (int i = 0; i < FM; ++i) {
-    const long long r = m0 + 8 * i + g;
-    aok[i] = r < p.M;
-    ao[i] = cm[i] = 0;
-    if (aok[i]) sub_offsets_as<I>(p.m, (I)r, ao[i], cm[i]);
+  for (int r = 0; r < R; ++r) {
+    long long bo;
+    sub_offsets_as<I>(p.n, (I)min(n0 + r, p.N - 1), bo, cn[r]);
+    B[r] = p.B + bo;
   }
+  double acc[R], odd[R];  // even and odd steps apart: shorter chains, smaller rounding errors
 #pragma unroll
-  for (int j = 0; j < FN; ++j) {
-    const long long r = n0 + 8 * j + g;
-    long long unused;
-    bok[j] = r < p.N;
-    bo[j] = 0;
-    if (bok[j]) sub_offsets_as<I>(p.n, (I)r, bo[j], unused);
-  }
-  double acc[FM][FN][2];
-#pragma unroll
-  for (int i = 0; i < FM; ++i)
-#pragma unroll
-    for (int j = 0; j < FN; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  for (int r = 0; r < R; ++r) acc[r] = odd[r] = 0.0;
 
-  for (long long k0 = kbeg + 16 * ks; k0 < kend; k0 += 16 * kw) {
-    double a[4][FM], b[4][FN];
+  for (long long k0 = kbeg; k0 < kend; k0 += 32) {
+    long long ka = 0, kb = 0;
+    if (k0 + lane < kend) sub_offsets_as<I>(p.k, (I)(k0 + lane), ka, kb);
+    __syncwarp();
+    koff[warp][lane] = make_longlong2(ka, kb);
+    __syncwarp();
+    const int kn = (int)min(32LL, kend - k0);
+    for (int u0 = 0; u0 < kn; u0 += U) {
+      double a[U], b[U][R];
 #pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      const long long k = k0 + 4 * s + t4;
-      const bool ok = k < kend;
-      long long ka = 0, kb = 0;
-      if (ok) sub_offsets_as<I>(p.k, (I)k, ka, kb);
+      for (int u = 0; u < U; ++u) {
+        const longlong2 o = koff[warp][min(u0 + u, kn - 1)];
+        a[u] = __ldg(A + o.x);
 #pragma unroll
-      for (int i = 0; i < FM; ++i) a[s][i] = (ok && aok[i]) ? __ldg(p.A + ao[i] + ka) : 0.0;
+        for (int r = 0; r < R; ++r) b[u][r] = __ldg(B[r] + o.y);
+      }
 #pragma unroll
-      for (int j = 0; j < FN; ++j) b[s][j] = (ok && bok[j]) ? __ldg(p.B + bo[j] + kb) : 0.0;
-    }
-    if (k0 + 12 < kend) {
+      for (int u = 0; u < U; ++u)
+        if (u0 + u < kn)
 #pragma unroll
-      for (int s = 0; s < 4; ++s)
-#pragma unroll
-        for (int i = 0; i < FM; ++i)
-#pragma unroll
-          for (int j = 0; j < FN; ++j) dmma(acc[i][j], a[s][i], b[s][j]);
-    } else {  // the last step multiplies the K it has
-#pragma unroll
-      for (int s = 0; s < 3; ++s)
-        if (k0 + 4 * s < kend)
-#pragma unroll
-          for (int i = 0; i < FM; ++i)
-#pragma unroll
-            for (int j = 0; j < FN; ++j) dmma(acc[i][j], a[s][i], b[s][j]);
+          for (int r = 0; r < R; ++r) {
+            double& x = u & 1 ? odd[r] : acc[r];
+            x = fma(a[u], b[u][r], x);
+          }
     }
   }
+#pragma unroll
+  for (int r = 0; r < R; ++r) acc[r] += odd[r];
 
   if (kw > 1) {  // the K slices of a tile add up in its first warp
     if (ks > 0)
 #pragma unroll
-      for (int f = 0; f < NF; ++f) red[warp][f][lane] = acc[f / (2 * FN)][(f / 2) % FN][f % 2];
+      for (int r = 0; r < R; ++r) red[warp][r][lane] = acc[r];
     __syncthreads();
-    if (ks > 0) return;
-    for (int w = warp + 1; w < warp + kw; ++w)
+    if (ks == 0)
+      for (int w = warp + 1; w < warp + kw; ++w)
 #pragma unroll
-      for (int f = 0; f < NF; ++f) acc[f / (2 * FN)][(f / 2) % FN][f % 2] += red[w][f][lane];
+        for (int r = 0; r < R; ++r) acc[r] += red[w][r][lane];
+    if (cy > 1) cluster_sums(acc, &red[0][0][lane], 32, cy, warp == 0);
+    if (ks > 0 || blockIdx.y % cy > 0) return;
   }
-  if (!live) return;
+  if (!live || row >= p.M) return;
 #pragma unroll
-  for (int j = 0; j < FN; ++j)
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const long long c = n0 + 8 * j + 2 * t4 + h;
-      if (c >= p.N) continue;
-      long long unused, cn;
-      sub_offsets_as<I>(p.n, (I)c, unused, cn);
-#pragma unroll
-      for (int i = 0; i < FM; ++i) {
-        if (!aok[i]) continue;
-        double* dst = p.C + cm[i] + cn;
-        const double v = p.alpha * acc[i][j][h];
-        if (p.atomic_out)
-          atomicAdd(dst, v);
-        else
-          *dst = p.beta == 0.0 ? v : p.beta * *dst + v;
-      }
-    }
+  for (int r = 0; r < R; ++r) {
+    if (n0 + r >= p.N) break;
+    store_sum(p, p.C + cm + cn[r], acc[r]);
+  }
 }
 
 // C[m, n] *= beta over the strided M x N range (used before a split-K accumulation).
@@ -174,38 +192,105 @@ __global__ void scale_strided_kernel(SubIdx m, SubIdx n, long long M, long long 
   }
 }
 
-// Stores one partial (or the whole) dot product of an output element: with K split across
-// blocks (blockIdx.y) the partials are atomic FP64 adds onto C, which the host scaled by
-// beta first.
-__device__ __forceinline__ void gemv_store(const F64Args& p, double* dst, double acc) {
-  const double v = p.alpha * acc;
-  if (p.atomic_out)
-    atomicAdd(dst, v);
-  else
-    *dst = (p.beta == 0.0) ? v : p.beta * *dst + v;
+// The same product with the lanes along K: a warp computes T x T outputs over a slice of K, so
+// that a few outputs of a long K are not padded to 32 rows, and adds its lanes' sums up by halves
+// (16 FP64 additions for up to 16 outputs; five for each would cost more than the products of a
+// short slice).  us, against 16 x 16 mma tiles: no = 9, nv = 53 'ijef,mnef->mnij' 94 -> 43,
+// 'ijab,mjab->im' 35 -> 17; no = 11, nv = 83 'mief,maef->ia' 333 -> 168, 'mnef,mnaf->ae' 263 ->
+// 133; no = 14, nv = 60 'ijef,mnef->mnij' 412 -> 241 (1.15 TFLOP/s).
+template <int T, typename I>
+__global__ void __launch_bounds__(256) contract_dot_kernel(const F64Args p, int kw, int cy,
+                                                           long long tiles_n, long long tiles) {
+  constexpr int U = 2, NV = 16;
+  __shared__ double red[8][NV];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, per = 8 / kw, ks = warp % kw;
+  const long long kbeg = (long long)blockIdx.y * p.k_per_split;
+  const long long kend = min(p.K, kbeg + p.k_per_split);
+  const long long t = (long long)blockIdx.x * per + warp / kw, tc = min(t, tiles - 1);
+  const long long tm = (long long)((I)tc / (I)tiles_n), m0 = tm * T, n0 = (tc - tm * tiles_n) * T;
+  const double *A[T], *B[T];
+#pragma unroll
+  for (int r = 0; r < T; ++r) {  // entries past the end repeat the last one
+    long long o, unused;
+    sub_offsets_as<I>(p.m, (I)min(m0 + r, p.M - 1), o, unused);
+    A[r] = p.A + o;
+    sub_offsets_as<I>(p.n, (I)min(n0 + r, p.N - 1), o, unused);
+    B[r] = p.B + o;
+  }
+  double v[NV];
+#pragma unroll
+  for (int j = 0; j < NV; ++j) v[j] = 0.0;
+  for (long long k = kbeg + 32 * U * ks + lane; k < kend; k += 32 * U * kw) {
+    double a[U][T], b[U][T];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const bool ok = k + 32 * u < kend;
+      long long ka = 0, kb = 0;
+      if (ok) sub_offsets_as<I>(p.k, (I)(k + 32 * u), ka, kb);
+#pragma unroll
+      for (int r = 0; r < T; ++r) {
+        a[u][r] = ok ? __ldg(A[r] + ka) : 0.0;
+        b[u][r] = ok ? __ldg(B[r] + kb) : 0.0;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int i = 0; i < T; ++i)
+#pragma unroll
+        for (int j = 0; j < T; ++j) v[i * T + j] = fma(a[u][i], b[u][j], v[i * T + j]);
+  }
+  int out = 0;  // this lane's output of the tile
+#pragma unroll
+  for (int h = NV / 2, s = 16; h > 0; h >>= 1, s >>= 1) {
+    const bool up = lane & s;
+    out += up ? h : 0;
+#pragma unroll
+    for (int j = 0; j < h; ++j) {
+      const double give = up ? v[j] : v[j + h], keep = up ? v[j + h] : v[j];
+      v[j] = keep + __shfl_xor_sync(0xffffffffu, give, s);
+    }
+  }
+  double x[1] = {v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1)};
+  if (kw > 1) {
+    if (ks > 0) red[warp][out] = x[0];
+    __syncthreads();
+    if (ks == 0)
+      for (int w = warp + 1; w < warp + kw; ++w) x[0] += red[w][out];
+    if (cy > 1) cluster_sums(x, &red[0][out], 0, cy, warp == 0);
+    if (ks > 0 || blockIdx.y % cy > 0) return;
+  }
+  const long long m = m0 + out / T, n = n0 + out % T;
+  if (!(lane & 1) && t < tiles && out < T * T && m < p.M && n < p.N) {
+    long long unused, cm, cn;
+    sub_offsets_as<I>(p.m, (I)m, unused, cm);
+    sub_offsets_as<I>(p.n, (I)n, unused, cn);
+    store_sum(p, p.C + cm + cn, x[0]);
+  }
 }
 
 // Outputs with a degenerate free dimension (matrix-vector shapes such as 'nf,mnef->me', and
-// full dot products): one warp per output element and K slice (blockIdx.y), a warp-wide FP64
-// dot over the slice, four products a lane in flight and (I) 32-bit index arithmetic where the
-// totals allow it.  'ijab,jb->ia' at no = 11, nv = 83: 17 us against 24 with one product in
-// flight and 64-bit divisions.
+// full dot products): kw warps of a block share an output and a K slice (blockIdx.y), a lane holds
+// four products in flight and (I) 32-bit index arithmetic where the totals allow it.  With one
+// warp per output the index divisions of K / 32 products were a serial chain.  us: 'ijab,jb->ia'
+// no = 11, nv = 83 15 -> 10; 'ijab,ijab->' no = 5, nv = 19 6.2 -> 5.0, no = 40, nv = 300 1730 ->
+// 380-430 (5.3-6 TB/s).
 template <typename I>
-__global__ void __launch_bounds__(256) contract_gemv_kernel(const F64Args p) {
-  const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
-  const int lane = threadIdx.x & 31;
+__global__ void __launch_bounds__(256) contract_gemv_kernel(const F64Args p, int kw) {
+  __shared__ double red[8];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, per = 8 / kw, ks = warp % kw;
   const long long total = p.M * p.N;
   const long long kbeg = (long long)blockIdx.y * p.k_per_split;
   const long long kend = min(p.K, kbeg + p.k_per_split);
-  for (long long o = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; o < total;
-       o += warps) {
-    const long long m = (long long)((I)o / (I)p.N), n = o - m * p.N;
+  for (long long o0 = (long long)blockIdx.x * per; o0 < total; o0 += (long long)gridDim.x * per) {
+    const long long o = o0 + warp / kw, oc = min(o, total - 1);
+    const long long m = (long long)((I)oc / (I)p.N), n = oc - m * p.N;
     long long am, cm, bn, cn;
     sub_offsets_as<I>(p.m, (I)m, am, cm);
     sub_offsets_as<I>(p.n, (I)n, bn, cn);
     const double *A = p.A + am, *B = p.B + bn;
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    for (long long k = kbeg + lane; k < kend; k += 128) {
+    for (long long k = kbeg + ks * 128 + lane; k < kend; k += 128 * kw) {
       double a[4], b[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
@@ -227,7 +312,14 @@ __global__ void __launch_bounds__(256) contract_gemv_kernel(const F64Args p) {
     }
     double sum = (acc[0] + acc[1]) + (acc[2] + acc[3]);
     for (int s = 16; s > 0; s >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, s);
-    if (lane == 0) gemv_store(p, p.C + cm + cn, sum);
+    if (kw > 1) {
+      if (lane == 0) red[warp] = sum;
+      __syncthreads();
+      if (ks == 0)
+        for (int w = warp + 1; w < warp + kw; ++w) sum += red[w];
+      __syncthreads();  // the next output's sums go to the same place
+    }
+    if (lane == 0 && ks == 0 && o < total) store_sum(p, p.C + cm + cn, sum);
   }
 }
 
@@ -256,14 +348,8 @@ __global__ void __launch_bounds__(256) contract_gemv_thread_kernel(const F64Args
     if (valid)
       for (int j = 0; j < kn; ++j) acc += p.A[am + ka[j]] * p.B[bn + kb[j]];
   }
-  if (valid) gemv_store(p, p.C + cm + cn, acc);
+  if (valid) store_sum(p, p.C + cm + cn, acc);
 }
-
-// K slices for a matrix-vector launch of `blocks` output blocks: enough blocks for about
-// eight per SM, each slice at least `kmin` long; beta is applied up front when split.  kmin is
-// 64 for a thread per output (with 1024, 'mf,mafe->ae' at no = 9, nv = 53 ran 11 blocks for
-// 79 us; 11 us now) and 512 for a warp.
-long long gemv_splits(const F64Args& p, long long blocks, long long kmin);
 
 // Reorder sub-indices by decreasing |stride| in the operand (s0), unit stride innermost.
 void sort_by_operand_stride(SubIdx& d) {
@@ -320,13 +406,6 @@ bool fill_sub(SubIdx& d, int n, const long long* ext, const long long* s0, const
   return true;
 }
 
-long long gemv_splits(const F64Args& p, long long blocks, long long kmin) {
-  const long long want = 8LL * 152;
-  if (blocks >= want || p.K < 2 * kmin) return 1;
-  long long splits = std::min((want + blocks - 1) / blocks, p.K / kmin);
-  return std::max(1LL, std::min(splits, 65535LL));
-}
-
 int num_sms() {
   static int sms = 0;
   if (!sms) {
@@ -336,6 +415,101 @@ int num_sms() {
     if (sms <= 0) sms = 148;
   }
   return sms;
+}
+
+// How a product is cut: R entries of the n side per warp (lanes along m), or T x T outputs
+// (lanes along K); kw warps per tile, blocks of nw warps, K over `splits` blocks in clusters of cy.
+struct F64Plan {
+  int R, T, kw, nw, cy;
+  bool swap;  // the operands exchanged
+  long long splits, tiles_n, tiles, blocks;
+  double clocks;
+};
+
+// Fills in the rest of a cut and keeps it if it is estimated to be the fastest yet, in clocks of
+// the SM with the most blocks: on each quarter's FP64 pipe `step` clocks per K step and `fixed`
+// per warp; and, only partly hidden by the other warps, the chain of a warp with `wait` more per
+// step.  The sums of a cluster cost 2000 and 800 per warp, K split over s of them a pass
+// over C and s atomic additions to each output (5000 + 200 s).
+void consider(F64Plan& best, F64Plan q, long long steps, double step, double wait, double fixed) {
+  const long long sms = num_sms();
+  q.nw = q.T ? 8 : std::max(4, q.kw);
+  q.blocks = (q.tiles * q.kw + q.nw - 1) / q.nw;
+  const long long top = q.kw < 8 ? 1 : std::max(1LL, std::min(steps / (q.T ? 16 : 64), 65528LL));
+  const long long fill = (4 * sms + q.blocks - 1) / q.blocks;
+  const long long tries[4] = {1, std::min(top, 8LL), std::min(top, fill / 2), std::min(top, fill)};
+  for (int i = 0; i < (top > 1 ? 4 : 1); ++i) {
+    if (i > 0 && tries[i] < 2) continue;
+    q.cy = tries[i] >= 8 ? 8 : 1;
+    q.splits = tries[i] / q.cy * q.cy;
+    const double ks = (double)((steps + q.splits * q.kw - 1) / (q.splits * q.kw));
+    const double warps = (double)((q.blocks * q.splits + sms - 1) / sms) * q.nw / 4;
+    const double each = fixed + (q.cy > 1 ? 800 : 0);
+    const double sums = 64.0 * (q.T ? 1 : q.R) * (q.kw - 1);  // of a tile's K slices
+    q.clocks = warps * (step * ks + each + sums / q.kw) +
+               0.4 * (1000 + ks * (step + wait) + each + sums) + (q.cy > 1 ? 2000 : 0) +
+               (q.splits > q.cy ? 5000 + 200.0 * q.splits / q.cy : 0);
+    if (best.clocks == 0 || q.clocks < best.clocks) best = q;
+  }
+}
+
+// Lanes along the first side, with every R and kw.
+void consider_rows(F64Plan& best, long long M, long long N, long long K, bool wide, bool swap) {
+  const int r0 = wide ? 4 : 2, r1 = wide ? 4 : 6;
+  F64Plan q{};
+  q.swap = swap;
+  for (q.R = r0; q.R <= r1; ++q.R) {
+    q.tiles_n = (N + q.R - 1) / q.R;
+    q.tiles = (M + 31) / 32 * q.tiles_n;
+    for (q.kw = 1; q.kw <= 8 && (q.kw == 1 || K >= 4 * q.kw); q.kw *= 2)
+      consider(best, q, K, 64.0 * q.R, 150, 250);
+  }
+}
+
+// Lanes along K.  Where K is not unit-stride a load touches 32 rows of the L1, which all four
+// quarters share.
+void consider_dots(F64Plan& best, const F64Args& p) {
+  const int la = p.k.s0[p.k.n - 1] == 1 ? 2 : 32, lb = p.k.s1[p.k.n - 1] == 1 ? 2 : 32;
+  F64Plan q{};
+  const long long steps = (p.K + 31) / 32;
+  for (q.T = 3; q.T <= 4; ++q.T) {
+    q.tiles_n = (p.N + q.T - 1) / q.T;
+    q.tiles = (p.M + q.T - 1) / q.T * q.tiles_n;
+    for (q.kw = 1; q.kw <= 8 && q.kw <= steps; q.kw *= 2)
+      consider(best, q, steps, std::max(64 * q.T * q.T, 4 * q.T * (la + lb)), 400, 1300);
+  }
+}
+
+// The cut of a product with M >= N > 1.  It depends on the sizes and on K's strides being one or
+// not; each thread keeps its last ones (a search takes a few us, as long as a small product).
+F64Plan f64_plan(const F64Args& p, bool wide) {
+  struct Known {
+    long long M, N, K;
+    int unit;
+    F64Plan q;
+  };
+  static thread_local Known known[64];
+  const int unit = (p.k.s0[p.k.n - 1] == 1) + 2 * (p.k.s1[p.k.n - 1] == 1);
+  Known& e = known[(unsigned long long)(p.M * 31 + p.N * 17 + p.K * 7 + unit) % 64];
+  if (e.M != p.M || e.N != p.N || e.K != p.K || e.unit != unit) {
+    F64Plan q{};
+    consider_rows(q, p.M, p.N, p.K, wide, false);
+    if (!wide && p.M < 512) {
+      if (p.M < 256) consider_rows(q, p.N, p.M, p.K, wide, true);  // may pad less
+      if (p.K >= 128) consider_dots(q, p);
+    }
+    e = {p.M, p.N, p.K, unit, q};
+  }
+  return e.q;
+}
+
+// the two operands exchanged
+F64Args swapped(F64Args p) {
+  std::swap(p.m, p.n);
+  std::swap(p.M, p.N);
+  std::swap(p.A, p.B);
+  for (int i = 0; i < p.k.n; ++i) std::swap(p.k.s0[i], p.k.s1[i]);
+  return p;
 }
 
 }  // namespace
@@ -365,83 +539,83 @@ extern "C" int pcg_contract_f64(int m_n, const long long* m_ext, const long long
   p.B = B;
   p.C = C;
   cudaStream_t st = (cudaStream_t)stream;
-  if (p.M == 1 || p.N == 1) {
-    // one free side: enumerate the outputs along the big operand's unit-stride index
-    F64Args q = p;
-    if (q.M == 1) {
-      sort_by_operand_stride(q.n);
-    } else {  // N == 1: swap roles so the free index is on the B side
-      std::swap(q.m, q.n);
-      std::swap(q.M, q.N);
-      std::swap(q.A, q.B);
-      for (int i = 0; i < q.k.n; ++i) std::swap(q.k.s0[i], q.k.s1[i]);
-      sort_by_operand_stride(q.n);
+  const bool wide = p.M > 0x7fffffffLL || p.N > 0x7fffffffLL || p.K > 0x7fffffffLL - 256;
+  if (p.M == 1) p = swapped(p);
+  if (p.N == 1) {
+    // one free side.  At least 1024 outputs along the operand's unit-stride index: a thread each,
+    // K in slices of 64 or more until there are about eight blocks per SM (with slices of 1024,
+    // 'mf,mafe->ae' at no = 9, nv = 53 ran 11 blocks for 79 us; 11 us now).  Otherwise warps,
+    // about six for each SM quarter: over K's 128-wide steps in a block, then over blocks.
+    p = swapped(p);
+    sort_by_operand_stride(p.n);
+    const bool threads = p.n.s0[p.n.n - 1] == 1 && p.N >= 1024;
+    long long blocks, splits = 1;
+    int kw = 1;
+    if (threads) {
+      blocks = (p.N + 255) / 256;
+      const long long want = 8LL * num_sms();
+      if (blocks < want && p.K >= 128) splits = std::min((want + blocks - 1) / blocks, p.K / 64);
+    } else {
+      const long long steps = (p.K + 127) / 128, want = 20LL * num_sms();
+      while (kw < 8 && 2 * kw <= steps && p.N * kw < want) kw *= 2;
+      blocks = std::min((p.N * kw + 7) / 8, 64LL * num_sms());
+      if (kw == 8) splits = std::min(want / 8 / blocks, steps / 8);
     }
-    if (q.n.s0[q.n.n - 1] == 1 && q.M * q.N >= 1024) {
-      const long long blocks = (q.M * q.N + 255) / 256;
-      const long long splits = gemv_splits(q, blocks, 64);
-      q.k_per_split = (q.K + splits - 1) / splits;
-      q.atomic_out = splits > 1;
-      if (q.atomic_out)
-        if (const int rc = scale_output(q, q.m, q.n, q.M, q.N, beta, st)) return rc;
-      contract_gemv_thread_kernel<<<dim3((unsigned)blocks, (unsigned)splits), 256, 0, st>>>(q);
-      PCG_CHECK_LAUNCH("pcg_contract_f64/gemv_thread");
-      return 0;
-    }
-  }
-  if (p.M == 1 || p.N == 1) {
-    long long warps = p.M * p.N;
-    int blocks = (int)std::min<long long>((warps * 32 + 255) / 256, 152LL * 64);
-    const long long splits = gemv_splits(p, blocks, 512);
+    splits = std::max(1LL, std::min(splits, 65535LL));
     p.k_per_split = (p.K + splits - 1) / splits;
     p.atomic_out = splits > 1;
     if (p.atomic_out)
       if (const int rc = scale_output(p, p.m, p.n, p.M, p.N, beta, st)) return rc;
     const dim3 grid((unsigned)blocks, (unsigned)splits);
-    if (p.M * p.N > 0x7fffffffLL || p.K > 0x7fffffffLL - 128)
-      contract_gemv_kernel<unsigned long long><<<grid, 256, 0, st>>>(p);
+    if (threads)
+      contract_gemv_thread_kernel<<<grid, 256, 0, st>>>(p);
+    else if (wide)
+      contract_gemv_kernel<unsigned long long><<<grid, 256, 0, st>>>(p, kw);
     else
-      contract_gemv_kernel<unsigned><<<grid, 256, 0, st>>>(p);
+      contract_gemv_kernel<unsigned><<<grid, 256, 0, st>>>(p, kw);
     PCG_CHECK_LAUNCH("pcg_contract_f64/gemv");
     return 0;
   }
-  // tiles of 16 x 16 outputs per warp, 8 x 32 or 32 x 8 where a side has at most 8, 8 x 8 where
-  // 16 x 16 tiles would leave fewer than two K steps for each quarter of an SM
-  const long long steps = (p.K + 15) / 16;
-  int fm = p.M <= 8 ? 1 : (p.N <= 8 ? 4 : 2), fn = 4 / fm;
-  if ((p.M + 15) / 16 * ((p.N + 15) / 16) * steps < 8LL * num_sms()) fm = fn = 1;
-  const long long nt = (p.N + 8 * fn - 1) / (8 * fn), mt = (p.M + 8 * fm - 1) / (8 * fm);
-  const long long tiles = mt * nt;
-  // warps per tile: K's 16-wide steps over up to 8 warps while that fills the chip (16 warps on
-  // each SM), then over blocks, each at least two steps a warp
-  const long long want = 16LL * num_sms();
-  int kw = 1;
-  while (kw < 8 && 2 * kw <= steps && tiles * kw < want) kw *= 2;
-  long long splits = 1;
-  if (kw == 8 && tiles * 8 < want)
-    splits = std::max(1LL, std::min((want + tiles * 8 - 1) / (tiles * 8), steps / 16));
-  long long kps = ((p.K + splits - 1) / splits + 15) / 16 * 16;
-  splits = (p.K + kps - 1) / kps;
-  p.k_per_split = kps;
-  p.atomic_out = splits > 1;
-  const long long blocks = (tiles + 8 / kw - 1) / (8 / kw);
-  if (blocks > 0x7fffffffLL) {
+  if (p.M < p.N) p = swapped(p);
+  const F64Plan q = f64_plan(p, wide);
+  if (q.swap) p = swapped(p);
+  if (q.blocks > 0x7fffffffLL) {
     set_error("pcg_contract_f64: M=%lld x N=%lld too large", p.M, p.N);
     return -1;
   }
+  p.k_per_split = (p.K + q.splits - 1) / q.splits;
+  p.atomic_out = q.splits > q.cy;
   if (p.atomic_out)
     if (const int rc = scale_output(p, p.m, p.n, p.M, p.N, beta, st)) return rc;
-  const dim3 grid((unsigned)blocks, (unsigned)splits);
-  const bool wide = p.M > 0x7fffffffLL || p.N > 0x7fffffffLL || p.K > 0x7fffffffLL;
-  auto go = [&](auto kernel) { kernel<<<grid, 256, 0, st>>>(p, kw, nt, tiles); };
-  if (fm == 1 && fn == 1)
-    wide ? go(contract_f64_kernel<1, 1, unsigned long long>) : go(contract_f64_kernel<1, 1, unsigned>);
-  else if (fm == 1)
-    wide ? go(contract_f64_kernel<1, 4, unsigned long long>) : go(contract_f64_kernel<1, 4, unsigned>);
-  else if (fm == 2)
-    wide ? go(contract_f64_kernel<2, 2, unsigned long long>) : go(contract_f64_kernel<2, 2, unsigned>);
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = attr.val.clusterDim.z = 1;
+  attr.val.clusterDim.y = (unsigned)q.cy;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)q.blocks, (unsigned)q.splits);
+  cfg.blockDim = dim3(32 * q.nw);
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = q.cy > 1 ? 1 : 0;
+  auto go = [&](auto kernel) {
+    cudaLaunchKernelEx(&cfg, kernel, (const F64Args)p, q.kw, q.cy, q.tiles_n, q.tiles);
+  };
+  if (q.T == 3)
+    go(contract_dot_kernel<3, unsigned>);
+  else if (q.T == 4)
+    go(contract_dot_kernel<4, unsigned>);
+  else if (wide)
+    go(contract_f64_kernel<4, unsigned long long>);
+  else if (q.R == 2)
+    go(contract_f64_kernel<2, unsigned>);
+  else if (q.R == 3)
+    go(contract_f64_kernel<3, unsigned>);
+  else if (q.R == 4)
+    go(contract_f64_kernel<4, unsigned>);
+  else if (q.R == 5)
+    go(contract_f64_kernel<5, unsigned>);
   else
-    wide ? go(contract_f64_kernel<4, 1, unsigned long long>) : go(contract_f64_kernel<4, 1, unsigned>);
+    go(contract_f64_kernel<6, unsigned>);
   PCG_CHECK_LAUNCH("pcg_contract_f64");
   return 0;
 }
