@@ -9,7 +9,7 @@ seed 2, matched coupling), mixed precision vs plain FP64 on one GB300.
   then K timed iterations.  The integral blocks (tens of GB) exceed L2 every iteration.
 * TFLOP/s uses the pinned per-iteration count of the reference formulation,
   F_iter = 2 o^2 v^4 + 18 o^3 v^3 + 10 o^2 v^3 + 4 o^4 v^2 (counted once for every mode).
-* ``fp64``: the plain FP64 GPU form (DMMA kernels) timed over one iteration at the same size.
+* ``fp64``: the plain FP64 GPU form timed over one iteration at the same size.
 * ``e2e``: whole iterations through the public API (``CCwfn.iterate`` + ``diis_step``, the
   body of ``solve_cc``) with t1/t2 copied in from pinned host memory and back out every step:
   the same work per step as the CPU arm's iteration.
@@ -532,7 +532,7 @@ def main():
     ap.add_argument("--triples-size", type=int, nargs=3, default=None, metavar=("NO", "NV", "SEED"),
                     help="(T) mode at another size (profiling; the measurement is no=30,nv=240)")
     ap.add_argument("--adjoint-sweep", default="tc", choices=["fp64", "tc"],
-                    help="adjoint mode: engine of the tape's sweeps (FP64 DMMA or tensor cores)")
+                    help="adjoint mode: engine of the tape's sweeps (FP64 or tensor cores)")
     ap.add_argument("--cpu-sample", type=int, nargs=3, default=None, metavar=("NO", "NV", "SEED"),
                     help="size of the CPU sample (default no=20, nv=180, seed 1)")
     ap.add_argument("--ref-budget", type=float, default=120.0,

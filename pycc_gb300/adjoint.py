@@ -20,7 +20,7 @@ gives the vector-Jacobian products of the residual:
   applied to an amplitude pair, the reference's ``CCderiv._ccsd_jacobian``
   (``pycc/ccderiv.py:149-180``), exact because every taped op is linear or bilinear.
 
-The sweeps' contractions run on the FP64 DMMA kernel, or, with ``sweep='tc'``, the large
+The sweeps' contractions run on the FP64 path, or, with ``sweep='tc'``, the large
 GEMM-shaped ones on the tcgen05 engine in split-BF16x3.  vvvv-sized cotangents are never
 stored separately: the ladder's adjoint contractions write straight into the gradient
 buffers of tau and of the <ab|ef> block.  ``pycc_gb300.lagrangian`` wraps the sweeps in the
@@ -112,8 +112,8 @@ TC_MIN_FLOPS = 1 << 26     # M*N*K from which a sweep's contraction goes to the 
 class CCSDAdjoint:
     """Tape of the FP64 residual + energy at the amplitudes of a converged ``CCwfn``.
 
-    ``sweep`` selects the engine of the sweeps' contractions: ``'fp64'`` (the FP64 DMMA
-    kernel; the default for ``precision='DP'``) or ``'tc'`` (GEMM-shaped contractions of at
+    ``sweep`` selects the engine of the sweeps' contractions: ``'fp64'`` (the FP64
+    path of ``contract``; the default for ``precision='DP'``) or ``'tc'`` (GEMM-shaped contractions of at
     least ``TC_MIN_FLOPS`` multiply-adds on the tensor cores in split-BF16x3 with separate
     accumulators, the integral blocks as cached static packs; the default for 'MIXED' and
     'SP').  The tape is always recorded from the FP64 residual; for a MIXED / SP wave function

@@ -5,9 +5,10 @@ the same method names, argument orders and return layouts -- ``build_tau``,
 ``build_Fae/Fmi/Fme``, ``build_Wmnij/Wmbej/Wmbje/Zmbij``, ``r_T1``, ``r_T2``, ``residuals``,
 ``cc_energy`` and ``solve_cc`` -- executed by the CUDA library ``libpycc_gb300.so``:
 
-* ``precision='DP'``: every pairwise contraction is one launch of the FP64 strided DMMA
-  kernel (``pcg_contract_f64``) through ``self.contract``; tau builds, the r2
-  symmetrisation, the Jacobi update with its norm and the energy are fused FP64 kernels.
+* ``precision='DP'``: every pairwise contraction goes through ``self.contract``, small ones as
+  one launch of an FP64 kernel (``pcg_contract_f64``), large ones in residue arithmetic on the
+  tensor cores (``pcg_contract_rns_f64``, FP64 accuracy); tau builds, the r2 symmetrisation, the
+  Jacobi update with its norm and the energy are fused FP64 kernels.
 * ``precision='MIXED'``: the residual runs on the tcgen05 tensor-core engine
   (``pycc_gb300.mixed``): BF16 operands with FP32 accumulation (FP8 with per-row scales for
   the <ab|ef> ladder), switching to compensated split-BF16x3 products once the update norm

@@ -2,9 +2,10 @@
 
 ``ContractionBackend.__call__(subscripts, *operands)`` keeps the einsum-string interface of
 ``pycc/device.py:64-87`` (the ``self.contract`` every CCSD builder calls), but executes each
-pairwise contraction as ONE launch of the FP64 strided DMMA kernel in the CUDA library:
-operand and output permutations become element strides, nothing is transposed or copied
-and nothing crosses PCIe/C2C (the reference copies CPU-resident integrals per call,
+pairwise contraction in the CUDA library, as one launch of an FP64 strided kernel or, where that
+is the shorter, as exact integer products modulo sixteen moduli on the tensor cores
+(``csrc/contract_rns.cu``): operand and output permutations become element strides, nothing is
+copied in FP64 and nothing crosses PCIe/C2C (the reference copies CPU-resident integrals per call,
 ``pycc/device.py:71-74``).
 
 Two keyword-only extensions make the builders allocation-free: ``out=`` accumulates into an
@@ -135,7 +136,7 @@ _CALLS = {}
 
 
 def contract_f64(subscripts, a, b, out=None, alpha=1.0, beta=0.0, stream=None):
-    """``out = beta*out + alpha * einsum(subscripts, a, b)`` in FP64: on the FP64 DMMA kernel, or,
+    """``out = beta*out + alpha * einsum(subscripts, a, b)`` in FP64: on the FP64 kernels, or,
     where that is the shorter (``_takes_rns``), on the tensor cores in residue arithmetic."""
     _check(a, "operand 0")
     _check(b, "operand 1")

@@ -1,6 +1,6 @@
 // (T) densities and Lambda sources (pycc/cctriples.py:1063-1157, t3_density), FP64: the two
 // elementwise kernels of one (i, j, k) triple.  The contractions that follow them run on the
-// FP64 DMMA contraction kernel.
+// FP64 contraction path.
 //
 // pcg_t3_ijk_f64: from the connected partials of the triple (P[3][v][v][v], laid out as in the
 // (T) energy: W[a,b,c] = P1[c][a][b] + P2[b][a][c] + P3[a][b][c]) and the integrals, the

@@ -4,7 +4,7 @@ The reference builds eleven HBAR blocks in ``cchbar.__init__`` (``pycc/cchbar.py
 spatial orbitals: ``build_Hov`` ... ``build_Hovoo``, ``:128-858``).  The engine's adjoint does
 not need them -- J x and J^T l are the residual tape's sweeps -- but callers that read the
 blocks themselves (EOM, response) do.  ``HBAR`` builds them on the GPU, in FP64 on the
-engine's DMMA contraction kernel, from the wave function's amplitudes and resident integral
+engine's contraction kernels, from the wave function's amplitudes and resident integral
 blocks, each block on first use (``Hvvvv`` alone is nv^4: 64.8 GB at nv = 300).
 
 Blocks the residual does not read (<am|ef>, <am|ei>, <am|ie> and L_amef) are index

@@ -13,7 +13,8 @@ tensor-core GEMM writes it with coalesced stores.  The energy kernel
 (``csrc/triples.cu``) adds the partials, the disconnected triples (``t3d_ijk``) and the
 Lee-Rendell weights, and accumulates E(T) in FP64.
 
-``precision='DP'`` uses the FP64 DMMA multi-term contraction; the mixed path
+``precision='DP'`` builds batches of triples in residue arithmetic on the tensor cores (or, without
+scratch for a batch, one triple at a time by the FP64 multi-term contraction); the mixed path
 (``t_energy_tc``) builds the partials for batches of triples with the grouped tcgen05 GEMM.
 """
 from __future__ import annotations

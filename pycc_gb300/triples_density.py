@@ -4,7 +4,7 @@
 and to the Lambda residuals of CCSD(T) gradients, and the (T) energy.
 
 For every ordered triple (i, j, k) -- all no^3 of them, as the reference loops -- the connected
-partials of the (T) energy path (``triples.orientation_terms``, FP64 multi-term DMMA
+partials of the (T) energy path (``triples.orientation_terms``, FP64 multi-term
 contraction) and ``pcg_t3_ijk_f64`` give M3 = t3c_ijk / D and N3 = t3d_ijk / D;
 ``pcg_t3_density_terms_f64`` forms their permutation combinations, and the FP64 contraction
 kernel accumulates every density block.  FP64 throughout; the result has the reference's
