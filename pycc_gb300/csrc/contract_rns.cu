@@ -22,9 +22,9 @@
 // A row with an infinity or a NaN (or a column of B) takes its outputs from a plain FP64
 // dot product in step 4, so non-finite inputs give what FP64 arithmetic gives.
 //
-// Measured on GB300 against the FP64 kernel (contract_f64.cu), no = 20, nv = 180: the ladder
-// 'ijef,abef->ijab' 882 -> 21.1 ms (GEMM 11.5, residues 8.1), a ring 'imae,mbej->ijab' 90.8 ->
-// 1.41 ms; at no = 9, nv = 53 3.2 -> 0.18 ms and 0.46 -> 0.09 ms.
+// Measured on GB300 against the FP64 pipe at its peak rate, no = 20, nv = 180: the ladder
+// 'ijef,abef->ijab' 727 -> 19.8 ms (GEMM 11.1, residues 7.2), a ring 'imae,mbej->ijab' 81 -> 1.33
+// ms; at no = 9, nv = 53 2.2 -> 0.16 ms and 0.20 -> 0.05 ms.
 //
 // The offsets of strided rows, columns and K indices are expanded into tables once per call;
 // operands larger than the workspace go through in panels of rows, columns or K.
@@ -310,7 +310,7 @@ extern "C" int pcg_contract_rns_f64(int m_n, const long long* m_ext, const long 
         const long long mm = std::min(p.PM, M - m0);
         // B's panel is packed with the first panel of A
         PackArgs q{{{a, m0, mm, pa, 0, 0}, {b, n0, m0 == 0 ? nn : 0, pb, 0, 0}}, k0, kn, p.Kp, log2k,
-                   t.mod};
+                   t.pairs};
         if (run_pack(q, st)) return -2;
         GemmArgs g{};
         g.M = mm;

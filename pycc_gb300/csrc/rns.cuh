@@ -6,6 +6,7 @@
 #include <cuda_bf16.h>
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 
 namespace pcg {
 namespace rns {
@@ -31,6 +32,10 @@ constexpr float kMagic = 12582912.f;  // 1.5 * 2^23: adding it rounds to an inte
 struct ModTab {
   float p[NM], inv[NM], c1[NM], c2[NM], c3[NM];
 };
+// ModTab's entries twice each (np: -p), for arithmetic on pairs.
+struct PairTab {
+  unsigned long long np[NM], inv[NM], c1[NM], c2[NM], c3[NM];
+};
 // Per modulus floor(2^96 q / p), q = ((P / p)^-1 mod p), in three 32-bit words; b: what the
 // bias of the stored bytes adds, negated; scale = P 2^-96.
 struct CrtTab {
@@ -39,20 +44,43 @@ struct CrtTab {
 };
 static_assert(NM * 8 <= 128, "the product fits a 128-bit integer");
 
-// Nearest residue of an integer-valued t, |t| < 2^24: FP32's 1/p is off by at most 2^-24.4
-// relative, so the quotient is off its nearest integer by less than 0.5 + 0.0027 and |r| <= 127
-// (128 for p = 256).
-__device__ __forceinline__ float mod_near(float t, float p, float inv) {
-  const float q = fmaf(t, inv, kMagic) - kMagic;
-  return fmaf(-p, q, t);
-}
-
 // Four residues as bytes r + 128 (modulo 256).
 __device__ __forceinline__ unsigned residue_bytes(float a, float b, float c, float d) {
   constexpr float bias = 8388608.f + 128.f;
   return __byte_perm(
       __byte_perm(__float_as_uint(a + bias), __float_as_uint(b + bias), 0x0040),
       __byte_perm(__float_as_uint(c + bias), __float_as_uint(d + bias), 0x0040), 0x5410);
+}
+
+// Two FP32 values in one register pair; each half is rounded as the scalar operation's.
+__device__ __forceinline__ unsigned long long pair(float a, float b) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpair(unsigned long long v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long fma_pair(unsigned long long a, unsigned long long b,
+                                                       unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ unsigned long long add_pair(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// Nearest residues of two integer-valued t, |t| < 2^24, with (-p, -p) and (1/p, 1/p): FP32's 1/p is
+// off by at most 2^-24.4 relative, so the quotient is off its nearest integer by less than 0.5 +
+// 0.0027 and |r| <= 127 (128 for p = 256).
+__device__ __forceinline__ unsigned long long mod_near_pair(unsigned long long t,
+                                                            unsigned long long np,
+                                                            unsigned long long inv) {
+  const unsigned long long q =
+      add_pair(fma_pair(t, inv, pair(kMagic, kMagic)), pair(-kMagic, -kMagic));
+  return fma_pair(np, q, t);
 }
 
 struct Operand {
@@ -218,8 +246,8 @@ __device__ __forceinline__ int row_shift(const Operand& o, long long row, int lo
   return (kBits2 - log2k - 2 * (max((int)o.top[row], 1) - 1022)) >> 1;
 }
 
-// The four digits (with the sign) of x 2^s rounded to an integer of at most 62 bits.
-__device__ __forceinline__ void digits(double x, int s, unsigned flip, float (&d)[4]) {
+// The magnitude of x 2^s rounded to an integer of at most 62 bits, and its sign as +-1.
+__device__ __forceinline__ unsigned long long scaled(double x, int s, unsigned flip, float& sign) {
   const unsigned hi = (unsigned)__double2hiint(x) ^ flip, lo = (unsigned)__double2loint(x);
   const unsigned ex = (hi >> 20) & 0x7ffu;
   const unsigned mh = (hi & 0xfffffu) | (ex ? 1u << 20 : 0u);
@@ -227,13 +255,23 @@ __device__ __forceinline__ void digits(double x, int s, unsigned flip, float (&d
   // by 9 - sh from 10 bits up, then rounded off by the last.  A shift past 63 leaves 0, as does
   // the exponent of an infinity or a NaN, whose row takes its outputs from the FP64 dot product.
   const unsigned r = min((unsigned)(9 + 1075 - s - (int)max(ex, 1u)), 63u);
-  unsigned long long m = (((unsigned long long)mh << 32) | lo) << 10;
-  m = ((m >> r) + 1ull) >> 1;
-  const float sign = __uint_as_float(0x3f800000u | (hi & 0x80000000u));
+  const unsigned long long m = (((unsigned long long)mh << 32) | lo) << 10;
+  sign = __uint_as_float(0x3f800000u | (hi & 0x80000000u));
+  return ((m >> r) + 1ull) >> 1;
+}
+
+// The four digits (with the sign) of two such integers.
+__device__ __forceinline__ void digits(double x, double y, int s, unsigned flip,
+                                       unsigned long long (&d)[4]) {
+  float sx, sy;
+  const unsigned long long m = scaled(x, s, flip, sx), n = scaled(y, s, flip, sy);
+  const unsigned long long sign = pair(sx, sy), low = pair(-8388608.f * sx, -8388608.f * sy);
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
-    const unsigned v = (unsigned)(m >> digit_bit(q)) & ((1u << (digit_bit(q + 1) - digit_bit(q))) - 1);
-    d[q] = fmaf(__uint_as_float(0x4b000000u | v), sign, -8388608.f * sign);
+    const unsigned mask = (1u << (digit_bit(q + 1) - digit_bit(q))) - 1;
+    d[q] = fma_pair(pair(__uint_as_float(0x4b000000u | ((unsigned)(m >> digit_bit(q)) & mask)),
+                         __uint_as_float(0x4b000000u | ((unsigned)(n >> digit_bit(q)) & mask))),
+                    sign, low);
   }
 }
 
@@ -249,39 +287,42 @@ struct PackArgs {
   PackSide s[2];
   long long k0, K, Kp;  // K indices [k0, k0 + K), padded with zeros to Kp
   int log2k;            // ceil(log2 K)
-  ModTab t;
+  PairTab t;
 };
 
-// Residues of four neighbouring K entries for every modulus, one 64-bit store per modulus: an
-// integer of at most 8 bits is exact in the upper half of its FP32 word, which is BF16.
+// Residues of eight neighbouring K entries for every modulus, two to an instruction and one
+// 128-bit store per modulus: an integer of at most 8 bits is exact in the upper half of its FP32
+// word, which is BF16.
 __device__ __forceinline__ void store_residues(const PackArgs& p, const PackSide& o,
-                                               const double (&x)[4], int s, long long at) {
-  float d[4][4];
+                                               const double (&x)[8], int s, long long at) {
+  unsigned long long d[4][4];
 #pragma unroll
-  for (int e = 0; e < 4; ++e) digits(x[e], s, o.flip, d[e]);
-  uint2* out = reinterpret_cast<uint2*>(o.out + at);
-  const long long plane = (o.nrow * p.Kp) >> 2;
+  for (int e = 0; e < 4; ++e) digits(x[2 * e], x[2 * e + 1], s, o.flip, d[e]);
+  uint4* out = reinterpret_cast<uint4*>(o.out + at);
+  const long long plane = (o.nrow * p.Kp) >> 3;
 #pragma unroll
   for (int l = 0; l < NM; ++l, out += plane) {
     unsigned r[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      const float t = fmaf(d[e][3], p.t.c3[l],
-                           fmaf(d[e][2], p.t.c2[l], fmaf(d[e][1], p.t.c1[l], d[e][0])));
-      r[e] = __float_as_uint(mod_near(t, p.t.p[l], p.t.inv[l]));
+      float a, b;
+      const unsigned long long t =
+          fma_pair(d[e][3], p.t.c3[l],
+                   fma_pair(d[e][2], p.t.c2[l], fma_pair(d[e][1], p.t.c1[l], d[e][0])));
+      unpair(mod_near_pair(t, p.t.np[l], p.t.inv[l]), a, b);
+      r[e] = __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
     }
-    *out = make_uint2(__byte_perm(r[0], r[1], 0x7632), __byte_perm(r[2], r[3], 0x7632));
+    __stcs(out, make_uint4(r[0], r[1], r[2], r[3]));
   }
 }
 
-// Operand -> residues: 8 bytes read and 2 NM written per element, about 150 instructions; bound
-// by the writes and, not far behind, by instruction issue.  A half warp takes 64 K of a row, four
-// neighbouring K a lane.  Gathered along K it loads them straight from global memory, two rows a
-// half warp; otherwise a tile of 64 walked rows x 64 K goes through shared memory, read along the
-// rows.  One launch packs a panel of each operand: the first blocks take A's, the others B's.
-// 8.1 ms at 1.05e9 elements (5.2 TB/s) against 9.5 with 250 instructions an element (two K a
-// lane, 64-bit tile indices, branches on the shift's sign).
-static __global__ void __launch_bounds__(256, 5)
+// Operand -> residues: 8 bytes read and 2 NM written per element, about 85 instructions; bound by
+// the writes.  A quarter warp takes 64 K of a row, eight neighbouring K a lane.  Gathered along K
+// it loads them straight from global memory; otherwise a tile of 64 walked rows x 64 K goes through
+// shared memory, read along the rows.  One launch packs a panel of each operand: the first blocks
+// take A's, the others B's.  163e6 elements: 1.07 ms (6.1 TB/s) against 1.15 with one element to
+// an instruction and 1.20 with four K a lane as well.
+static __global__ void __launch_bounds__(256, 4)
     rns_pack_kernel(const __grid_constant__ PackArgs p) {
   __shared__ double tile[64][65];
   __shared__ long long off[64], kof[64];
@@ -293,28 +334,21 @@ static __global__ void __launch_bounds__(256, 5)
   const unsigned nk = (unsigned)(p.Kp >> 6), bw = b / nk;
   const long long w = (long long)bw * (o.kfast ? 32 : 64);  // first row of the block
   const long long kk0 = (long long)(b - bw * nk) * 64;      // first K, in the panel
-  const int half = threadIdx.x >> 4, kk = 4 * (threadIdx.x & 15);
+  const int half = threadIdx.x >> 3, kk = 8 * (threadIdx.x & 7);
   if (o.kfast) {
-    const long long w1 = w + 2 * half;
-    double x[2][4];
-    int row[2];
+    if (w + half < ps.nrow) {
+      const int row = o.walk[ps.w0 + w + half];
+      const double* q = o.X + o.off[row];
+      double x[8];
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      row[u] = w1 + u < ps.nrow ? o.walk[ps.w0 + w1 + u] : -1;
-      const double* q = o.X + (row[u] >= 0 ? o.off[row[u]] : 0);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
+      for (int e = 0; e < 8; ++e) {
         const long long k = kk0 + kk + e;
-        x[u][e] = row[u] >= 0 && k < p.K ? __ldg(q + k_offset(o, p.k0 + k)) : 0.0;
+        x[e] = k < p.K ? __ldg(q + k_offset(o, p.k0 + k)) : 0.0;
       }
+      const int sh = row_shift(o, row, p.log2k);
+      if (o.sh && kk0 + kk == 0) o.sh[row] = o.top[row] == 2047u ? kNotFinite : sh;
+      store_residues(p, ps, x, sh, (row - ps.w0) * p.Kp + kk0 + kk);
     }
-#pragma unroll
-    for (int u = 0; u < 2; ++u)
-      if (row[u] >= 0) {
-        const int sh = row_shift(o, row[u], p.log2k);
-        if (o.sh && kk0 + kk == 0) o.sh[row[u]] = o.top[row[u]] == 2047u ? kNotFinite : sh;
-        store_residues(p, ps, x[u], sh, (row[u] - ps.w0) * p.Kp + kk0 + kk);
-      }
   } else {
     if (threadIdx.x < 64) {
       kof[threadIdx.x] = kk0 + threadIdx.x < p.K ? k_offset(o, p.k0 + kk0 + threadIdx.x) : 0;
@@ -339,8 +373,10 @@ static __global__ void __launch_bounds__(256, 5)
     for (int u = 0; u < 16; ++u) tile[rr][(threadIdx.x >> 6) + 4 * u] = v[u];
     __syncthreads();
 #pragma unroll 1
-    for (int r = half; r < 64 && w + r < ps.nrow; r += 16) {
-      const double x[4] = {tile[r][kk], tile[r][kk + 1], tile[r][kk + 2], tile[r][kk + 3]};
+    for (int r = half; r < 64 && w + r < ps.nrow; r += 32) {
+      double x[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) x[e] = tile[r][kk + e];
       store_residues(p, ps, x, ssh[r], (srow[r] - ps.w0) * p.Kp + kk0 + kk);
     }
   }
@@ -449,9 +485,10 @@ __device__ __forceinline__ Unit decode_unit(const GemmArgs& p, unsigned u) {
 // Persistent and warp-specialised: warp 0 TMA, warp 1 MMA, warps 2-9 epilogue (a TMEM lane
 // quarter and a column half each).  The two TMEM accumulators alternate between chunks of
 // kChunk K blocks; the epilogue warps add each chunk to their running residues (BN / 2
-// registers per thread) and reduce modulo p while the other accumulator fills: four FP32
-// instructions per element and chunk.  Every wait is bounded; an expired one leaves its code in
-// *status and the caller's outputs become NaN.
+// registers per thread) and reduce modulo p while the other accumulator fills: two FP32
+// instructions per element and chunk.  3600 x 3600 x 3600: 921 us (1.62 PFLOP/s) against 993 with
+// four, 3600 x 3600 x 400 159 against 180.  Every wait is bounded; an expired one leaves its code
+// in *status and the caller's outputs become NaN.
 template <int BN, bool TRIP>
 static __global__ void __launch_bounds__(kGemmThreads, 1)
     rns_gemm_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ GemmArgs p,
@@ -584,10 +621,11 @@ static __global__ void __launch_bounds__(kGemmThreads, 1)
     bool stop = false;
     for (unsigned u = blockIdx.x; u < units && !stop; u += gridDim.x) {
       const Unit x = decode_unit<TRIP, false>(p, u);
-      const float pm = p.t.p[x.mod], inv = p.t.inv[x.mod];
-      float r[HB];
+      const unsigned long long np = pair(-p.t.p[x.mod], -p.t.p[x.mod]),
+                               inv = pair(p.t.inv[x.mod], p.t.inv[x.mod]);
+      unsigned long long r[HB / 2];  // two columns each
 #pragma unroll
-      for (int j = 0; j < HB; ++j) r[j] = 0.f;
+      for (int j = 0; j < HB / 2; ++j) r[j] = 0;
       for (int k0 = 0; k0 < x.blocks; k0 += kChunk, ++c) {
         const int b = c & 1;
         int okw = 1;
@@ -611,8 +649,11 @@ static __global__ void __launch_bounds__(kGemmThreads, 1)
           uint32_t v[32];
           tmem_ld32(tbase + 32 * f, v);
 #pragma unroll
-          for (int j = 0; j < 32; ++j)
-            r[32 * f + j] = mod_near(__uint_as_float(v[j]) + r[32 * f + j], pm, inv);
+          for (int j = 0; j < 16; ++j)
+            r[16 * f + j] = mod_near_pair(
+                add_pair(pair(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1])),
+                         r[16 * f + j]),
+                np, inv);
         }
         tc_fence_before();
         __syncwarp();
@@ -626,7 +667,9 @@ static __global__ void __launch_bounds__(kGemmThreads, 1)
         for (int f = 0; f < HB / 16; ++f) {
           const int cj = h * HB + 16 * f;  // 16 columns: inside the tile and the row, or not at all
           if (cj < p.bs && x.n0 + cj < p.ld) {
-            const float* e = r + 16 * f;
+            float e[16];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) unpair(r[8 * f + j], e[2 * j], e[2 * j + 1]);
             *reinterpret_cast<uint4*>(o + x.n0 + cj) =
                 make_uint4(residue_bytes(e[0], e[1], e[2], e[3]),
                            residue_bytes(e[4], e[5], e[6], e[7]),
@@ -706,6 +749,7 @@ struct CrtSum {
 // ---- host side --------------------------------------------------------------------------
 struct Tables {
   ModTab mod;
+  PairTab pairs;
   CrtTab crt;
 };
 
@@ -722,6 +766,16 @@ inline const Tables& tables() {
       x.mod.c1[l] = sym(1ll << digit_bit(1));
       x.mod.c2[l] = sym(1ll << digit_bit(2));
       x.mod.c3[l] = sym(1ll << digit_bit(3));
+      auto twice = [](float f) {
+        unsigned u;
+        std::memcpy(&u, &f, 4);
+        return (unsigned long long)u << 32 | u;
+      };
+      x.pairs.np[l] = twice(-x.mod.p[l]);
+      x.pairs.inv[l] = twice(x.mod.inv[l]);
+      x.pairs.c1[l] = twice(x.mod.c1[l]);
+      x.pairs.c2[l] = twice(x.mod.c2[l]);
+      x.pairs.c3[l] = twice(x.mod.c3[l]);
       const unsigned m = (unsigned)((P / (unsigned)p) % (unsigned)p);
       unsigned q = 1;
       while ((q * m) % p != 1) ++q;

@@ -231,7 +231,7 @@ extern "C" int pcg_t3_rns_pack(const double* V, const double* O, const double* t
   for (auto& x : pass) {
     PackArgs a{{{x.a, 0, x.a.R, (__nv_bfloat16*)(w + x.pa), 0, 0},
                 {x.b, 0, x.b.R, (__nv_bfloat16*)(w + x.pb), x.b.X == O ? 0x80000000u : 0u, 0}},
-               0, x.K, x.Kp, 0, tables().mod};
+               0, x.K, x.Kp, 0, tables().pairs};
     if (run_pack(a, st)) return -2;
   }
   return 0;
