@@ -568,7 +568,7 @@ struct PackArgs {
 // six sources are decomposed (or read from the tables) once per tile into shared memory;
 // values are gathered along whichever index is unit-stride in X (kfast) and written out
 // along K, so both the FP64 reads and the packed writes are coalesced.  The value type V is
-// double for BF16x6 (three pieces carry 24 bits) and float otherwise: FP64 inputs are
+// double for BF16x6 (three pieces carry 24 bits; split in integer arithmetic) and float otherwise: FP64 inputs are
 // rounded to FP32 in integer arithmetic (f64_to_f32) and combined and split in FP32, which
 // keeps the kernel a stream instead of a loop on GB300's FP64 pipe.  A BF16 hi/lo pair
 // holds 16 bits, so the FP32 rounding (2^-24 of the operands) is far below the split's own
@@ -657,7 +657,10 @@ __device__ __forceinline__ void pack_tile_load(const PackArgs& p, PackTile<V>& t
       // each source's walked offset is read inside its (block-uniform) branch, so an
       // operand with X alone reads one offset per element
       auto wof = [&](int src) { return KF ? t.rof[src][wv] : t.kof[src][wv]; };
-      if (p.X) v = a * pack_ld<V>(p.X + f[0] + wof(0));
+      if (p.X) {
+        v = pack_ld<V>(p.X + f[0] + wof(0));
+        if (sizeof(V) == 4 || a != (V)1) v *= a;  // an FP64 product is 64 clocks
+      }
       if (p.Y) v += b * pack_ld<V>(p.Y + f[1] + wof(1));
       if (p.k_w) v *= KF ? t.kw[fx] : t.kw[wv];
     }
@@ -731,27 +734,74 @@ __global__ void __launch_bounds__(PACK_THREADS, 8) pack_bf16_kernel(const PackAr
   }
 }
 
-// Split-BF16x6 (hi, mid, lo) from an FP64 tile.
+// The next BF16 piece of (-1)^neg A 2^(e - 1075): A rounded to its eight leading bits, ties to
+// even; A and neg become the remainder's.
+__device__ __forceinline__ unsigned bf16_piece(unsigned& neg, unsigned long long& A, int e) {
+  if (A == 0) return 0u;
+  const int lz = __clzll((long long)A) - 1;  // A < 2^63
+  const unsigned long long B = A << lz;
+  const unsigned q = (unsigned)((B + ((1ull << 54) - 1) + ((B >> 55) & 1u)) >> 55);  // 128..256
+  const unsigned bits = (neg << 15) | (((unsigned)(e + 63 - lz - 949) << 7) + q - 128u);
+  const long long rest = (long long)(B - ((unsigned long long)q << 55));
+  neg ^= (unsigned)(rest < 0);
+  A = (unsigned long long)(rest < 0 ? -rest : rest) >> lz;
+  return bits;
+}
+
+// hi = bf16(v), mid = bf16(v - hi), lo = bf16(v - hi - mid), each rounded to nearest even, in
+// integer arithmetic: in FP64 the conversions and subtractions held up 64 clocks of an SM quarter
+// each.  Outside 2^-73 .. 2^126, where a piece may leave BF16's normal range, in FP64.
+__device__ __forceinline__ void split_bf16x6(double v, unsigned& hi, unsigned& mid, unsigned& lo) {
+  const unsigned long long u = (unsigned long long)__double_as_longlong(v);
+  const int e = (int)(u >> 52) & 0x7ff;
+  if (e >= 950 && e <= 1148) {
+    unsigned neg = (unsigned)(u >> 63);
+    unsigned long long A = (u & 0xfffffffffffffull) | (1ull << 52);
+    hi = bf16_piece(neg, A, e);
+    mid = bf16_piece(neg, A, e);
+    lo = bf16_piece(neg, A, e);
+  } else if ((u << 1) == 0) {
+    hi = (unsigned)(u >> 63) << 15;
+    mid = lo = 0;
+  } else {
+    const __nv_bfloat16 h = __double2bfloat16(v);
+    double rest = v - (double)__bfloat162float(h);
+    const __nv_bfloat16 m = __double2bfloat16(rest);
+    rest -= (double)__bfloat162float(m);
+    hi = __bfloat16_as_ushort(h);
+    mid = __bfloat16_as_ushort(m);
+    lo = __bfloat16_as_ushort(__double2bfloat16(rest));
+  }
+}
+
+// Split-BF16x6 (hi, mid, lo) from an FP64 tile, two adjacent K entries per thread as in
+// pack_bf16_kernel.  no = 12, nv = 71: packs of 11-37 us that took 20-64 with the split in FP64 and
+// two-byte stores; the single-precision-class residual at no = 15, nv = 109 3.22 -> 2.79 ms.
 template <bool KF>
 __global__ void __launch_bounds__(PACK_THREADS) pack_bf16x6_kernel(const PackArgs p) {
   __shared__ PackTile<double> t;
   const long long r0 = (long long)blockIdx.x * TR, k0 = (long long)blockIdx.y * TK;
   pack_tile_load<double, KF>(p, t, r0, k0);
-  __nv_bfloat16* hi = reinterpret_cast<__nv_bfloat16*>(p.hi);
-  __nv_bfloat16* mid = reinterpret_cast<__nv_bfloat16*>(p.mid);
-  __nv_bfloat16* lo = reinterpret_cast<__nv_bfloat16*>(p.lo);
-  for (int e = threadIdx.x; e < TR * TK; e += PACK_THREADS) {
-    const int rr = e / TK, kk = e % TK;
-    if (r0 + rr >= p.R) continue;
+  const int kk = 2 * (threadIdx.x & 31);
+  // a caller's buffers may be 2-byte aligned only
+  const bool words = (((uintptr_t)p.hi | (uintptr_t)p.mid | (uintptr_t)p.lo) & 3) == 0;
+  auto put = [words](void* base, long long at, unsigned a, unsigned b) {
+    if (words) {
+      reinterpret_cast<unsigned*>(base)[at >> 1] = a | (b << 16);
+    } else {
+      reinterpret_cast<unsigned short*>(base)[at] = (unsigned short)a;
+      reinterpret_cast<unsigned short*>(base)[at + 1] = (unsigned short)b;
+    }
+  };
+  for (int rr = threadIdx.x >> 5; rr < TR; rr += PACK_THREADS / 32) {
+    if (r0 + rr >= p.R) break;
     const long long at = t.orow[rr] * p.Kp + k0 + kk;
-    const double v = t.v[rr][kk];
-    const __nv_bfloat16 h = __double2bfloat16(v);
-    hi[at] = h;
-    double rest = v - (double)__bfloat162float(h);
-    const __nv_bfloat16 m = __double2bfloat16(rest);
-    mid[at] = m;
-    rest -= (double)__bfloat162float(m);
-    lo[at] = __double2bfloat16(rest);
+    unsigned h[2], m[2], l[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) split_bf16x6(t.v[rr][kk + e], h[e], m[e], l[e]);
+    put(p.hi, at, h[0], h[1]);
+    put(p.mid, at, m[0], m[1]);
+    put(p.lo, at, l[0], l[1]);
   }
 }
 
