@@ -278,14 +278,15 @@ __device__ __forceinline__ void digits(double x, double y, int s, unsigned flip,
 struct PackSide {
   Operand o;
   long long w0, nrow;  // rows of this panel: walk positions [w0, w0 + nrow); nrow 0: none
-  __nv_bfloat16* out;  // [modulus][nrow][Kp]
+  __nv_bfloat16* out;  // [modulus][nrow][ld]
   unsigned flip;       // 0x80000000: the negated operand
   long long blocks;
 };
 
 struct PackArgs {
   PackSide s[2];
-  long long k0, K, Kp;  // K indices [k0, k0 + K), padded with zeros to Kp
+  long long k0, K;      // K indices [k0, k0 + K)
+  long long width, ld;  // columns written, zeros from K on, of each row's ld (multiples of 8)
   int log2k;            // ceil(log2 K)
   PairTab t;
 };
@@ -299,7 +300,7 @@ __device__ __forceinline__ void store_residues(const PackArgs& p, const PackSide
 #pragma unroll
   for (int e = 0; e < 4; ++e) digits(x[2 * e], x[2 * e + 1], s, o.flip, d[e]);
   uint4* out = reinterpret_cast<uint4*>(o.out + at);
-  const long long plane = (o.nrow * p.Kp) >> 3;
+  const long long plane = (o.nrow * p.ld) >> 3;
 #pragma unroll
   for (int l = 0; l < NM; ++l, out += plane) {
     unsigned r[4];
@@ -331,12 +332,12 @@ static __global__ void __launch_bounds__(256, 4)
   const PackSide& ps = p.s[side];
   const Operand& o = ps.o;
   const unsigned b = blockIdx.x - (side ? (unsigned)p.s[0].blocks : 0u);
-  const unsigned nk = (unsigned)(p.Kp >> 6), bw = b / nk;
+  const unsigned nk = (unsigned)((p.width + 63) >> 6), bw = b / nk;
   const long long w = (long long)bw * (o.kfast ? 32 : 64);  // first row of the block
   const long long kk0 = (long long)(b - bw * nk) * 64;      // first K, in the panel
   const int half = threadIdx.x >> 3, kk = 8 * (threadIdx.x & 7);
   if (o.kfast) {
-    if (w + half < ps.nrow) {
+    if (w + half < ps.nrow && kk0 + kk < p.width) {
       const int row = o.walk[ps.w0 + w + half];
       const double* q = o.X + o.off[row];
       double x[8];
@@ -347,7 +348,7 @@ static __global__ void __launch_bounds__(256, 4)
       }
       const int sh = row_shift(o, row, p.log2k);
       if (o.sh && kk0 + kk == 0) o.sh[row] = o.top[row] == 2047u ? kNotFinite : sh;
-      store_residues(p, ps, x, sh, (row - ps.w0) * p.Kp + kk0 + kk);
+      store_residues(p, ps, x, sh, (row - ps.w0) * p.ld + kk0 + kk);
     }
   } else {
     if (threadIdx.x < 64) {
@@ -373,11 +374,11 @@ static __global__ void __launch_bounds__(256, 4)
     for (int u = 0; u < 16; ++u) tile[rr][(threadIdx.x >> 6) + 4 * u] = v[u];
     __syncthreads();
 #pragma unroll 1
-    for (int r = half; r < 64 && w + r < ps.nrow; r += 32) {
+    for (int r = half; r < 64 && w + r < ps.nrow && kk0 + kk < p.width; r += 32) {
       double x[8];
 #pragma unroll
       for (int e = 0; e < 8; ++e) x[e] = tile[r][kk + e];
-      store_residues(p, ps, x, ssh[r], (srow[r] - ps.w0) * p.Kp + kk0 + kk);
+      store_residues(p, ps, x, ssh[r], (srow[r] - ps.w0) * p.ld + kk0 + kk);
     }
   }
 }
@@ -385,7 +386,7 @@ static __global__ void __launch_bounds__(256, 4)
 // ---- GEMM over the residues -------------------------------------------------------------
 // Output tiles and K of a launch.  Plain: C[split][modulus] = A B^T over K blocks
 // [split kb_per_split, ...).  Triples (TRIP): group g = 3 t + q is orientation q of triple t,
-// the sum of four products of row blocks (pycc_gb300/triples.py, orientation_terms).
+// the sum of two products of row blocks (csrc/triples_rns.cu).
 struct GemmArgs {
   long long M, N;    // rows of A and of B in this panel (TRIP: v^2 and v)
   long long mt, nt;  // 128-row and bs-column tiles
@@ -400,12 +401,12 @@ struct GemmArgs {
   ModTab t;
   // TRIP
   const int* ijk;  // [triples][3]
-  int no, kv, ko;  // occupied orbitals, K blocks of the products over e and over m
+  int no, kc;      // occupied orbitals, K blocks of a product over e and m
 };
 
 struct GemmMaps {
-  CUtensorMap a[4];  // TRIP: VT, VN, TM, TMT
-  CUtensorMap b[2];  // TRIP: T2P, OB
+  CUtensorMap a[2];  // TRIP: [VT | TM], [VN | TMT]
+  CUtensorMap b[1];  // TRIP: [T2P | OB]
 };
 
 constexpr int kEpiWarps = 8;
@@ -423,11 +424,11 @@ struct RSmem {
   static_assert(BN == 64 || BN == 128 || BN == 256, "two accumulators in a power of two columns");
 };
 
-// One unit of work: an output tile of one modulus, the sum of up to four runs of K blocks.
+// One unit of work: an output tile of one modulus, the sum of up to two runs of K blocks.
 struct Unit {
   int plane, mod, n0, blocks;  // plane: split or group; blocks: K blocks in all
   long long m0;
-  int nseg, ma[4], mb[4], ya[4], yb[4], kb[4], nk[4];
+  int ma[2], mb[2], ya[2], yb[2], kb[2], nk[2];
 };
 
 // Unit u -> (modulus, split or group, tile): neighbouring groups share row blocks of one
@@ -447,7 +448,6 @@ __device__ __forceinline__ Unit decode_unit(const GemmArgs& p, unsigned u) {
   x.m0 = (long long)(group * gm + (rg - n * here)) * BM;
   x.n0 = (int)n * p.bs;
   if (!TRIP) {
-    x.nseg = 1;
     x.kb[0] = x.plane * p.kb_per_split;
     x.blocks = x.nk[0] = min(p.nkb, x.kb[0] + p.kb_per_split) - x.kb[0];
     if (SEGS) {
@@ -457,26 +457,22 @@ __device__ __forceinline__ Unit decode_unit(const GemmArgs& p, unsigned u) {
     }
     return x;
   }
-  x.nseg = 4;
-  x.blocks = 2 * (p.kv + p.ko);
+  x.blocks = 2 * p.kc;
   if (SEGS) {
     const int q = x.plane % 3;
     const int i = p.ijk[x.plane - q], j = p.ijk[x.plane - q + 1], k = p.ijk[x.plane - q + 2];
     // (A map, its occupied index, the pair of B's row block) per product
     const int s0 = q == 2 ? k : i, s1 = q == 0 ? j : (q == 1 ? k : j);
-    const int bx[4] = {q == 0 ? k : (q == 1 ? j : i), q == 0 ? k : (q == 1 ? j : i),
-                       q == 0 ? j : (q == 1 ? k : j), q == 0 ? i : (q == 1 ? i : k)};
-    const int by[4] = {q == 0 ? j : (q == 1 ? k : j), q == 0 ? i : (q == 1 ? i : k),
-                       q == 0 ? k : (q == 1 ? j : i), q == 0 ? k : (q == 1 ? j : i)};
-    const int ma[4] = {q == 2 ? 1 : 0, q == 2 ? 0 : 1, q == 2 ? 3 : 2, q == 2 ? 2 : 3};
+    const int bx = q == 0 ? k : (q == 1 ? j : i);
+    const int by[2] = {q == 0 ? j : (q == 1 ? k : j), q == 0 ? i : (q == 1 ? i : k)};
 #pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      x.ma[s] = ma[s];
-      x.mb[s] = s >> 1;
-      x.ya[s] = (int)(((long long)x.mod * p.no + ((s & 1) ? s1 : s0)) * p.M + x.m0);
-      x.yb[s] = (int)(((long long)x.mod * p.no * p.no + bx[s] * p.no + by[s]) * p.N + x.n0);
+    for (int s = 0; s < 2; ++s) {
+      x.ma[s] = (q == 2) != (s == 1);
+      x.mb[s] = 0;
+      x.ya[s] = (int)(((long long)x.mod * p.no + (s ? s1 : s0)) * p.M + x.m0);
+      x.yb[s] = (int)(((long long)x.mod * p.no * p.no + bx * p.no + by[s]) * p.N + x.n0);
       x.kb[s] = 0;
-      x.nk[s] = s < 2 ? p.kv : p.ko;
+      x.nk[s] = p.kc;
     }
   }
   return x;
@@ -541,7 +537,7 @@ static __global__ void __launch_bounds__(kGemmThreads, 1)
       for (unsigned u = blockIdx.x; u < units && !stop; u += gridDim.x) {
         const Unit x = decode_unit<TRIP, true>(p, u);
 #pragma unroll
-        for (int g = 0; g < (TRIP ? 4 : 1); ++g) {
+        for (int g = 0; g < (TRIP ? 2 : 1); ++g) {
           const CUtensorMap* ta = &maps.a[x.ma[g]];
           const CUtensorMap* tb = &maps.b[x.mb[g]];
           for (int kb = x.kb[g]; kb < x.kb[g] + x.nk[g] && !stop; ++kb, ++it) {
@@ -835,7 +831,7 @@ inline int run_norm(const Operand& a, const Operand& b, long long k0, long long 
 inline int run_pack(PackArgs& p, cudaStream_t st) {
   for (PackSide& s : p.s) {
     const int rows = s.o.kfast ? 32 : 64;
-    s.blocks = (p.Kp >> 6) * ((s.nrow + rows - 1) / rows);
+    s.blocks = ((p.width + 63) >> 6) * ((s.nrow + rows - 1) / rows);
   }
   rns_pack_kernel<<<(unsigned)(p.s[0].blocks + p.s[1].blocks), 256, 0, st>>>(p);
   PCG_CHECK_LAUNCH("rns pack");

@@ -6,14 +6,17 @@
 //   A side (rows (x, p, q)):  VT = <qp|ex>,  VN = <pq|ex>  (K = e);  TM = t2_xmpq,
 //                             TMT = t2_xmqp  (K = m)
 //   B side (rows (x, y, p)):  T2P = t2_xype  (K = e);  OB = -<mp|xy>  (K = m)
-// One GEMM launch computes the three orientations of a batch of triples, each the sum of four
-// products (pycc_gb300/triples.py, orientation_terms) in one accumulator: a sum of residues is
-// the residue of the sum when all four products carry the same scale, so a matrix has one power
-// of two for all its rows, chosen from its largest row norm so that the sum of the four stays
-// below half the product of the moduli.  A second kernel rebuilds the partials in FP64, in the
-// layout the energy kernel reads.  E(T) at no = 7, nv = 45: 63.4 ms with one FP64 launch per
+// An orientation is a sum of four products (pycc_gb300/triples.py, orientation_terms), in which VT
+// meets T2P's rows (y, z) where TM of the same index meets OB's (z, y), and VN and TMT likewise.
+// So the residues are stored side by side along K, [VT | TM], [VN | TMT] and [T2P | OB with x and y
+// exchanged], and an orientation is two products of K = nv + no: at no = 7, nv = 45 two 64-K
+// blocks in place of four.  The residue of the sum is the sum's when all four products carry the
+// same scale, so a matrix has one power of two for all its rows, chosen from its largest row norm
+// so that the sum of the four stays below half the product of the moduli.  One GEMM launch computes
+// the three orientations of a batch of triples, a second kernel rebuilds the partials in FP64, in
+// the layout the energy kernel reads.  E(T) at no = 7, nv = 45: 63.4 ms with one FP64 launch per
 // triple and orientation (46.6 ms on a few SMs' FP64 pipes, a host synchronisation per triple),
-// 1.9 ms here (GEMM 0.73, rebuild 0.19, energy 0.44).
+// 1.3 ms here (GEMM 0.43, 0.67 with the four products apart; rebuild 0.18, energy 0.31).
 #include "rns.cuh"
 
 namespace pcg {
@@ -108,11 +111,12 @@ __global__ void __launch_bounds__(256) t3_join_kernel(const __grid_constant__ T3
   }
 }
 
-// Workspace of a wave function: status and shifts, the residues of the six matrices, then each
+// Workspace of a wave function: status and shifts, the residues of the matrices, then each
 // batch's products (during packing the rows' tables lie there instead).
 struct T3Plan {
-  long long no, nv, rows_a, rows_b, kv, ko, ld;  // kv, ko: K padded to whole 64-K blocks
-  long long vt, vn, tm, tmt, t2p, ob, fixed;     // byte offsets; fixed: the end of the residues
+  long long no, nv, rows_a, rows_b, ld;
+  long long c0, kc;          // first column of the m part, a multiple of 8; columns in 64-K blocks
+  long long a1, a2, b, fixed;  // byte offsets; fixed: the end of the residues
   long long tables, per_triple;
 };
 
@@ -122,21 +126,18 @@ bool t3_plan(T3Plan& p, long long no, long long nv) {
   p.nv = nv;
   p.rows_a = no * nv * nv;
   p.rows_b = no * no * nv;
-  p.kv = up(nv, 64);
-  p.ko = up(no, 64);
+  p.c0 = up(nv, 8);
+  p.kc = up(p.c0 + no, 64);
   p.ld = up(nv, 16);
-  const long long av = up(NM * p.rows_a * p.kv * 2, 256), ao = up(NM * p.rows_a * p.ko * 2, 256);
-  p.vt = 256;
-  p.vn = p.vt + av;
-  p.tm = p.vn + av;
-  p.tmt = p.tm + ao;
-  p.t2p = p.tmt + ao;
-  p.ob = p.t2p + up(NM * p.rows_b * p.kv * 2, 256);
-  p.fixed = p.ob + up(NM * p.rows_b * p.ko * 2, 256);
+  const long long a = up(NM * p.rows_a * p.kc * 2, 256);
+  p.a1 = 256;
+  p.a2 = p.a1 + a;
+  p.b = p.a2 + a;
+  p.fixed = p.b + up(NM * p.rows_b * p.kc * 2, 256);
   p.tables = (4 * p.rows_a + 2 * p.rows_b) * (8 + 4 + 4 + 4) + 6 * 4 * 16;
   p.per_triple = 3 * NM * nv * nv * p.ld;
   return NM * p.rows_a < 0x7fffffffLL - BM && NM * p.rows_b < 0x7fffffffLL - 256 &&
-         (p.rows_a / 64 + p.rows_b / 32 + 4) * (p.kv / 64) < 0x7fffffffLL;
+         (p.rows_a / 64 + p.rows_b / 32 + 4) * (p.kc / 64) < 0x7fffffffLL;
 }
 
 }  // namespace
@@ -202,13 +203,13 @@ extern "C" int pcg_t3_rns_pack(const double* V, const double* O, const double* t
   const Operand tm = operand(t2, o, o * v * v, v, v, v, 1, v * v, 2, 2);
   const Operand tmt = operand(t2, o, o * v * v, v, 1, v, v, v * v, 1, 2);
   const Operand t2p = operand(t2, o, o * v * v, o, v * v, v, v, 1, 2, 1);
-  const Operand ob = operand(O, o, o, o, 1, v, o * o, v * o * o, 1, 3);
+  const Operand ob = operand(O, o, 1, o, o, v, o * o, v * o * o, 0, 3);
   const Operand none{};
   struct {
     Operand a, b;
-    long long K, Kp, pa, pb;
-  } pass[4] = {{vt, t2p, v, p.kv, p.vt, p.t2p}, {tm, ob, o, p.ko, p.tm, p.ob},
-               {vn, none, v, p.kv, p.vn, 0}, {tmt, none, o, p.ko, p.tmt, 0}};
+    long long K, c0, width, pa, pb;  // columns [c0, c0 + width) of the panels at pa and pb
+  } pass[4] = {{vt, t2p, v, 0, p.c0, p.a1, p.b}, {tm, ob, o, p.c0, p.kc - p.c0, p.a1, p.b},
+               {vn, none, v, 0, p.c0, p.a2, 0}, {tmt, none, o, p.c0, p.kc - p.c0, p.a2, 0}};
   cudaMemsetAsync(w, 0, 256, st);
   for (auto& x : pass) {
     TableArgs t{x.a, x.b, SubIdx{}, 0, nullptr, nullptr, nullptr};
@@ -229,9 +230,9 @@ extern "C" int pcg_t3_rns_pack(const double* V, const double* O, const double* t
   t3_shift_kernel<<<1, 1, 0, st>>>(mx, log2up(v), log2up(o), shift);
   PCG_CHECK_LAUNCH("pcg_t3_rns_pack/shift");
   for (auto& x : pass) {
-    PackArgs a{{{x.a, 0, x.a.R, (__nv_bfloat16*)(w + x.pa), 0, 0},
-                {x.b, 0, x.b.R, (__nv_bfloat16*)(w + x.pb), x.b.X == O ? 0x80000000u : 0u, 0}},
-               0, x.K, x.Kp, 0, tables().pairs};
+    PackArgs a{{{x.a, 0, x.a.R, (__nv_bfloat16*)(w + x.pa) + x.c0, 0, 0},
+                {x.b, 0, x.b.R, (__nv_bfloat16*)(w + x.pb) + x.c0, x.b.X == O ? 0x80000000u : 0u, 0}},
+               0, x.K, x.width, p.kc, 0, tables().pairs};
     if (run_pack(a, st)) return -2;
   }
   return 0;
@@ -263,18 +264,12 @@ extern "C" int pcg_t3_rns_partials(long long no, long long nv, const int* ijk, i
   g.t = tables().mod;
   g.ijk = ijk;
   g.no = (int)no;
-  g.kv = (int)(p.kv / 64);
-  g.ko = (int)(p.ko / 64);
+  g.kc = (int)(p.kc / 64);
   GemmMaps maps{};
-  const long long a_off[4] = {p.vt, p.vn, p.tm, p.tmt}, b_off[2] = {p.t2p, p.ob};
-  for (int q = 0; q < 4; ++q) {
-    const long long kb = 2 * (q < 2 ? p.kv : p.ko);
-    if (!make_map(&maps.a[q], w + a_off[q], NM * p.rows_a, kb, kb, 2, BM)) return -1;
-  }
-  for (int q = 0; q < 2; ++q) {
-    const long long kb = 2 * (q == 0 ? p.kv : p.ko);
-    if (!make_map(&maps.b[q], w + b_off[q], NM * p.rows_b, kb, kb, 2, g.bs)) return -1;
-  }
+  if (!make_map(&maps.a[0], w + p.a1, NM * p.rows_a, 2 * p.kc, 2 * p.kc, 2, BM) ||
+      !make_map(&maps.a[1], w + p.a2, NM * p.rows_a, 2 * p.kc, 2 * p.kc, 2, BM) ||
+      !make_map(&maps.b[0], w + p.b, NM * p.rows_b, 2 * p.kc, 2 * p.kc, 2, g.bs))
+    return -1;
   const int rc = BN == 256   ? run_gemm<256, true>(maps, g, st)
                  : BN == 128 ? run_gemm<128, true>(maps, g, st)
                              : run_gemm<64, true>(maps, g, st);
