@@ -571,8 +571,8 @@ struct PackArgs {
 // double for BF16x6 (three pieces carry 24 bits; split in integer arithmetic) and float
 // otherwise: FP64 inputs are rounded to FP32 in integer arithmetic (f64_to_f32) and combined and
 // split in FP32, which keeps the kernel a stream instead of a loop on GB300's FP64 pipe.  A
-// BF16 hi/lo pair holds 16 bits, so the FP32 rounding (2^-24 of the operands) is far below the split's own
-// error.  The K multipliers are powers of two in practice (exact in FP32).
+// BF16 hi/lo pair holds 16 bits, so the FP32 rounding (2^-24 of the operands) is far below the
+// split's own error.  The K multipliers are powers of two in practice (exact in FP32).
 constexpr int TR = 64, TK = 64, PACK_THREADS = 256;
 static_assert((TR * TK) % PACK_THREADS == 0, "pack tile: whole elements per thread");
 

@@ -358,8 +358,8 @@ long long tile_triples(long long nv) {
 // sets of each partial arrive as 8 x 8 x 8 boxes by TMA (18 boxes of 2 KB, zeros beyond nv) and W is
 // summed where it is used.  The 8 x 8 blocks of integrals and amplitudes are the threads' own
 // loads: 36 more small copies by TMA, which takes 2.6 clocks for a 32-byte row, made the kernel
-// 15 % slower.  The staging of the kernel above cost about 500 instructions a thread and, at a pitch that is no multiple of 32 bytes, two sectors for each 32-byte run; what bounds
-// this one is shared-memory reads, so a warp takes 2 x 4 x 4 elements (a, b, c), which keeps the
+// 15 % slower.  The staging of the kernel above cost about 500 instructions a thread and, at a
+// pitch that is no multiple of 32 bytes, two sectors for each 32-byte run; what bounds this one is shared-memory reads, so a warp takes 2 x 4 x 4 elements (a, b, c), which keeps the
 // boxes' 256-byte slices at two to four reads to a bank.
 // At nv = 121, 32 triples: 260 us against 400.
 struct CubeArgs {
