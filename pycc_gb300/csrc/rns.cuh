@@ -22,6 +22,15 @@ constexpr int NM = 16;
 constexpr int kModuli[NM] = {256, 253, 251, 247, 241, 239, 233, 229,
                              227, 223, 217, 211, 199, 197, 193, 191};
 constexpr int kBits2 = 123;         // |a'|^2 |b'|^2 <= 2^(2 * 123.75); log2(product / 2) = 123.95
+constexpr int kSumBits = 123;       // sums of up to 2^kSumBits are certain to be in range
+// The product of the moduli above 2^(kSumBits + 1) times 2^0.9: room for kBits2's 0.75 bits too.
+constexpr bool moduli_hold_sums() {
+  double half = 0.5;
+  for (int p : kModuli) half *= p;
+  for (int b = 0; b < kSumBits; ++b) half *= 0.5;
+  return half > 1.866;  // 2^0.9
+}
+static_assert(moduli_hold_sums(), "half the product of the moduli exceeds 2^(kSumBits + 0.9)");
 // first bit of the four digits of a scaled integer (16, 15, 15 and 16 bits): with residues of
 // the powers of at most 127, a digit sum stays below 2^16 + 127 * 2^17 < 2^24, exact in FP32
 __host__ __device__ constexpr int digit_bit(int q) { return q == 0 ? 0 : (q == 4 ? 62 : 1 + 15 * q); }

@@ -54,8 +54,11 @@ __global__ void __launch_bounds__(256) t3_max_kernel(const T3MaxArgs p) {
   }
 }
 
-// Powers of two with every product of rows at most 2^122 in norm: four of them sum to less than
-// half the product of the moduli (2^123.95).
+// Powers of two that keep every product of two row norms at or below 2^kT3Bits.  By Cauchy-Schwarz
+// the four products of an orientation sum to at most 4 2^kT3Bits = 2^123, and the residues
+// determine a sum of up to half the product of the moduli, 2^123.95.
+constexpr int kT3Bits = 121;
+static_assert(kT3Bits + 2 <= kSumBits, "four products stay in the range of the residues");
 __global__ void t3_shift_kernel(const unsigned* mx, int log2v, int log2o, T3Shift* out) {
   int e[4];  // row norms are at most 2^e
   bool bad = false;
@@ -68,10 +71,10 @@ __global__ void t3_shift_kernel(const unsigned* mx, int log2v, int log2o, T3Shif
                        : 2 * (max(top, 1) - 1022) + (q < 2 ? log2v : log2o);
     e[q] = (l2 + 1) >> 1;
   }
-  const int s1 = 122 - e[0] - e[1], s2 = 122 - e[2] - e[3], s = min(s1, s2);
-  out->sh[0] = 61 - e[0] - ((s1 - s) >> 1);
+  const int s1 = kT3Bits - e[0] - e[1], s2 = kT3Bits - e[2] - e[3], s = min(s1, s2);
+  out->sh[0] = kT3Bits / 2 - e[0] - ((s1 - s) >> 1);
   out->sh[1] = s - out->sh[0];
-  out->sh[2] = 61 - e[2] - ((s2 - s) >> 1);
+  out->sh[2] = kT3Bits / 2 - e[2] - ((s2 - s) >> 1);
   out->sh[3] = s - out->sh[2];
   out->total = s;
   out->bad = bad;

@@ -58,3 +58,23 @@ def test_not_finite(cuda):
     V, O, t2 = rand(7, 7, 7, 3), rand(3, 7, 3, 3), rand(3, 3, 7, 7)
     t2[1, 2, 3, 4] = float("inf")
     assert bool(partials(V, O, t2, [(2, 1, 0)], 1).isnan().all())
+
+
+@pytest.mark.parametrize("n,x,wide", [(1, 0.99, 0.0), (1, 1.99, 0.0), (2, 0.7, 0.0),
+                                      (4, 0.4975, 0.0), (4, 0.489, 0.02), (16, 0.249, 0.0)])
+def test_range(cuda, n, x, wide):
+    """Collinear rows with norms just below a power of two: the four products of an orientation
+    add up to the largest sum that the scales allow, which the moduli have to hold."""
+    gen = torch.Generator(device=cuda).manual_seed(n)
+    near = lambda *s: x * (1 + wide * (2 * torch.rand(s, dtype=torch.float64, device=cuda,
+                                                      generator=gen) - 1))
+    V, O, t2 = near(n, n, n, n), -near(n, n, n, n), near(n, n, n, n)
+    trips = [(n - 1, n // 2, 0), (n - 1, n - 1, n - 1)]
+    got = partials(V, O, t2, trips, 2)
+    for t, (i, j, k) in enumerate(trips):
+        for q, (lab, terms) in enumerate(orientation_terms(i, j, k, t2, V, O)):
+            ref = torch.empty_like(got[t, q])
+            contract_multi(ref.permute(1, 2, 0), lab, terms)
+            # every product is positive: the sums of magnitudes are the sums
+            tol = 2.0 ** -53 * (4 * n + 8) * ref + 2.0 ** -56 * float(ref.max())
+            assert bool(((got[t, q] - ref).abs() <= tol).all())
