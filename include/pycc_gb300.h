@@ -49,11 +49,15 @@ int pcg_contract_f64(int m_n, const long long* m_ext, const long long* m_sa,
                      void* stream);
 
 /* The same contraction on the BF16 tensor cores in residue arithmetic (csrc/contract_rns.cu):
- * operands scaled by row to integers of at least 54 bits, one exact BF16 GEMM per modulus,
- * the FP64 result rebuilt from the residues.  `work` is device scratch of `work_len` bytes,
- * 256-byte aligned, not read after the call's kernels; an operand larger than it goes through
- * in panels.  pcg_contract_rns_f64_work gives the bytes for flat extents M, N, K within
- * `limit` (0 when no panel fits).  An expired device-side wait makes the outputs NaN. */
+ * the rows of both operands (over K) scaled by powers of two to a 2-norm of 2^60.3 to 2^61.9 and
+ * rounded to integers, one exact BF16 GEMM per modulus, the FP64 result rebuilt from the residues.
+ * An output whose sum |a||b| is small against its rows' norms, so that this rounding would reach
+ * it, is computed by FP64 multiply-adds; the error of every output is at most
+ * max(sqrt(K) 2^-52, K 2^-53) sum |a||b| and the roundings of the result.  `work` is device
+ * scratch of `work_len` bytes, 256-byte aligned, not read after the call's kernels; an operand
+ * larger than it goes through in panels.  pcg_contract_rns_f64_work gives the bytes for flat
+ * extents M, N, K within `limit` (0 when no panel fits).  An expired device-side wait makes the
+ * outputs NaN. */
 int pcg_contract_rns_f64(int m_n, const long long* m_ext, const long long* m_sa,
                          const long long* m_sc, int n_n, const long long* n_ext,
                          const long long* n_sb, const long long* n_sc, int k_n,
@@ -69,12 +73,20 @@ int pcg_contract_rns_f64_work(long long M, long long N, long long K, long long l
  * O = <mp|xy> ([o][v][o][o]) and t2 ([o][o][v][v]), all contiguous FP64, into `work` (256-byte
  * aligned).  pcg_t3_rns_partials: for the ntrip triples ijk (device int [ntrip][3]) the partial
  * tensors of the three orientations, P[triple][orientation][z][x][y], as pcg_triples_energy reads
- * them.  An Inf or NaN in an operand, or an expired device-side wait, makes them NaN. */
+ * them, accurate to about 2^-56 of the largest products of row norms (all rows of a matrix share one
+ * scale); an Inf or NaN in an operand makes them NaN.  pcg_t3_rns_partials_of takes the operands that
+ * were packed as well, and computes by FP64 multiply-adds the partials whose products are small
+ * against those norms, or all of them if an operand holds an Inf or a NaN: the error of every partial
+ * is at most (nv + no) 2^-51 times the sum of its products' magnitudes.  In both an expired
+ * device-side wait makes the partials NaN. */
 int pcg_t3_rns_work(long long no, long long nv, int batch, long long* bytes);
 int pcg_t3_rns_pack(const double* V, const double* O, const double* t2, long long no, long long nv,
                     void* work, long long work_len, void* stream);
 int pcg_t3_rns_partials(long long no, long long nv, const int* ijk, int ntrip, double* P, void* work,
                         long long work_len, void* stream);
+int pcg_t3_rns_partials_of(const double* V, const double* O, const double* t2, long long no,
+                           long long nv, const int* ijk, int ntrip, double* P, void* work,
+                           long long work_len, void* stream);
 
 /* Sum of up to four FP64 contractions into one output (written once):
  *   C = beta*C + sum_t alpha[t] * A_t[m,k] B_t[n,k]

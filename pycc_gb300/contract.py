@@ -137,7 +137,9 @@ _CALLS = {}
 
 def contract_f64(subscripts, a, b, out=None, alpha=1.0, beta=0.0, stream=None):
     """``out = beta*out + alpha * einsum(subscripts, a, b)`` in FP64: on the FP64 kernels, or,
-    where that is the shorter (``_takes_rns``), on the tensor cores in residue arithmetic."""
+    where that is the shorter (``_takes_rns``), on the tensor cores in residue arithmetic.  Both
+    keep every output's error within about K 2^-53 sum |a||b| over its K products (an output for
+    which the residues' common scale of a row is too coarse is summed in FP64)."""
     _check(a, "operand 0")
     _check(b, "operand 1")
     if out is not None:
@@ -195,8 +197,8 @@ def _takes_rns(m, n, k):
     """Whether an m x n x k contraction runs on the tensor cores in residue arithmetic rather
     than on the FP64 pipe: where its estimated time is the shorter one.
 
-    FP64 pipe: 6 us and 1.05 TFLOP/s.  Residues: 42 us of launches, 48 bytes moved per operand
-    element at 5 TB/s, 0.3 ns per step of K (a row's norm), 16 BF16 products over whole 128 x 16 x
+    FP64 pipe: 6 us and 1.05 TFLOP/s.  Residues: 42 us of launches, 50 bytes moved per operand
+    element at 5 TB/s, 0.3 ns per step of K (a row's norm), 17 BF16 products over whole 128 x 16 x
     64 tiles at 1.1 PFLOP/s and at least 2.5 us for 128 x 256 of them on an SM, and 13 ps per
     output to rebuild it.  Measured on both sides of the line (us, FP64 pipe / residues): 2809 x 81
     x 81 48 / 46, 53 x 53 x 4293 42 / 44, 60 x 60 x 8640 73 / 53, 110 x 21560 x 14 88 / 92, 11 x
@@ -207,9 +209,9 @@ def _takes_rns(m, n, k):
     up = lambda x, t: -(-x // t) * t
     fp64 = 6e-6 + 2.0 * m * n * k / 1.05e12
     lo, hi = (m, n) if m < n else (n, m)
-    gemm = max(32.0 * up(lo, 128) * hi * up(k, 64) / 1.1e15,
-               16 * up(lo, 128) // 128 * up(hi, 256) // 256 * 2.5e-6 / 152)
-    rns = 42e-6 + 48.0 * (m + n) * k / 5e12 + 0.3e-9 * k + gemm + 13e-12 * m * n
+    gemm = max(34.0 * up(lo, 128) * hi * up(k, 64) / 1.1e15,
+               17 * up(lo, 128) // 128 * up(hi, 256) // 256 * 2.5e-6 / 152)
+    rns = 42e-6 + 50.0 * (m + n) * k / 5e12 + 0.3e-9 * k + gemm + 13e-12 * m * n
     return rns < fp64
 
 

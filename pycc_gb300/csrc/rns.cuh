@@ -21,6 +21,18 @@ using namespace pcg::tc;
 constexpr int NM = 16;
 constexpr int kModuli[NM] = {256, 253, 251, 247, 241, 239, 233, 229,
                              227, 223, 217, 211, 199, 197, 193, 191};
+// Planes of a packed operand and of a product: the residues, then magnitudes.  A row is rounded to
+// integers at one power of two, so an output's error is a fixed number of units: 0.29 sqrt(|a'|^2 +
+// |b'|^2) <= 2^60.6 of them (root mean square).  Where large entries of a row meet small or zero
+// ones, that can be all of a sum of small products.  So |a'| and |b'|, truncated to BF16, go through
+// the GEMM as well and give sum |a'||b'|; an output whose sum is not zero and below kDoubt units
+// is computed again in FP64.  Elsewhere the error is at most 2^-53.4 sum |a||b| (root mean
+// square) and sqrt(K) 2^-52 sum |a||b| in the worst case, against K 2^-53 for FP64 multiply-adds.
+constexpr int NP = NM + 1;
+constexpr float kDoubt = 0x1p114f;
+// The magnitude of an entry that rounds to zero and is not: large enough that the product of two of
+// them is a normal FP32 number, so that sum |a'||b'| is zero for outputs without a product only.
+constexpr unsigned kTinyBf16 = (127 - 60) << 7;
 constexpr int kBits2 = 123;         // |a'|^2 |b'|^2 <= 2^(2 * 123.75); log2(product / 2) = 123.95
 constexpr int kSumBits = 123;       // sums of up to 2^kSumBits are certain to be in range
 // The product of the moduli above 2^(kSumBits + 1) times 2^0.9: room for kBits2's 0.75 bits too.
@@ -37,9 +49,10 @@ __host__ __device__ constexpr int digit_bit(int q) { return q == 0 ? 0 : (q == 4
 constexpr int kChunk = 15;          // 64-K blocks per exact FP32 accumulation: 960 K
 constexpr float kMagic = 12582912.f;  // 1.5 * 2^23: adding it rounds to an integer
 
-// Per modulus: p, 1/p and the residues of 2^16, 2^31, 2^46 (symmetric).
+// Per modulus: p, 1/p and the residues of 2^16, 2^31, 2^46 (symmetric).  The magnitudes' p and 1/p
+// are zero: nothing is taken off their sums.
 struct ModTab {
-  float p[NM], inv[NM], c1[NM], c2[NM], c3[NM];
+  float p[NP], inv[NP], c1[NM], c2[NM], c3[NM];
 };
 // ModTab's entries twice each (np: -p), for arithmetic on pairs.
 struct PairTab {
@@ -59,6 +72,16 @@ __device__ __forceinline__ unsigned residue_bytes(float a, float b, float c, flo
   return __byte_perm(
       __byte_perm(__float_as_uint(a + bias), __float_as_uint(b + bias), 0x0040),
       __byte_perm(__float_as_uint(c + bias), __float_as_uint(d + bias), 0x0040), 0x5410);
+}
+
+// Exponent bits of four sums of magnitudes (not negative, below 2^128).
+__device__ __forceinline__ unsigned exponent_bytes(float a, float b, float c, float d) {
+  return (__float_as_uint(a) >> 23) | (__float_as_uint(b) >> 23 << 8) |
+         (__float_as_uint(c) >> 23 << 16) | (__float_as_uint(d) >> 23 << 24);
+}
+// A sum of magnitudes, to a factor of two, from byte e of a word of them.
+__device__ __forceinline__ float magnitude_sum(unsigned w, int e) {
+  return __uint_as_float(__byte_perm(w, 0u, 0x4440u + e) << 23);
 }
 
 // Two FP32 values in one register pair; each half is rounded as the scalar operation's.
@@ -99,8 +122,7 @@ struct Operand {
   long long* off;       // [R] element offset of each row in X
   long long* coff;      // [R] element offset of each row (or column) in C
   int* walk;            // [R] rows in an order whose neighbours are close in X
-  unsigned* top;        // [R] biased exponent of the row's largest |x| (2047: Inf or NaN)
-  float* norm2;         // [R] sum of the row's squares, each term truncated to 20 bits
+  unsigned long long* norm;  // [R] the row's largest exponent and sum of squares (RowNorm)
   const int* shift;     // one power of two for all rows, or null: each row its own
   int* sh;              // [R] the rows' powers of two as the pack used them (kNotFinite: the row
                         // holds an Inf or a NaN), or null
@@ -145,12 +167,10 @@ static __global__ void rns_tables_kernel(const TableArgs t) {
     if (i == 0 && t.status) *t.status = 0;
     if (i < t.a.R) {
       fill_row(t.a, i);
-      t.a.top[i] = 0;
-      t.a.norm2[i] = 0.f;
+      t.a.norm[i] = 0;
     } else if (i < t.a.R + t.b.R) {
       fill_row(t.b, i - t.a.R);
-      t.b.top[i - t.a.R] = 0;
-      t.b.norm2[i - t.a.R] = 0.f;
+      t.b.norm[i - t.a.R] = 0;
     } else if (t.ka) {
       const long long k = i - t.a.R - t.b.R;
       long long ka, kb;
@@ -165,94 +185,168 @@ __device__ __forceinline__ long long k_offset(const Operand& o, long long k) {
   return o.kstep > 0 ? k * o.kstep : o.k[k];
 }
 
-// |x| as FP32 from the upper word of a double (20 mantissa bits, truncated); below FP32's
-// range 0, above it infinity.
-__device__ __forceinline__ float abs_hi_f32(unsigned h) {
-  h &= 0x7fffffffu;
-  if (h < (897u << 20)) return 0.f;
-  return h < (1151u << 20) ? __uint_as_float((h - (896u << 20)) << 3)
-                           : __uint_as_float(0x7f800000u);
-}
-
-// Largest exponent and sum of squares of each row over K indices [k0, k1): one read of the
-// operand, bound by HBM.  Gathered along K (KF: a warp per row) or along the rows (a thread
-// per row), eight loads in flight per lane; blockIdx.y cuts K.
-template <bool KF>
-__device__ __forceinline__ void norm_rows(const Operand& o, long long k0, long long k1,
-                                          long long seg, long long bx, long long by) {
-  const long long kb = k0 + by * seg, ke = min(k1, kb + seg);
-  const int lane = threadIdx.x & 31;
-  const long long w = KF ? bx * 8 + (threadIdx.x >> 5) : bx * 256 + threadIdx.x;
-  if (w >= o.R) return;
-  constexpr int STEP = KF ? 32 : 1;
-  const int row = o.walk[w];
-  const double* x = o.X + o.off[row];
-  unsigned m = 0;
+// Sum of squares of a row's |x| 2^(1023 - top), |x| truncated to 20 mantissa bits; top: the biased
+// exponent of the largest, at least 1 (2047: an Inf or a NaN).  With an exponent of its own the sum
+// holds for rows of any magnitude, where a plain FP32 one holds norms of 2^-40 to 2^50.  Subnormal
+// numbers, and zeros of rows below 2^-900, count as more than they are.
+struct RowNorm {
+  int top = 1;
   float s = 0.f;
+  __device__ __forceinline__ void raise(int t) {
+    if (t > top) {
+      const int d = 127 - 2 * (t - top);
+      s *= d > 0 ? __int_as_float(d << 23) : 0.f;
+      top = t;
+    }
+  }
+  // h: the upper words of finite doubles or not, without their signs
+  template <int N>
+  __device__ __forceinline__ void add(const unsigned (&h)[N]) {
+    unsigned m = 0;
+#pragma unroll
+    for (int u = 0; u < N; ++u) m = max(m, h[u]);
+    raise((int)(m >> 20));
+    const int off = (top - 127) * (1 << 20);
+    float t = 0.f;
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+      const float f = __uint_as_float((unsigned)max((int)h[u] - off, 0) << 3);
+      t = fmaf(f, f, t);
+    }
+    s += t;
+  }
+  __device__ __forceinline__ void add(RowNorm r) {
+    raise(r.top);
+    r.raise(top);
+    s += r.s;
+  }
+  __device__ __forceinline__ void reduce() {  // over a warp
+    raise(__reduce_max_sync(0xffffffffu, top));
+    for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+  }
+  __device__ __forceinline__ unsigned long long bits() const {
+    return (unsigned long long)top << 32 | __float_as_uint(s);
+  }
+  static __device__ __forceinline__ RowNorm from(unsigned long long b) {
+    RowNorm r;
+    r.top = max((int)(b >> 32), 1);
+    r.s = __uint_as_float((unsigned)b);
+    return r;
+  }
+  // floor(log2) of the sum in units of one, with 2^-7 for its truncation and summation, and the
+  // significand's upper bits
+  __device__ __forceinline__ int log2(unsigned& frac) const {
+    const unsigned u = __float_as_uint(s * 1.0078125f);
+    frac = u & 0x7fffffu;
+    return (int)(u >> 23) - 127 + 2 * (top - 1023);
+  }
+};
+
+// Norms of the rows over K indices [k0, k1): one read of the operand, bound by HBM.  Gathered along K
+// (KF: a warp per row) or along the rows (a thread per row, or, of few rows, one per row and slice
+// of K: the eight warps of a block then share 32 rows), eight loads in flight per lane.  Block by of
+// segs has K indices [k0 + by seg, ..).
+template <bool KF>
+__device__ __forceinline__ void norm_rows(const Operand& o, unsigned long long* part, long long k0,
+                                          long long k1, bool slices, long long seg, long long segs,
+                                          long long bx, long long by) {
+  __shared__ unsigned long long sums[8][32];
+  long long kb = k0 + by * seg, ke = min(k1, kb + seg);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long w = KF ? bx * 8 + warp : (slices ? bx * 32 + lane : bx * 256 + threadIdx.x);
+  if (w >= o.R && !slices) return;
+  if (slices) {
+    const long long each = (seg + 7) / 8;
+    kb = min(ke, kb + warp * each);
+    ke = min(ke, kb + each);
+  }
+  constexpr int STEP = KF ? 32 : 1;
+  const int row = o.walk[min(w, o.R - 1)];
+  const double* x = o.X + o.off[row];
+  RowNorm n;
   long long k = kb + (KF ? lane : 0);
   for (; k + 7 * STEP < ke; k += 8 * STEP) {
     unsigned h[8];
 #pragma unroll
     for (int u = 0; u < 8; ++u)
-      h[u] = (unsigned)__double2hiint(__ldg(x + k_offset(o, k + STEP * u)));
-    float t = 0.f;
+      h[u] = (unsigned)__double2hiint(__ldg(x + k_offset(o, k + STEP * u))) & 0x7fffffffu;
+    n.add(h);
+  }
+  if (k < ke) {  // zeros past the end
+    unsigned h[7];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const float f = abs_hi_f32(h[u]);
-      m = max(m, h[u] & 0x7fffffffu);
-      t = fmaf(f, f, t);
-    }
-    s += t;
+    for (int u = 0; u < 7; ++u)
+      h[u] = k + STEP * u < ke
+                 ? (unsigned)__double2hiint(__ldg(x + k_offset(o, k + STEP * u))) & 0x7fffffffu
+                 : 0u;
+    n.add(h);
   }
-  for (; k < ke; k += STEP) {
-    const unsigned h = (unsigned)__double2hiint(__ldg(x + k_offset(o, k)));
-    const float f = abs_hi_f32(h);
-    m = max(m, h & 0x7fffffffu);
-    s = fmaf(f, f, s);
+  if (KF) n.reduce();
+  if (slices) {
+    sums[warp][lane] = n.bits();
+    __syncthreads();
+    if (warp > 0 || w >= o.R) return;
+    for (int q = 1; q < 8; ++q) n.add(RowNorm::from(sums[q][lane]));
   }
-  if (KF) {
-    for (int d = 16; d > 0; d >>= 1) {
-      m = max(m, __shfl_xor_sync(0xffffffffu, m, d));
-      s += __shfl_xor_sync(0xffffffffu, s, d);
-    }
-    if (lane != 0) return;
+  if (segs == 1) {
+    if (!KF || lane == 0) o.norm[row] = n.bits();
+    return;
   }
-  atomicMax(o.top + row, m >> 20);
-  atomicAdd(o.norm2 + row, s);
+  // the last of the row's parts adds them up (norm, zero before, counts them)
+  bool last = false;
+  if (!KF || lane == 0) {
+    part[by * o.R + row] = n.bits();
+    __threadfence();
+    last = atomicAdd(o.norm + row, 1ull) + 1 == (unsigned long long)segs;
+    if (last) __threadfence();
+  }
+  if (KF ? !__shfl_sync(0xffffffffu, last, 0) : !last) return;
+  RowNorm sum;
+  for (int q0 = KF ? lane : 0; q0 < segs; q0 += 8 * STEP) {  // eight loads in flight here too
+    unsigned long long r[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      r[u] = q0 + STEP * u < segs ? __ldcg(part + (q0 + STEP * u) * o.R + row) : 0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) sum.add(RowNorm::from(r[u]));
+  }
+  if (KF) sum.reduce();
+  if (!KF || lane == 0) o.norm[row] = sum.bits();
 }
 
 struct NormArgs {
   Operand o[2];
-  long long gx[2], blocks[2], seg[2];  // row blocks, blocks and K segment of each operand
+  long long gx[2], blocks[2], seg[2], segs[2];  // row blocks, blocks, K segment and their number
+  bool slices[2];                               // a block's warps have K slices of 32 rows
+  unsigned long long* part[2];                  // [segs][R] sums of the segments
   long long k0, k1;
 };
 
 // Both operands in one launch: the first blocks take A, the others B.
-static __global__ void __launch_bounds__(256) rns_norm_kernel(const __grid_constant__ NormArgs p) {
+static __global__ void __launch_bounds__(256, 8) rns_norm_kernel(const __grid_constant__ NormArgs p) {
   const int side = blockIdx.x >= p.blocks[0];
   const long long b = (long long)blockIdx.x - (side ? p.blocks[0] : 0);
   const long long bx = b % p.gx[side], by = b / p.gx[side];
   if (p.o[side].kfast)
-    norm_rows<true>(p.o[side], p.k0, p.k1, p.seg[side], bx, by);
+    norm_rows<true>(p.o[side], p.part[side], p.k0, p.k1, false, p.seg[side], p.segs[side], bx, by);
   else
-    norm_rows<false>(p.o[side], p.k0, p.k1, p.seg[side], bx, by);
+    norm_rows<false>(p.o[side], p.part[side], p.k0, p.k1, p.slices[side], p.seg[side], p.segs[side],
+                     bx, by);
 }
 
 constexpr int kNotFinite = 1 << 20;
 
-// Power of two s of a row: |x| 2^s has a 2-norm of at most 2^61.9.  From the sum of squares
-// where FP32 holds it (1 + 2^-7 covers its truncation and summation), else from the largest
-// element and K.  A zero row may take any.
-__device__ __forceinline__ int row_shift(const Operand& o, long long row, int log2k) {
+// Power of two s of a row: |x| 2^s has a 2-norm of at most 2^61.9 (and of at least 2^60.3, where its
+// entries are normal numbers).  A zero row may take any.
+__device__ __forceinline__ int row_shift(const Operand& o, long long row) {
   if (o.shift) return *o.shift;
-  const float n2 = o.norm2[row] * 1.0078125f;
-  if (n2 >= 0x1p-80f && n2 <= 0x1p100f) {
-    const unsigned u = __float_as_uint(n2);
-    const int e = (int)(u >> 23) - 127;
-    // log2 n2 <= e + 0.75 or e + 1.75
-    return ((u & 0x7fffffu) < 0x570000u ? kBits2 - e : kBits2 - 1 - e) >> 1;
-  }
-  return (kBits2 - log2k - 2 * (max((int)o.top[row], 1) - 1022)) >> 1;
+  unsigned frac;
+  const int e = RowNorm::from(o.norm[row]).log2(frac);
+  // log2 of the sum of squares <= e + 0.75 or e + 1.75; scaled() takes up to 1083
+  return min((frac < 0x570000u ? kBits2 - e : kBits2 - 1 - e) >> 1, 1083);
+}
+__device__ __forceinline__ bool not_finite(const Operand& o, long long row) {
+  return o.norm[row] >> 32 == 2047u;
 }
 
 // The magnitude of x 2^s rounded to an integer of at most 62 bits, and its sign as +-1.
@@ -262,7 +356,7 @@ __device__ __forceinline__ unsigned long long scaled(double x, int s, unsigned f
   const unsigned mh = (hi & 0xfffffu) | (ex ? 1u << 20 : 0u);
   // |x| 2^s = m 2^sh, sh = max(ex, 1) - 1075 + s at most 9 since |x| 2^s <= 2^61.9: shifted left
   // by 9 - sh from 10 bits up, then rounded off by the last.  A shift past 63 leaves 0, as does
-  // the exponent of an infinity or a NaN, whose row takes its outputs from the FP64 dot product.
+  // the exponent of an infinity or a NaN, whose row takes its outputs from FP64 dot products.
   const unsigned r = min((unsigned)(9 + 1075 - s - (int)max(ex, 1u)), 63u);
   const unsigned long long m = (((unsigned long long)mh << 32) | lo) << 10;
   sign = __uint_as_float(0x3f800000u | (hi & 0x80000000u));
@@ -287,7 +381,7 @@ __device__ __forceinline__ void digits(double x, double y, int s, unsigned flip,
 struct PackSide {
   Operand o;
   long long w0, nrow;  // rows of this panel: walk positions [w0, w0 + nrow); nrow 0: none
-  __nv_bfloat16* out;  // [modulus][nrow][ld]
+  __nv_bfloat16* out;  // [plane][nrow][ld]
   unsigned flip;       // 0x80000000: the negated operand
   long long blocks;
 };
@@ -296,13 +390,16 @@ struct PackArgs {
   PackSide s[2];
   long long k0, K;      // K indices [k0, k0 + K)
   long long width, ld;  // columns written, zeros from K on, of each row's ld (multiples of 8)
-  int log2k;            // ceil(log2 K)
   PairTab t;
 };
 
-// Residues of eight neighbouring K entries for every modulus, two to an instruction and one
-// 128-bit store per modulus: an integer of at most 8 bits is exact in the upper half of its FP32
-// word, which is BF16.
+__device__ __forceinline__ bool not_zero(double x) {
+  return ((unsigned)__double2hiint(x) << 1 | (unsigned)__double2loint(x)) != 0u;
+}
+
+// Magnitudes and residues of eight neighbouring K entries, two to an instruction and one 128-bit
+// store per plane: an integer of at most 8 bits is exact in the upper half of its FP32 word, which
+// is BF16.
 __device__ __forceinline__ void store_residues(const PackArgs& p, const PackSide& o,
                                                const double (&x)[8], int s, long long at) {
   unsigned long long d[4][4];
@@ -310,9 +407,20 @@ __device__ __forceinline__ void store_residues(const PackArgs& p, const PackSide
   for (int e = 0; e < 4; ++e) digits(x[2 * e], x[2 * e + 1], s, o.flip, d[e]);
   uint4* out = reinterpret_cast<uint4*>(o.out + at);
   const long long plane = (o.nrow * p.ld) >> 3;
+  unsigned r[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    float a, b;
+    unpair(fma_pair(d[e][3], pair(0x1p46f, 0x1p46f),
+                    fma_pair(d[e][2], pair(0x1p31f, 0x1p31f),
+                             fma_pair(d[e][1], pair(0x1p16f, 0x1p16f), d[e][0]))), a, b);
+    r[e] = __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632) & 0x7fff7fffu;
+    if ((r[e] & 0xffffu) == 0u && not_zero(x[2 * e])) r[e] |= kTinyBf16;
+    if ((r[e] >> 16) == 0u && not_zero(x[2 * e + 1])) r[e] |= kTinyBf16 << 16;
+  }
+  __stcs(out + NM * plane, make_uint4(r[0], r[1], r[2], r[3]));
 #pragma unroll
   for (int l = 0; l < NM; ++l, out += plane) {
-    unsigned r[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       float a, b;
@@ -326,12 +434,13 @@ __device__ __forceinline__ void store_residues(const PackArgs& p, const PackSide
   }
 }
 
-// Operand -> residues: 8 bytes read and 2 NM written per element, about 85 instructions; bound by
+// Operand -> residues: 8 bytes read and 2 NP written per element, about 95 instructions; bound by
 // the writes.  A quarter warp takes 64 K of a row, eight neighbouring K a lane.  Gathered along K
 // it loads them straight from global memory; otherwise a tile of 64 walked rows x 64 K goes through
 // shared memory, read along the rows.  One launch packs a panel of each operand: the first blocks
-// take A's, the others B's.  163e6 elements: 1.07 ms (6.1 TB/s) against 1.15 with one element to
-// an instruction and 1.20 with four K a lane as well.
+// take A's, the others B's.  163e6 elements: 1.12 ms (6.1 TB/s), 1.07
+// before the plane of magnitudes, against 1.15 with one element to an instruction and 1.20 with four
+// K a lane as well.
 static __global__ void __launch_bounds__(256, 4)
     rns_pack_kernel(const __grid_constant__ PackArgs p) {
   __shared__ double tile[64][65];
@@ -355,8 +464,8 @@ static __global__ void __launch_bounds__(256, 4)
         const long long k = kk0 + kk + e;
         x[e] = k < p.K ? __ldg(q + k_offset(o, p.k0 + k)) : 0.0;
       }
-      const int sh = row_shift(o, row, p.log2k);
-      if (o.sh && kk0 + kk == 0) o.sh[row] = o.top[row] == 2047u ? kNotFinite : sh;
+      const int sh = row_shift(o, row);
+      if (o.sh && kk0 + kk == 0) o.sh[row] = not_finite(o, row) ? kNotFinite : sh;
       store_residues(p, ps, x, sh, (row - ps.w0) * p.ld + kk0 + kk);
     }
   } else {
@@ -366,9 +475,9 @@ static __global__ void __launch_bounds__(256, 4)
         const int r = o.walk[ps.w0 + w + threadIdx.x];
         srow[threadIdx.x] = r;
         off[threadIdx.x] = o.off[r];
-        const int sh = row_shift(o, r, p.log2k);
+        const int sh = row_shift(o, r);
         ssh[threadIdx.x] = sh;
-        if (o.sh && kk0 == 0) o.sh[r] = o.top[r] == 2047u ? kNotFinite : sh;
+        if (o.sh && kk0 == 0) o.sh[r] = not_finite(o, r) ? kNotFinite : sh;
       }
     }
     __syncthreads();
@@ -393,7 +502,7 @@ static __global__ void __launch_bounds__(256, 4)
 }
 
 // ---- GEMM over the residues -------------------------------------------------------------
-// Output tiles and K of a launch.  Plain: C[split][modulus] = A B^T over K blocks
+// Output tiles and K of a launch.  Plain: C[split][plane] = A B^T over K blocks
 // [split kb_per_split, ...).  Triples (TRIP): group g = 3 t + q is orientation q of triple t,
 // the sum of two products of row blocks (csrc/triples_rns.cu).
 struct GemmArgs {
@@ -404,7 +513,7 @@ struct GemmArgs {
   int planes;        // splits, or groups
   int nkb, kb_per_split;
   long long ld;        // bytes of one output row: N rounded up to 16
-  unsigned char* out;  // [split or group][modulus][M][ld]
+  unsigned char* out;  // [split or group][NP][M][ld]: bytes of residues, exponents of magnitudes
   int* status;
   unsigned long long wait_ns;
   ModTab t;
@@ -433,16 +542,29 @@ struct RSmem {
   static_assert(BN == 64 || BN == 128 || BN == 256, "two accumulators in a power of two columns");
 };
 
-// One unit of work: an output tile of one modulus, the sum of up to two runs of K blocks.
+// One unit of work: an output tile of one plane, the sum of up to two runs of K blocks.
 struct Unit {
   int plane, mod, n0, blocks;  // plane: split or group; blocks: K blocks in all
   long long m0;
   int ma[2], mb[2], ya[2], yb[2], kb[2], nk[2];
 };
 
-// Unit u -> (modulus, split or group, tile): neighbouring groups share row blocks of one
-// modulus.  The tile order within a modulus is
-// tc_gemm_kernel's raster (groups of gm M tiles, M fastest), so a wave shares the row blocks of
+// The two products of orientation q of a triple (i, j, k): [VT | TM] (swap false) or [VN | TMT] of
+// occupied index a, with [T2P | OB] of the pair (bx, by).
+struct T3Product {
+  int swap, a, bx, by;
+};
+__device__ __forceinline__ T3Product t3_product(int q, int s, int i, int j, int k) {
+  T3Product t;
+  t.swap = (q == 2) != (s == 1);
+  t.a = s == 0 ? (q == 2 ? k : i) : (q == 1 ? k : j);
+  t.bx = q == 0 ? k : (q == 1 ? j : i);
+  t.by = s == 0 ? (q == 1 ? k : j) : (q == 2 ? k : i);
+  return t;
+}
+
+// Unit u -> (plane, split or group, tile): neighbouring groups share row blocks of one plane (mod:
+// a modulus, or NM for the magnitudes).  The tile order within a plane is tc_gemm_kernel's raster (groups of gm M tiles, M fastest), so a wave shares the row blocks of
 // both operands in L2.
 template <bool TRIP, bool SEGS>
 __device__ __forceinline__ Unit decode_unit(const GemmArgs& p, unsigned u) {
@@ -470,16 +592,13 @@ __device__ __forceinline__ Unit decode_unit(const GemmArgs& p, unsigned u) {
   if (SEGS) {
     const int q = x.plane % 3;
     const int i = p.ijk[x.plane - q], j = p.ijk[x.plane - q + 1], k = p.ijk[x.plane - q + 2];
-    // (A map, its occupied index, the pair of B's row block) per product
-    const int s0 = q == 2 ? k : i, s1 = q == 0 ? j : (q == 1 ? k : j);
-    const int bx = q == 0 ? k : (q == 1 ? j : i);
-    const int by[2] = {q == 0 ? j : (q == 1 ? k : j), q == 0 ? i : (q == 1 ? i : k)};
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
-      x.ma[s] = (q == 2) != (s == 1);
+      const T3Product t = t3_product(q, s, i, j, k);
+      x.ma[s] = t.swap;
       x.mb[s] = 0;
-      x.ya[s] = (int)(((long long)x.mod * p.no + (s ? s1 : s0)) * p.M + x.m0);
-      x.yb[s] = (int)(((long long)x.mod * p.no * p.no + bx * p.no + by[s]) * p.N + x.n0);
+      x.ya[s] = (int)(((long long)x.mod * p.no + t.a) * p.M + x.m0);
+      x.yb[s] = (int)(((long long)x.mod * p.no * p.no + t.bx * p.no + t.by) * p.N + x.n0);
       x.kb[s] = 0;
       x.nk[s] = p.kc;
     }
@@ -491,9 +610,9 @@ __device__ __forceinline__ Unit decode_unit(const GemmArgs& p, unsigned u) {
 // quarter and a column half each).  The two TMEM accumulators alternate between chunks of
 // kChunk K blocks; the epilogue warps add each chunk to their running residues (BN / 2
 // registers per thread) and reduce modulo p while the other accumulator fills: two FP32
-// instructions per element and chunk.  3600 x 3600 x 3600: 921 us (1.62 PFLOP/s) against 993 with
-// four, 3600 x 3600 x 400 159 against 180.  Every wait is bounded; an expired one leaves its code
-// in *status and the caller's outputs become NaN.
+// instructions per element and chunk.  Sixteen planes of 3600 x 3600 x 3600: 921 us (1.62 PFLOP/s)
+// against 993 with four, of 3600 x 3600 x 400 159 against 180 (seventeen: 169).  Every wait is
+// bounded; an expired one leaves its code in *status and the caller's outputs become NaN.
 template <int BN, bool TRIP>
 static __global__ void __launch_bounds__(kGemmThreads, 1)
     rns_gemm_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ GemmArgs p,
@@ -667,7 +786,8 @@ static __global__ void __launch_bounds__(kGemmThreads, 1)
       if (stop) break;
       const long long row = x.m0 + q * 32 + lane;
       if (row < p.M) {
-        unsigned char* o = p.out + (((long long)x.plane * NM + x.mod) * p.M + row) * p.ld;
+        unsigned char* o = p.out + (((long long)x.plane * NP + x.mod) * p.M + row) * p.ld;
+        const bool mags = x.mod == NM;
 #pragma unroll
         for (int f = 0; f < HB / 16; ++f) {
           const int cj = h * HB + 16 * f;  // 16 columns: inside the tile and the row, or not at all
@@ -675,11 +795,18 @@ static __global__ void __launch_bounds__(kGemmThreads, 1)
             float e[16];
 #pragma unroll
             for (int j = 0; j < 8; ++j) unpair(r[8 * f + j], e[2 * j], e[2 * j + 1]);
-            *reinterpret_cast<uint4*>(o + x.n0 + cj) =
-                make_uint4(residue_bytes(e[0], e[1], e[2], e[3]),
-                           residue_bytes(e[4], e[5], e[6], e[7]),
-                           residue_bytes(e[8], e[9], e[10], e[11]),
-                           residue_bytes(e[12], e[13], e[14], e[15]));
+            uint4 w;
+            if (mags)
+              w = make_uint4(exponent_bytes(e[0], e[1], e[2], e[3]),
+                             exponent_bytes(e[4], e[5], e[6], e[7]),
+                             exponent_bytes(e[8], e[9], e[10], e[11]),
+                             exponent_bytes(e[12], e[13], e[14], e[15]));
+            else
+              w = make_uint4(residue_bytes(e[0], e[1], e[2], e[3]),
+                             residue_bytes(e[4], e[5], e[6], e[7]),
+                             residue_bytes(e[8], e[9], e[10], e[11]),
+                             residue_bytes(e[12], e[13], e[14], e[15]));
+            *reinterpret_cast<uint4*>(o + x.n0 + cj) = w;
           }
         }
       }
@@ -706,8 +833,8 @@ struct CrtSum {
       s2[e] = t.b2;
     }
   }
-  // w[l]: the four outputs' bytes modulo the l-th modulus
-  __device__ __forceinline__ void add(const CrtTab& t, const unsigned (&w)[NM]) {
+  // w[l]: the four outputs' bytes of plane l
+  __device__ __forceinline__ void add(const CrtTab& t, const unsigned (&w)[NP]) {
 #pragma unroll
     for (int l = 0; l < NM; ++l)
 #pragma unroll
@@ -817,7 +944,14 @@ inline int blocks_for(long long n, int per) {
   return (int)std::max(1LL, std::min((n + per - 1) / per, 16LL * num_sms()));
 }
 
-inline int run_norm(const Operand& a, const Operand& b, long long k0, long long k1, cudaStream_t st) {
+// Scratch for the sums of K segments: `bytes` of each operand's panel, which is packed later.
+struct NormScratch {
+  void* at[2];
+  long long bytes[2];
+};
+
+inline int run_norm(const Operand& a, const Operand& b, long long k0, long long k1,
+                    const NormScratch& scratch, cudaStream_t st) {
   NormArgs p{};
   p.o[0] = a;
   p.o[1] = b;
@@ -826,11 +960,18 @@ inline int run_norm(const Operand& a, const Operand& b, long long k0, long long 
   const long long K = k1 - k0;
   for (int s = 0; s < 2; ++s) {
     const Operand& o = p.o[s];
-    p.gx[s] = o.kfast ? (o.R + 7) / 8 : (o.R + 255) / 256;
-    const long long most = std::max(1LL, K / (o.kfast ? 512 : 32));
-    const long long segs = std::max(1LL, std::min((8LL * num_sms() + p.gx[s] - 1) / p.gx[s], most));
+    if (o.R == 0) continue;
+    p.slices[s] = !o.kfast && K >= 512 && o.R < 256LL * 8 * num_sms();
+    const int rows = o.kfast ? 8 : (p.slices[s] ? 32 : 256);
+    p.gx[s] = (o.R + rows - 1) / rows;
+    // about eight blocks per SM; each a few hundred K, and few enough parts to add up at the end
+    const long long most = o.kfast ? K / 512 : (p.slices[s] ? std::min(K / 256, 128LL) : K / 32);
+    const long long segs = std::max(1LL, std::min({(8LL * num_sms() + p.gx[s] - 1) / p.gx[s], most,
+                                                   scratch.bytes[s] / (8 * o.R)}));
     p.seg[s] = (K + segs - 1) / segs;
-    p.blocks[s] = p.gx[s] * ((K + p.seg[s] - 1) / p.seg[s]);
+    p.segs[s] = (K + p.seg[s] - 1) / p.seg[s];
+    p.blocks[s] = p.gx[s] * p.segs[s];
+    p.part[s] = (unsigned long long*)scratch.at[s];
   }
   rns_norm_kernel<<<(unsigned)(p.blocks[0] + p.blocks[1]), 256, 0, st>>>(p);
   PCG_CHECK_LAUNCH("rns norm");
@@ -852,7 +993,7 @@ inline int run_gemm(const GemmMaps& maps, const GemmArgs& a, cudaStream_t st) {
   const int smem = RSmem<BN>::TOTAL;
   cudaFuncSetAttribute(rns_gemm_kernel<BN, TRIP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        smem);
-  const long long units = a.mt * a.nt * NM * a.planes;
+  const long long units = a.mt * a.nt * NP * a.planes;
   if (units > 0x7fffffffLL) {
     set_error("rns gemm: %lld units of work", units);
     return -1;

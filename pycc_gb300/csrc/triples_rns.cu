@@ -12,11 +12,12 @@
 // exchanged], and an orientation is two products of K = nv + no: at no = 7, nv = 45 two 64-K
 // blocks in place of four.  The residue of the sum is the sum's when all four products carry the
 // same scale, so a matrix has one power of two for all its rows, chosen from its largest row norm
-// so that the sum of the four stays below half the product of the moduli.  One GEMM launch computes
+// so that the sum of the four stays below half the product of the moduli; a partial whose products
+// are small at that scale is computed again in FP64 (kDoubt in rns.cuh).  One GEMM launch computes
 // the three orientations of a batch of triples, a second kernel rebuilds the partials in FP64, in
 // the layout the energy kernel reads.  E(T) at no = 7, nv = 45: 63.4 ms with one FP64 launch per
 // triple and orientation (46.6 ms on a few SMs' FP64 pipes, a host synchronisation per triple),
-// 1.3 ms here (GEMM 0.43, 0.67 with the four products apart; rebuild 0.18, energy 0.31).
+// 1.34 ms here (GEMM 0.45, by half more with the four products apart; rebuild 0.20, energy 0.32).
 #include "rns.cuh"
 
 namespace pcg {
@@ -30,27 +31,28 @@ struct T3Shift {
 };
 
 struct T3MaxArgs {
-  const float* norm2[4];
-  const unsigned* top[4];
+  const unsigned long long* norm[4];
   long long R[4];
-  unsigned* out;  // [4] largest squared row norm (float bits), [4] largest exponent
+  unsigned* out;  // [4] largest log2 of a squared row norm, rounded up, + kT3Bias (0: no row is above
+                  // zero); [1] an Inf or a NaN
 };
+constexpr int kT3Bias = 1 << 16;
 
 __global__ void __launch_bounds__(256) t3_max_kernel(const T3MaxArgs p) {
   const int q = blockIdx.y;
-  unsigned m = 0, t = 0;
+  unsigned m = 0, bad = 0;
   for (long long r = (long long)blockIdx.x * 256 + threadIdx.x; r < p.R[q];
        r += (long long)gridDim.x * 256) {
-    m = max(m, __float_as_uint(p.norm2[q][r]));  // non-negative: bits are ordered as values
-    t = max(t, p.top[q][r]);
+    const RowNorm n = RowNorm::from(p.norm[q][r]);
+    unsigned frac;
+    if (n.s > 0.f) m = max(m, (unsigned)(n.log2(frac) + 1 + kT3Bias));
+    bad |= n.top == 2047;
   }
-  for (int s = 16; s > 0; s >>= 1) {
-    m = max(m, __shfl_xor_sync(0xffffffffu, m, s));
-    t = max(t, __shfl_xor_sync(0xffffffffu, t, s));
-  }
+  m = __reduce_max_sync(0xffffffffu, m);
+  bad = __reduce_or_sync(0xffffffffu, bad);
   if ((threadIdx.x & 31) == 0) {
     atomicMax(p.out + q, m);
-    atomicMax(p.out + 4 + q, t);
+    if (bad) p.out[4] = 1;
   }
 }
 
@@ -59,58 +61,91 @@ __global__ void __launch_bounds__(256) t3_max_kernel(const T3MaxArgs p) {
 // determine a sum of up to half the product of the moduli, 2^123.95.
 constexpr int kT3Bits = 121;
 static_assert(kT3Bits + 2 <= kSumBits, "four products stay in the range of the residues");
-__global__ void t3_shift_kernel(const unsigned* mx, int log2v, int log2o, T3Shift* out) {
+__global__ void t3_shift_kernel(const unsigned* mx, T3Shift* out) {
   int e[4];  // row norms are at most 2^e
-  bool bad = false;
-  for (int q = 0; q < 4; ++q) {
-    const float n2 = __uint_as_float(mx[q]) * 1.0078125f;
-    const int top = (int)mx[4 + q];
-    bad = bad || top == 2047;
-    const int l2 = (n2 >= 0x1p-80f && n2 <= 0x1p100f)
-                       ? (int)(__float_as_uint(n2) >> 23) - 126
-                       : 2 * (max(top, 1) - 1022) + (q < 2 ? log2v : log2o);
-    e[q] = (l2 + 1) >> 1;
-  }
+  for (int q = 0; q < 4; ++q) e[q] = mx[q] ? ((int)mx[q] - kT3Bias + 1) >> 1 : -1000;
   const int s1 = kT3Bits - e[0] - e[1], s2 = kT3Bits - e[2] - e[3], s = min(s1, s2);
   out->sh[0] = kT3Bits / 2 - e[0] - ((s1 - s) >> 1);
   out->sh[1] = s - out->sh[0];
   out->sh[2] = kT3Bits / 2 - e[2] - ((s2 - s) >> 1);
   out->sh[3] = s - out->sh[2];
   out->total = s;
-  out->bad = bad;
+  out->bad = mx[4] != 0;
 }
 
 struct T3JoinArgs {
-  const unsigned char* res;  // [group][modulus][v^2][ld]
+  const unsigned char* res;  // [group][plane][v^2][ld]
   long long ld;
   int nv, groups;
   double* P;  // [group][z][x][y]
   const T3Shift* shift;
   const int* status;
   CrtTab t;
+  // operands for partials that are computed again in FP64, or null: none is
+  const double *V, *O, *t2;
+  const int* ijk;
+  int no;
 };
 
-// Lanes along the rows (x, y), which are P's unit stride; four columns z per thread.
-__global__ void __launch_bounds__(256) t3_join_kernel(const __grid_constant__ T3JoinArgs p) {
+// One partial, orientation g % 3 of triple g / 3, by a warp with the lanes along K (e, then m).
+__device__ __noinline__ double t3_dot(const T3JoinArgs& p, int g, long long row, int z) {
+  const int q = g % 3, lane = threadIdx.x & 31;
+  const int i = p.ijk[g - q], j = p.ijk[g - q + 1], k = p.ijk[g - q + 2];
+  const long long o = p.no, v = p.nv, x = row / v, y = row - x * v;
+  double s = 0.0;
+  for (int part = 0; part < 2; ++part) {  // [VT | TM] or [VN | TMT], as decode_unit has them
+    const T3Product t = t3_product(q, part, i, j, k);
+    const long long a = t.swap ? x : y, b = t.swap ? y : x;  // VT = <qp|ex>, VN = <pq|ex>
+    const double* V = p.V + (a * v + b) * v * o + t.a;
+    const double* T = p.t2 + ((t.bx * o + t.by) * v + z) * v;
+    for (long long e = lane; e < v; e += 32) s = fma(__ldg(V + e * o), __ldg(T + e), s);
+    const double* M = p.t2 + t.a * o * v * v + b * v + a;    // TM = t2_xmpq, TMT = t2_xmqp
+    const double* O = p.O + (z * o + t.by) * o + t.bx;
+    for (long long m = lane; m < o; m += 32)
+      s = fma(-__ldg(M + m * v * v), __ldg(O + m * v * o * o), s);
+  }
+  for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+  return s;
+}
+
+// Lanes along the rows (x, y), which are P's unit stride; four columns z per thread.  A partial
+// whose products are small against the norms behind its scale (kDoubt in rns.cuh) is computed again
+// in FP64, a warp each, and so are all of them with an Inf or a NaN in an operand: at most a third of the time of one FP64 launch per triple and orientation.
+__global__ void __launch_bounds__(256, 4) t3_join_kernel(const __grid_constant__ T3JoinArgs p) {
   const long long M = (long long)p.nv * p.nv;
-  const long long row = (long long)blockIdx.x * 32 + threadIdx.x;
+  const long long row0 = (long long)blockIdx.x * 32, row = row0 + threadIdx.x;
   const int col = 4 * (int)(blockIdx.y * 8 + threadIdx.y);
-  if (row >= M || col >= p.nv) return;
-  const bool bad = *p.status != 0 || p.shift->bad;
+  if (col >= p.nv) return;  // a whole warp
+  const bool failed = *p.status != 0, bad = p.shift->bad;
   const int ex = -p.shift->total;
   for (int g = blockIdx.z; g < p.groups; g += gridDim.z) {
-    const unsigned char* src = p.res + ((long long)g * NM * M + row) * p.ld + col;
-    unsigned w[NM];
-#pragma unroll
-    for (int l = 0; l < NM; ++l)
-      w[l] = __ldg(reinterpret_cast<const unsigned*>(src + (long long)l * M * p.ld));
-    CrtSum sum(p.t);
-    sum.add(p.t, w);
     double* out = p.P + ((long long)g * p.nv + col) * M + row;
+    unsigned doubt = 0;
+    if (row < M) {
+      const unsigned char* src = p.res + ((long long)g * NP * M + row) * p.ld + col;
+      unsigned w[NP];
 #pragma unroll
-    for (int e = 0; e < 4; ++e)
-      if (col + e < p.nv)
-        out[e * M] = bad ? __longlong_as_double(0x7ff8000000000000ll) : sum.value(p.t, e, ex);
+      for (int l = 0; l < NP; ++l)
+        w[l] = __ldg(reinterpret_cast<const unsigned*>(src + (long long)l * M * p.ld));
+      CrtSum sum(p.t);
+      sum.add(p.t, w);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float mag = magnitude_sum(w[NM], e);
+        if (col + e < p.nv) {
+          out[e * M] =
+              failed || bad ? __longlong_as_double(0x7ff8000000000000ll) : sum.value(p.t, e, ex);
+          if (p.V && !failed && (bad || (mag > 0.f && mag < kDoubt))) doubt |= 1u << e;
+        }
+      }
+    }
+    if (__any_sync(0xffffffffu, doubt != 0u))
+      for (int e = 0; e < 4; ++e)
+        for (unsigned m = __ballot_sync(0xffffffffu, doubt >> e & 1u); m; m &= m - 1) {
+          const int l = __ffs((int)m) - 1;
+          const double v = t3_dot(p, g, row0 + l, col + e);
+          if (threadIdx.x == l) out[e * M] = v;
+        }
   }
 }
 
@@ -132,14 +167,14 @@ bool t3_plan(T3Plan& p, long long no, long long nv) {
   p.c0 = up(nv, 8);
   p.kc = up(p.c0 + no, 64);
   p.ld = up(nv, 16);
-  const long long a = up(NM * p.rows_a * p.kc * 2, 256);
+  const long long a = up(NP * p.rows_a * p.kc * 2, 256);
   p.a1 = 256;
   p.a2 = p.a1 + a;
   p.b = p.a2 + a;
-  p.fixed = p.b + up(NM * p.rows_b * p.kc * 2, 256);
-  p.tables = (4 * p.rows_a + 2 * p.rows_b) * (8 + 4 + 4 + 4) + 6 * 4 * 16;
-  p.per_triple = 3 * NM * nv * nv * p.ld;
-  return NM * p.rows_a < 0x7fffffffLL - BM && NM * p.rows_b < 0x7fffffffLL - 256 &&
+  p.fixed = p.b + up(NP * p.rows_b * p.kc * 2, 256);
+  p.tables = (4 * p.rows_a + 2 * p.rows_b) * (8 + 8 + 4) + 6 * 3 * 16;
+  p.per_triple = 3 * NP * nv * nv * p.ld;
+  return NP * p.rows_a < 0x7fffffffLL - BM && NP * p.rows_b < 0x7fffffffLL - 256 &&
          (p.rows_a / 64 + p.rows_b / 32 + 4) * (p.kc / 64) < 0x7fffffffLL;
 }
 
@@ -192,9 +227,8 @@ extern "C" int pcg_t3_rns_pack(const double* V, const double* O, const double* t
     x.r.s0[2] = s2;
     x.R = e0 * e1 * e2;
     x.off = (long long*)take(8 * x.R);
+    x.norm = (unsigned long long*)take(8 * x.R);
     x.walk = (int*)take(4 * x.R);
-    x.top = (unsigned*)take(4 * x.R);
-    x.norm2 = (float*)take(4 * x.R);
     x.kstep = kstep;
     x.kfast = kstep == 1;
     x.wq = near;
@@ -219,34 +253,31 @@ extern "C" int pcg_t3_rns_pack(const double* V, const double* O, const double* t
     rns_tables_kernel<<<blocks_for(x.a.R + x.b.R, 256), 256, 0, st>>>(t);
     PCG_CHECK_LAUNCH("pcg_t3_rns_pack/tables");
   }
+  const NormScratch scratch{{w + p.a1, w + p.b}, {p.a2 - p.a1, p.fixed - p.b}};
   for (int q = 0; q < 2; ++q)
-    if (run_norm(pass[q].a, pass[q].b, 0, pass[q].K, st)) return -2;
-  T3MaxArgs m{{vt.norm2, t2p.norm2, tm.norm2, ob.norm2}, {vt.top, t2p.top, tm.top, ob.top},
-              {vt.R, t2p.R, tm.R, ob.R}, mx};
+    if (run_norm(pass[q].a, pass[q].b, 0, pass[q].K, scratch, st)) return -2;
+  T3MaxArgs m{{vt.norm, t2p.norm, tm.norm, ob.norm}, {vt.R, t2p.R, tm.R, ob.R}, mx};
   t3_max_kernel<<<dim3(num_sms(), 4), 256, 0, st>>>(m);
   PCG_CHECK_LAUNCH("pcg_t3_rns_pack/max");
-  auto log2up = [](long long x) {
-    int l = 0;
-    while ((1LL << l) < x) ++l;
-    return l;
-  };
-  t3_shift_kernel<<<1, 1, 0, st>>>(mx, log2up(v), log2up(o), shift);
+  t3_shift_kernel<<<1, 1, 0, st>>>(mx, shift);
   PCG_CHECK_LAUNCH("pcg_t3_rns_pack/shift");
   for (auto& x : pass) {
     PackArgs a{{{x.a, 0, x.a.R, (__nv_bfloat16*)(w + x.pa) + x.c0, 0, 0},
                 {x.b, 0, x.b.R, (__nv_bfloat16*)(w + x.pb) + x.c0, x.b.X == O ? 0x80000000u : 0u, 0}},
-               0, x.K, x.width, p.kc, 0, tables().pairs};
+               0, x.K, x.width, p.kc, tables().pairs};
     if (run_pack(a, st)) return -2;
   }
   return 0;
 }
 
-extern "C" int pcg_t3_rns_partials(long long no, long long nv, const int* ijk, int ntrip, double* P,
-                                   void* work, long long work_len, void* stream) {
+namespace {
+int t3_partials(const double* V, const double* O, const double* t2, long long no, long long nv,
+                const int* ijk, int ntrip, double* P, void* work, long long work_len, void* stream,
+                const char* who) {
   T3Plan p;
   if (!ijk || ntrip < 1 || ntrip > 21845 || !P || !work || ((uintptr_t)work & 255u) ||
       !t3_plan(p, no, nv) || work_len < p.fixed + ntrip * p.per_triple) {
-    set_error("pcg_t3_rns_partials: bad arguments, or too little workspace");
+    set_error("%s: bad arguments, or too little workspace", who);
     return -1;
   }
   cudaStream_t st = (cudaStream_t)stream;
@@ -269,18 +300,36 @@ extern "C" int pcg_t3_rns_partials(long long no, long long nv, const int* ijk, i
   g.no = (int)no;
   g.kc = (int)(p.kc / 64);
   GemmMaps maps{};
-  if (!make_map(&maps.a[0], w + p.a1, NM * p.rows_a, 2 * p.kc, 2 * p.kc, 2, BM) ||
-      !make_map(&maps.a[1], w + p.a2, NM * p.rows_a, 2 * p.kc, 2 * p.kc, 2, BM) ||
-      !make_map(&maps.b[0], w + p.b, NM * p.rows_b, 2 * p.kc, 2 * p.kc, 2, g.bs))
+  if (!make_map(&maps.a[0], w + p.a1, NP * p.rows_a, 2 * p.kc, 2 * p.kc, 2, BM) ||
+      !make_map(&maps.a[1], w + p.a2, NP * p.rows_a, 2 * p.kc, 2 * p.kc, 2, BM) ||
+      !make_map(&maps.b[0], w + p.b, NP * p.rows_b, 2 * p.kc, 2 * p.kc, 2, g.bs))
     return -1;
   const int rc = BN == 256   ? run_gemm<256, true>(maps, g, st)
                  : BN == 128 ? run_gemm<128, true>(maps, g, st)
                              : run_gemm<64, true>(maps, g, st);
   if (rc) return rc;
   T3JoinArgs j{w + p.fixed, p.ld, (int)nv, g.planes, P, (const T3Shift*)(w + 128),
-               (const int*)w, crt_tab(1, 1.0)};
+               (const int*)w, crt_tab(1, 1.0), V, O, t2, ijk, (int)no};
   const dim3 grid((unsigned)((g.M + 31) / 32), (unsigned)((nv + 31) / 32), (unsigned)g.planes);
   t3_join_kernel<<<grid, dim3(32, 8), 0, st>>>(j);
-  PCG_CHECK_LAUNCH("pcg_t3_rns_partials");
+  PCG_CHECK_LAUNCH(who);
   return 0;
+}
+}  // namespace
+
+extern "C" int pcg_t3_rns_partials(long long no, long long nv, const int* ijk, int ntrip, double* P,
+                                   void* work, long long work_len, void* stream) {
+  return t3_partials(nullptr, nullptr, nullptr, no, nv, ijk, ntrip, P, work, work_len, stream,
+                     "pcg_t3_rns_partials");
+}
+
+extern "C" int pcg_t3_rns_partials_of(const double* V, const double* O, const double* t2, long long no,
+                                      long long nv, const int* ijk, int ntrip, double* P, void* work,
+                                      long long work_len, void* stream) {
+  if (!V || !O || !t2) {
+    set_error("pcg_t3_rns_partials_of: null operand");
+    return -1;
+  }
+  return t3_partials(V, O, t2, no, nv, ijk, ntrip, P, work, work_len, stream,
+                     "pcg_t3_rns_partials_of");
 }

@@ -157,8 +157,8 @@ def t_energy_fp64(w, t1=None, t2=None):
                   work.data_ptr(), work.numel(), st)
         for t0 in range(0, len(trips), batch):
             n = min(batch, len(trips) - t0)
-            _lib.call("pcg_t3_rns_partials", no, nv, ijk[t0:].data_ptr(), n, P.data_ptr(),
-                      work.data_ptr(), work.numel(), st)
+            _lib.call("pcg_t3_rns_partials_of", V.data_ptr(), O.data_ptr(), t2.data_ptr(), no, nv,
+                      ijk[t0:].data_ptr(), n, P.data_ptr(), work.data_ptr(), work.numel(), st)
             energy(t0, n, P)
     out = torch.zeros((), dtype=torch.float64, device=dev)
     _lib.call("pcg_reduce_sum_f64", part.data_ptr(), part.numel(), out.data_ptr(), st)

@@ -154,3 +154,64 @@ def test_dispatch(cuda):
     st.synchronize()
     assert torch.equal(got, side)
     assert (abs(got[::23, ::23].cpu().numpy() - ref) <= tol).all()
+
+
+def graded(shape, gen, decades):
+    """Random signs and mantissas, magnitudes over as many decades."""
+    x = torch.randn(shape, dtype=torch.float64, device="cuda:0", generator=gen)
+    return x * 10.0 ** (-decades * torch.rand(shape, dtype=torch.float64, device="cuda:0",
+                                              generator=gen))
+
+
+def check_products(got, a, b, subs, c0=None, alpha=1.0, beta=0.0):
+    """Every output within the bound of FP64 multiply-adds: the residues' rounding gives at most
+    sqrt(K) 2^-52 sum |a||b| where they are used, FP64 sums K 2^-53, and the rest eight roundings."""
+    A, B = (x.cpu().numpy().astype(np.longdouble) for x in (a, b))
+    S = np.einsum(subs, abs(A), abs(B))
+    want = alpha * np.einsum(subs, A, B)
+    k = math.prod(n for c, n in zip(subs, A.shape) if c not in subs.split("->")[1])
+    tol = abs(alpha) * 2.0 ** -53 * (max(2 * math.sqrt(k), k) + 8) * S
+    if c0 is not None:
+        c = beta * c0.cpu().numpy().astype(np.longdouble)
+        want, tol = want + c, tol + 2.0 ** -51 * abs(c)
+    assert (abs(got.cpu().numpy() - want) <= tol).all()
+    zero = (S == 0) if c0 is None else np.zeros_like(S, dtype=bool)
+    assert (got.cpu().numpy()[zero] == 0).all()
+
+
+@pytest.mark.parametrize("subs", ["mk,nk->mn", "km,kn->mn", "mk,kn->nm"])
+@pytest.mark.parametrize("m,n,k,limit", [(3, 5, 2, None), (65, 33, 64, None), (130, 70, 961, None),
+                                         (13, 16, 30011, None), (300, 260, 3000, 30 << 20)])
+def test_graded_rows(cuda, subs, m, n, k, limit):
+    """Magnitudes over twenty decades within the rows, some rows with zeros where the others are
+    large: products that are far below the norms of their rows keep FP64's relative accuracy."""
+    gen = torch.Generator(device=cuda).manual_seed(m + k)
+    a, b = graded((m, k), gen, 20.0), graded((n, k), gen, 20.0)
+    a[m // 2:, : k // 2] *= 1e30
+    b[n // 2:, : k // 2] = 0.0
+    a[0, k // 3:] = 0.0
+    b[1, : k // 3] = 0.0
+    la, lb = subs.split("->")[0].split(",")
+    a = a if la == "mk" else a.t().contiguous()
+    b = b if lb == "nk" else b.t().contiguous()
+    shape = (m, n) if subs.endswith("mn") else (n, m)
+    nan = torch.full(shape, float("nan"), dtype=torch.float64, device=cuda)
+    kw = {} if limit is None else {"limit": limit}
+    check_products(rns(subs, a, b, nan, **kw), a, b, subs)
+    c0 = graded(shape, gen, 20.0)
+    check_products(rns(subs, a, b, c0.clone(), alpha=-1.5, beta=0.25, **kw), a, b, subs, c0, -1.5,
+                   0.25)
+
+
+@pytest.mark.parametrize("s", [1e-9, 1e-15, 1e-18, 2.0 ** -70, 1e-100, 1e-300])
+def test_small_products_of_large_rows(cuda, s):
+    """(1, s, s, ...) times (0, 1-sized, ...): the rows' largest entries meet zeros."""
+    gen = torch.Generator(device=cuda).manual_seed(6)
+    a, b = (torch.randn(70, 512, dtype=torch.float64, device=cuda, generator=gen)
+            for _ in range(2))
+    a[:, 1:] *= s
+    a[:, 0] = 1.0
+    b[::2, 0] = 0.0
+    out = torch.empty(70, 70, dtype=torch.float64, device=cuda)
+    check_products(rns("mk,nk->mn", a, b, out), a, b, "mk,nk->mn")
+    check_products(contract_f64("mk,nk->mn", a.repeat(8, 1), b), a.repeat(8, 1), b, "mk,nk->mn")
