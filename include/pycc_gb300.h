@@ -78,12 +78,27 @@ int pcg_contract_rns_f64_work(long long M, long long N, long long K, long long l
  * were packed as well, and computes by FP64 multiply-adds the partials whose products are small
  * against those norms, or all of them if an operand holds an Inf or a NaN: the error of every partial
  * is at most (nv + no) 2^-51 times the sum of its products' magnitudes.  In both an expired
- * device-side wait makes the partials NaN. */
+ * device-side wait makes the partials NaN.
+ * The residues of all occupied orbitals take about 68 no nv^2 (nv + no) bytes.  In windows they take
+ * 2 c / no of that: i, j and k come from slots of at most c orbitals, [first[q], first[q] + c)
+ * for q = 0, 1, 2, which start at multiples of c and do not increase.  pcg_t3_rns_scales once per
+ * amplitudes (it clears the workspace's status), pcg_t3_rns_window_pack for each window (`changed`:
+ * bits of the slots that differ from the window packed before, 7 for the first), then
+ * pcg_t3_rns_window_partials for its triples.  pcg_t3_rns_pack is scales and pack with c = no. */
 int pcg_t3_rns_work(long long no, long long nv, int batch, long long* bytes);
 int pcg_t3_rns_pack(const double* V, const double* O, const double* t2, long long no, long long nv,
                     void* work, long long work_len, void* stream);
 int pcg_t3_rns_partials(long long no, long long nv, const int* ijk, int ntrip, double* P, void* work,
                         long long work_len, void* stream);
+int pcg_t3_rns_window_work(long long no, long long nv, long long c, int batch, long long* bytes);
+int pcg_t3_rns_scales(const double* V, const double* O, const double* t2, long long no, long long nv,
+                      long long c, void* work, long long work_len, void* stream);
+int pcg_t3_rns_window_pack(const double* V, const double* O, const double* t2, long long no,
+                           long long nv, long long c, const int* first, int changed, void* work,
+                           long long work_len, void* stream);
+int pcg_t3_rns_window_partials(const double* V, const double* O, const double* t2, long long no,
+                               long long nv, long long c, const int* first, const int* ijk, int ntrip,
+                               double* P, void* work, long long work_len, void* stream);
 int pcg_t3_rns_partials_of(const double* V, const double* O, const double* t2, long long no,
                            long long nv, const int* ijk, int ntrip, double* P, void* work,
                            long long work_len, void* stream);

@@ -38,6 +38,12 @@ SIGNATURES = {
     "pcg_t3_rns_work": (C.c_int, [_i64, _i64, C.c_int, _pi64]),
     "pcg_t3_rns_pack": (C.c_int, [_p, _p, _p, _i64, _i64, _p, _i64, _p]),
     "pcg_t3_rns_partials": (C.c_int, [_i64, _i64, _p, C.c_int, _p, _p, _i64, _p]),
+    "pcg_t3_rns_window_work": (C.c_int, [_i64, _i64, _i64, C.c_int, _pi64]),
+    "pcg_t3_rns_scales": (C.c_int, [_p, _p, _p, _i64, _i64, _i64, _p, _i64, _p]),
+    "pcg_t3_rns_window_pack": (C.c_int, [_p, _p, _p, _i64, _i64, _i64, C.POINTER(C.c_int), C.c_int,
+                                         _p, _i64, _p]),
+    "pcg_t3_rns_window_partials": (C.c_int, [_p, _p, _p, _i64, _i64, _i64, C.POINTER(C.c_int), _p,
+                                             C.c_int, _p, _p, _i64, _p]),
     "pcg_t3_rns_partials_of": (C.c_int, [_p, _p, _p, _i64, _i64, _p, C.c_int, _p, _p, _i64, _p]),
     "pcg_tau_f64": (C.c_int, [_p, _p, _i64, _i64, _d, _d, _p, _p]),
     "pcg_combine4_f64": (C.c_int, [_pi64, _d, _p, _pi64, _d, _p, _pi64, _p, _pi64, _p]),

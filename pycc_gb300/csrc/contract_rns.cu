@@ -481,8 +481,9 @@ extern "C" int pcg_contract_rns_f64(int m_n, const long long* m_ext, const long 
       for (long long m0 = 0; m0 < M; m0 += p.PM) {
         const long long mm = std::min(p.PM, M - m0);
         // B's panel is packed with the first panel of A
-        PackArgs q{{{a, m0, mm, pa, 0, 0}, {b, n0, m0 == 0 ? nn : 0, pb, 0, 0}}, k0, kn, p.Kp, p.Kp,
-                   t.pairs};
+        PackArgs q{{{a, m0, mm, pa, mm * p.Kp / 8, 0, 0},
+                    {b, n0, m0 == 0 ? nn : 0, pb, nn * p.Kp / 8, 0, 0}},
+                   k0, kn, p.Kp, p.Kp, t.pairs};
         if (run_pack(q, st)) return -2;
         GemmArgs g{};
         g.M = mm;

@@ -381,7 +381,8 @@ __device__ __forceinline__ void digits(double x, double y, int s, unsigned flip,
 struct PackSide {
   Operand o;
   long long w0, nrow;  // rows of this panel: walk positions [w0, w0 + nrow); nrow 0: none
-  __nv_bfloat16* out;  // [plane][nrow][ld]
+  __nv_bfloat16* out;  // [plane][row][ld]
+  long long plane;     // 16-byte units from a plane to the next
   unsigned flip;       // 0x80000000: the negated operand
   long long blocks;
 };
@@ -406,7 +407,7 @@ __device__ __forceinline__ void store_residues(const PackArgs& p, const PackSide
 #pragma unroll
   for (int e = 0; e < 4; ++e) digits(x[2 * e], x[2 * e + 1], s, o.flip, d[e]);
   uint4* out = reinterpret_cast<uint4*>(o.out + at);
-  const long long plane = (o.nrow * p.ld) >> 3;
+  const long long plane = o.plane;
   unsigned r[4];
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
@@ -517,9 +518,12 @@ struct GemmArgs {
   int* status;
   unsigned long long wait_ns;
   ModTab t;
-  // TRIP
-  const int* ijk;  // [triples][3]
-  int no, kc;      // occupied orbitals, K blocks of a product over e and m
+  // TRIP (T3Plan in triples_rns.cu)
+  const int* ijk;           // [triples][3]
+  int kc;                   // K blocks of a product over e and m
+  int blocks_a, pairs;      // blocks of v^2 rows of an A matrix, pairs (blocks of v rows) of B
+  int c, first[3], width[3];  // of i, j, k: slots of c occupied indices from first on, width of them
+                              // present; c = 0: one slot for all of them
 };
 
 struct GemmMaps {
@@ -549,17 +553,18 @@ struct Unit {
   int ma[2], mb[2], ya[2], yb[2], kb[2], nk[2];
 };
 
-// The two products of orientation q of a triple (i, j, k): [VT | TM] (swap false) or [VN | TMT] of
-// occupied index a, with [T2P | OB] of the pair (bx, by).
+// The two products of orientation q of a triple, in indices 0, 1, 2 for i, j, k: [VT | TM] (swap 0)
+// or [VN | TMT] of occupied index a, with [T2P | OB] of the pair (bx, by).  [VT | TM] meets i and j
+// only, [VN | TMT] j and k.
 struct T3Product {
   int swap, a, bx, by;
 };
-__device__ __forceinline__ T3Product t3_product(int q, int s, int i, int j, int k) {
+__device__ __forceinline__ T3Product t3_product(int q, int s) {
   T3Product t;
   t.swap = (q == 2) != (s == 1);
-  t.a = s == 0 ? (q == 2 ? k : i) : (q == 1 ? k : j);
-  t.bx = q == 0 ? k : (q == 1 ? j : i);
-  t.by = s == 0 ? (q == 1 ? k : j) : (q == 2 ? k : i);
+  t.a = s == 0 ? (q == 2 ? 2 : 0) : (q == 1 ? 2 : 1);
+  t.bx = 2 - q;
+  t.by = s == 0 ? (q == 1 ? 2 : 1) : (q == 2 ? 2 : 0);
   return t;
 }
 
@@ -591,14 +596,20 @@ __device__ __forceinline__ Unit decode_unit(const GemmArgs& p, unsigned u) {
   x.blocks = 2 * p.kc;
   if (SEGS) {
     const int q = x.plane % 3;
-    const int i = p.ijk[x.plane - q], j = p.ijk[x.plane - q + 1], k = p.ijk[x.plane - q + 2];
+    int at[3];  // place of i, j, k in their slots
+#pragma unroll
+    for (int r = 0; r < 3; ++r) at[r] = p.ijk[x.plane - q + r] - p.first[r];
+    auto of = [](const int (&v)[3], int r) { return r == 0 ? v[0] : (r == 1 ? v[1] : v[2]); };
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
-      const T3Product t = t3_product(q, s, i, j, k);
+      const T3Product t = t3_product(q, s);
+      const int block = (t.a - t.swap) * p.c + of(at, t.a);
+      const int pair = (3 * t.bx + t.by) * p.c * p.c + of(at, t.bx) * of(p.width, t.by) +
+                       of(at, t.by);
       x.ma[s] = t.swap;
       x.mb[s] = 0;
-      x.ya[s] = (int)(((long long)x.mod * p.no + t.a) * p.M + x.m0);
-      x.yb[s] = (int)(((long long)x.mod * p.no * p.no + t.bx * p.no + t.by) * p.N + x.n0);
+      x.ya[s] = (int)(((long long)x.mod * p.blocks_a + block) * p.M + x.m0);
+      x.yb[s] = (int)(((long long)x.mod * p.pairs + pair) * p.N + x.n0);
       x.kb[s] = 0;
       x.nk[s] = p.kc;
     }

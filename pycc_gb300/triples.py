@@ -21,6 +21,7 @@ from __future__ import annotations
 
 import contextlib
 import ctypes as C
+import functools
 
 import torch
 
@@ -91,36 +92,81 @@ def triples_list(no):
     return [(i, j, k) for i in range(no) for j in range(i + 1) for k in range(j + 1)]
 
 
-T3_WORK_LIMIT = 8 << 30      # bytes of scratch (residues, products and partials) of one E(T)
+# Bytes of scratch (residues, products and partials) of one E(T), or, where that is more, what one
+# triple needs: 136 nv^2 (nv + no) of residues and 75 nv^3 of products and partials.
+T3_WORK_LIMIT = 8 << 30
 
 
-def _t3_scratch(no, nv, ntrip, device, stream):
-    """(work, partials, batch) for the residue path on ``device``, owned by the launching stream,
-    or None when the device has no room for it.  The residues of the operands are one block for
-    all triples; the batch takes what the limit leaves, at least one triple."""
-    def bytes_of(batch):
-        out = C.c_longlong(0)
-        _lib.call("pcg_t3_rns_work", no, nv, batch, C.byref(out))
-        return out.value
-    if not bytes_of(1):
+@functools.lru_cache(maxsize=4096)
+def _t3_bytes(no, nv, c, batch):
+    """Scratch for windows of c occupied orbitals a slot and batches of triples (0: sizes refused)."""
+    out = C.c_longlong(0)
+    _lib.call("pcg_t3_rns_window_work", no, nv, c, batch, C.byref(out))
+    return out.value and out.value + 24 * batch * nv ** 3
+
+
+def _t3_plan(no, nv, limit):
+    """(c, batch): the window width and the triples of a batch that fit ``limit`` bytes, at least one
+    orbital and one triple; None for sizes that the residue path refuses.
+
+    All orbitals in one window where that leaves room for about 16e6 elements of partials (fewer keep
+    the launches longer than the work), else the widest windows: the packs of a slot are repeated for
+    each window that it is in."""
+    if not _t3_bytes(no, nv, 1, 1):
         return None
-    each = bytes_of(1 << 20) - bytes_of((1 << 20) - 1) + 24 * nv ** 3
-    batch = max(1, min(ntrip, 4096, (T3_WORK_LIMIT - bytes_of(1)) // each))
+    ntrip = no * (no + 1) * (no + 2) // 6
+    for c in [no] + list(range((no - 1) // 2, 0, -1)):
+        most = min(4096, ntrip, c ** 3 if c < no else ntrip)
+        want = max(1, min(most, 2 ** 24 // (3 * nv ** 3)))
+        if not 0 < _t3_bytes(no, nv, c, want) <= limit:
+            continue
+        each = _t3_bytes(no, nv, c, 4096) - _t3_bytes(no, nv, c, 4095)
+        return c, min(most, want + (limit - _t3_bytes(no, nv, c, want)) // each)
+    return 1, 1
+
+
+def _t3_scratch(no, nv, device, stream):
+    """(work, partials, c, batch) for the residue path on ``device``, owned by the launching stream,
+    or None when it cannot run there or the device has no room even for one triple."""
+    if device.type != "cuda":
+        return None
     with torch.cuda.stream(stream) if stream is not None else contextlib.nullcontext():
-        for b in sorted({batch, min(batch, 4), 1}, reverse=True):
+        limit = T3_WORK_LIMIT
+        while (plan := _t3_plan(no, nv, limit)) is not None:
+            c, batch = plan
+            nbytes = _t3_bytes(no, nv, c, batch) - 24 * batch * nv ** 3
             try:
-                return (torch.empty(bytes_of(b), dtype=torch.uint8, device=device),
-                        torch.empty((b, 3, nv, nv, nv), dtype=torch.float64, device=device), b)
+                return (torch.empty(nbytes, dtype=torch.uint8, device=device),
+                        torch.empty((batch, 3, nv, nv, nv), dtype=torch.float64, device=device),
+                        c, batch)
             except torch.cuda.OutOfMemoryError:
-                pass
+                if plan == (1, 1):
+                    break
+                limit = min(limit, nbytes) // 4
     return None
+
+
+def _t3_windows(no, c):
+    """The triples i >= j >= k in windows of c orbitals a slot: (first orbitals of the slots, which
+    slots differ from the window before, triples)."""
+    last = None
+    for i0 in range(0, no, c):
+        for j0 in range(0, i0 + 1, c):
+            for k0 in range(0, j0 + 1, c):
+                first = (i0, j0, k0)
+                trips = [(i, j, k) for i in range(i0, min(i0 + c, no))
+                         for j in range(j0, min(j0 + c, i + 1)) for k in range(k0, min(k0 + c, j + 1))]
+                changed = 7 if last is None else sum((first[r] != last[r]) << r for r in range(3))
+                last = first
+                yield first, changed, trips
 
 
 def t_energy_fp64(w, t1=None, t2=None):
     """E(T) with FP64 partials and FP64 energy arithmetic.
 
     The partials of a batch of triples come from one launch of the residue GEMM on the tensor
-    cores (``csrc/triples_rns.cu``); without room for its scratch, from the FP64 multi-term
+    cores (``csrc/triples_rns.cu``), in windows of the occupied index where the residues of all
+    would exceed ``T3_WORK_LIMIT``; without room for one triple, from the FP64 multi-term
     contraction, one triple and orientation at a time."""
     t1 = (w.t1 if t1 is None else t1).contiguous()
     t2 = (w.t2 if t2 is None else t2).contiguous()
@@ -130,8 +176,9 @@ def t_energy_fp64(w, t1=None, t2=None):
     O = w.H.ERI[o, v, o, o]
     dev = t2.device
     st = _lib.stream_handle(w.stream)
-    trips = triples_list(no)
-    scratch = _t3_scratch(no, nv, len(trips), dev, w.stream) if t2.is_cuda else None
+    scratch = _t3_scratch(no, nv, dev, w.stream)
+    windows = list(_t3_windows(no, no if scratch is None else scratch[2]))
+    trips = [t for window in windows for t in window[2]]
     part = torch.empty((len(trips), nv), dtype=torch.float64, device=dev)
     ijk = torch.tensor(trips, dtype=torch.int32, device=dev)
     fov = w.H.F[o, v].contiguous()
@@ -151,15 +198,20 @@ def t_energy_fp64(w, t1=None, t2=None):
                 contract_multi(P[0, q].permute(1, 2, 0), lab, terms, stream=w.stream)
             energy(t, 1, P)
     else:
-        work, P, batch = scratch
+        work, P, c, batch = scratch
         V, O = V.contiguous(), O.contiguous()
-        _lib.call("pcg_t3_rns_pack", V.data_ptr(), O.data_ptr(), t2.data_ptr(), no, nv,
-                  work.data_ptr(), work.numel(), st)
-        for t0 in range(0, len(trips), batch):
-            n = min(batch, len(trips) - t0)
-            _lib.call("pcg_t3_rns_partials_of", V.data_ptr(), O.data_ptr(), t2.data_ptr(), no, nv,
-                      ijk[t0:].data_ptr(), n, P.data_ptr(), work.data_ptr(), work.numel(), st)
-            energy(t0, n, P)
+        ops = (V.data_ptr(), O.data_ptr(), t2.data_ptr(), no, nv, c)
+        room = (work.data_ptr(), work.numel(), st)
+        _lib.call("pcg_t3_rns_scales", *ops, *room)
+        t0 = 0
+        for first, changed, of_window in windows:
+            slots = (C.c_int * 3)(*first)
+            _lib.call("pcg_t3_rns_window_pack", *ops, slots, changed, *room)
+            for n in [min(batch, len(of_window) - q) for q in range(0, len(of_window), batch)]:
+                _lib.call("pcg_t3_rns_window_partials", *ops, slots, ijk[t0:].data_ptr(), n,
+                          P.data_ptr(), *room)
+                energy(t0, n, P)
+                t0 += n
     out = torch.zeros((), dtype=torch.float64, device=dev)
     _lib.call("pcg_reduce_sum_f64", part.data_ptr(), part.numel(), out.data_ptr(), st)
     return float(out)

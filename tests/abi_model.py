@@ -299,6 +299,30 @@ class ABIModel:
                                                                 list(range(n_n, n_n + kn))))
         Cv[...] = acc if beta == 0.0 else beta * Cv + acc
 
+    # -- FP64 (T) in residue arithmetic: the same partials, from slots that were packed ----------
+    def t3_rns_scales(self, V, O, t2, no, nv, c, work, length, _st):
+        self.t3_slots = [None] * 3
+
+    def t3_rns_window_pack(self, V, O, t2, no, nv, c, first, changed, work, length, _st):
+        for q in range(3):
+            assert 0 <= first[q] < no and first[q] % c == 0 and (q == 0 or first[q] <= first[q - 1])
+            if changed >> q & 1:
+                self.t3_slots[q] = first[q]
+
+    def t3_rns_window_partials(self, V, O, t2, no, nv, c, first, ijk, ntrip, P, work, length, _st):
+        assert self.t3_slots == [first[q] for q in range(3)]
+        from pycc_gb300.triples import orientation_terms
+        import torch
+        arr = [torch.from_numpy(flat(p, int(np.prod(s))).reshape(s).copy()) for p, s in
+               ((V, (nv, nv, nv, no)), (O, (no, nv, no, no)), (t2, (no, no, nv, nv)))]
+        out = flat(P, 3 * ntrip * nv ** 3).reshape(ntrip, 3, nv, nv, nv)
+        for t, (i, j, k) in enumerate(flat(ijk, 3 * ntrip, np.int32).reshape(ntrip, 3)):
+            assert all(0 <= x - f < c for x, f in zip((i, j, k), self.t3_slots))
+            for q, (lab, terms) in enumerate(orientation_terms(i, j, k, arr[2], arr[0], arr[1])):
+                W = sum(a * torch.einsum("%s,%s->%s" % (la, lb, lab), A, B)
+                        for a, A, la, B, lb in terms)
+                out[t, q] = W.permute(2, 0, 1).numpy()   # [z][x][y]
+
     def tc_grouped_gemm(self, na, a_ptr, a_rows, a_ld, nb, b_ptr, b_rows, b_ld, groups, ngroups,
                         M, N, Cp, ldm, ldn, _status, _st):
         from pycc_gb300.triples_tc import GROUP_DTYPE

@@ -152,3 +152,34 @@ def test_energy_with_a_large_idle_slab(cuda, monkeypatch):
     monkeypatch.setattr(triples, "_t3_scratch", lambda *a: None)
     ref = triples.t_energy_fp64(w)
     assert ref != 0.0 and abs(got - ref) <= 1e-12 * abs(ref)
+
+
+def wave_function(no, nv, device, seed=2):
+    import pycc_gb300 as pg
+    F, ERI, L = pg.SyntheticFactors(no, nv, seed).hamiltonian()
+    return pg.CCwfn(pg.Hamiltonian.from_arrays(F, ERI, no, L=L, device=device))
+
+
+@pytest.mark.parametrize("no,nv,c,batch", [(7, 12, 3, 1000), (7, 12, 2, 3), (5, 70, 1, 1),
+                                           (9, 9, 4, 5)])
+def test_windows(cuda, monkeypatch, no, nv, c, batch):
+    """Windows of the occupied index, the last ragged, give the energy of one window for all."""
+    from pycc_gb300 import triples
+    w = wave_function(no, nv, cuda)
+    full = triples.t_energy_fp64(w)
+    monkeypatch.setattr(triples, "_t3_plan", lambda *a: (c, batch))
+    assert abs(triples.t_energy_fp64(w) - full) <= 1e-13 * abs(full)
+
+
+def test_scratch_limit(cuda, monkeypatch):
+    """The scratch of an E(T) stays within T3_WORK_LIMIT where all residues (58 MB) do not fit."""
+    from pycc_gb300 import triples
+    w = wave_function(8, 40, cuda)
+    full = triples.t_energy_fp64(w)
+    monkeypatch.setattr(triples, "T3_WORK_LIMIT", 32 << 20)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    assert abs(triples.t_energy_fp64(w) - full) <= 1e-13 * abs(full)
+    assert torch.cuda.max_memory_allocated() - before <= (32 << 20) + (2 << 20)
