@@ -152,7 +152,7 @@ def contract_f64(subscripts, a, b, out=None, alpha=1.0, beta=0.0, stream=None):
     if out is None:
         out = torch.empty(call.shape, dtype=torch.float64, device=a.device)
         beta = 0.0
-    work = _rns_scratch(*call.mnk, out.device, stream) if call.rns and out.is_cuda else None
+    work = _rns_scratch(*call.mnk, out.device, stream) if call.rns else None
     st = _lib.stream_handle(stream)
     pa, pb, pc = a.data_ptr(), b.data_ptr(), out.data_ptr()
     for oa, ob, oc in call.batch:
@@ -217,7 +217,9 @@ def _takes_rns(m, n, k):
 
 def _rns_scratch(m, n, k, device, stream):
     """Scratch for the call on ``device``, owned by the launching stream, or None when the
-    device has no room even for small panels (the FP64 kernel needs none)."""
+    device has no room even for small panels (the FP64 kernel needs none) or is not a GPU."""
+    if device.type != "cuda":
+        return None
     limit = RNS_WORK_LIMIT
     while limit >= 256 << 20:
         nbytes = _rns_work(m, n, k, limit)

@@ -38,7 +38,7 @@ T2P, OB = 0, 1
 class TriplesTC:
     """Packed (T) operands for one set of amplitudes, and the batched driver."""
 
-    pitch = None      # elements between the partials' rows (None: nv)
+    pitch = None      # elements between the partials' rows; None: nv, and the unpitched kernels
 
     def __init__(self, w, t1, t2, batch=32):
         self.w = w
@@ -141,7 +141,7 @@ class TriplesTC:
             chunk = trips[b0:b0 + nb]
             gemm = (4, a_ptr, a_rows, a_ld, 2, b_ptr, b_rows, b_ld,
                     gall.data_ptr() + 3 * b0 * gsz, 3 * len(chunk), nv * nv, nv, P.data_ptr())
-            if P.is_cuda:
+            if self.pitch:
                 _lib.call("pcg_tc_grouped_gemm_pitched", *gemm, nv, pitch, nv * pitch,
                           self.status.data_ptr(), st)
                 _lib.call("pcg_triples_energy_pitched", P.data_ptr(), pitch,

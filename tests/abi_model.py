@@ -65,6 +65,12 @@ class ABIModel:
         res = alpha * prod if beta == 0.0 else beta * Cv + alpha * prod
         Cv[...] = res
 
+    def contract_rns_f64(self, *args):
+        """The same contraction; ``work`` and its length come before the stream."""
+        work, length, st = args[-3:]
+        assert work and length > 0
+        self.contract_f64(*args[:-3], st)
+
     def combine4_f64(self, ext4, a, X, xs4, b, Y, ys4, out, os4, _st):
         ext = _ints(ext4, 4)
         res = a * view(X, ext, _ints(xs4, 4))
@@ -340,6 +346,35 @@ class ABIModel:
                 acc += A @ B.T
             idx = int(rec["out"]) + m[:, None] * ldm + n[None, :] * ldn
             flat(Cp, int(idx.max()) + 1, np.float32)[idx] = acc.astype(np.float32)
+
+    def tc_grouped_gemm_pitched(self, na, a_ptr, a_rows, a_ld, nb, b_ptr, b_rows, b_ld, groups,
+                                ngroups, M, N, Cp, inner, outer, ldn, _status, _st):
+        """Row m of a group at (m / inner) * outer + m % inner."""
+        assert M % inner == 0 and outer >= inner
+        tmp = np.zeros((ngroups, N, M), dtype=np.float32)
+        from pycc_gb300.triples_tc import GROUP_DTYPE
+        g = np.frombuffer((C.c_char * (ngroups * GROUP_DTYPE.itemsize)).from_address(groups),
+                          dtype=GROUP_DTYPE).copy()
+        outs = g["out"].copy()
+        g["out"] = np.arange(ngroups) * N * M
+        self.tc_grouped_gemm(na, a_ptr, a_rows, a_ld, nb, b_ptr, b_rows, b_ld, g.ctypes.data,
+                             ngroups, M, N, tmp.ctypes.data, 1, M, _status, _st)
+        for o, block in zip(outs, tmp):
+            view(Cp + 4 * int(o), (N, M // inner, inner), (ldn, outer, 1), np.float32)[...] = \
+                block.reshape(N, M // inner, inner)
+
+    def triples_energy_pitched(self, P, pitch, ijk, ntrip, eps, eoovv, t1, t2, fov, no, nv, part,
+                               _status, _st):
+        assert pitch >= nv and pitch % 4 == 0
+        rows = lambda p, lead: np.ascontiguousarray(
+            view(p, (lead, nv, nv), (nv * pitch, pitch, 1), np.float32))
+        dense = np.ascontiguousarray(
+            view(P, (ntrip, 3, nv, nv, nv),
+                 (3 * nv * nv * pitch, nv * nv * pitch, nv * pitch, pitch, 1), np.float32))
+        e, t = rows(eoovv, no * no), rows(t2, no * no)
+        self.triples_energy(1, dense.ctypes.data, dense.ctypes.data + 4 * nv ** 3,
+                            dense.ctypes.data + 8 * nv ** 3, 3 * nv ** 3, ijk, ntrip, eps,
+                            e.ctypes.data, t1, t.ctypes.data, fov, no, nv, part, _st)
 
     def triples_energy(self, fp32, P1, P2, P3, pstride, ijk, ntrip, eps, eoovv, t1, t2, fov,
                        no, nv, part, _st):
