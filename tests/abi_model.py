@@ -65,11 +65,12 @@ class ABIModel:
         res = alpha * prod if beta == 0.0 else beta * Cv + alpha * prod
         Cv[...] = res
 
-    def contract_rns_f64(self, *args):
-        """The same contraction; ``work`` and its length come before the stream."""
-        work, length, st = args[-3:]
+    def contract_rns_f64(self, m_n, m_ext, m_sa, m_sc, n_n, n_ext, n_sb, n_sc, k_n, k_ext, k_sa,
+                         k_sb, alpha, A, B, beta, Cp, work, length, _st):
+        """The same contraction with scratch."""
         assert work and length > 0
-        self.contract_f64(*args[:-3], st)
+        self.contract_f64(m_n, m_ext, m_sa, m_sc, n_n, n_ext, n_sb, n_sc, k_n, k_ext, k_sa, k_sb,
+                          alpha, A, B, beta, Cp, _st)
 
     def combine4_f64(self, ext4, a, X, xs4, b, Y, ys4, out, os4, _st):
         ext = _ints(ext4, 4)
