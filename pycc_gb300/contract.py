@@ -111,8 +111,8 @@ def _check(t, name):
 
 class _Call:
     """The launch arguments of one contraction that its labels, extents and strides fix: the
-    sub-index groups as C arrays, the offsets of its batch indices, the output shape and whether
-    it goes to the residue path."""
+    sub-index groups as C arrays, the extents and strides of its batch indices, the output shape and
+    whether it goes to the residue path."""
 
     def __init__(self, subscripts, a, b, out):
         plan = ContractPlan(subscripts, a, b)
@@ -127,9 +127,15 @@ class _Call:
         self.mnk = tuple(math.prod([g[0] for g in G]) for G in (M, N, K))
         self.rns = _takes_rns(*self.mnk)
         # batch indices (present in both operands and the output): one launch per value
-        self.batch = [tuple(8 * sum(v * st[c] for v, c in zip(vals, batch))
-                            for st in (ast, bst, cst))
-                      for vals in itertools.product(*[range(plan.ext[c]) for c in batch])]
+        self.batch = [plan.ext[c] for c in batch]
+        self.steps = [[8 * st[c] for c in batch] for st in (ast, bst, cst)]
+
+    def offsets(self):
+        """Byte offsets of the operands and the output at every value of the batch indices."""
+        if not self.batch:
+            return ((0, 0, 0),)
+        return (tuple([sum(v * s for v, s in zip(vals, step)) for step in self.steps])
+                for vals in itertools.product(*[range(n) for n in self.batch]))
 
 
 _CALLS = {}
@@ -155,7 +161,7 @@ def contract_f64(subscripts, a, b, out=None, alpha=1.0, beta=0.0, stream=None):
     work = _rns_scratch(*call.mnk, out.device, stream) if call.rns else None
     st = _lib.stream_handle(stream)
     pa, pb, pc = a.data_ptr(), b.data_ptr(), out.data_ptr()
-    for oa, ob, oc in call.batch:
+    for oa, ob, oc in call.offsets():
         _launch_groups(call.groups, alpha, pa + oa, pb + ob, beta, pc + oc, st, work)
     return out
 

@@ -122,3 +122,19 @@ def test_random_contractions_through_the_entry_point_model(monkeypatch):
         contract_f64(subs, A, B, out=out, alpha=1.5, beta=0.5)
         assert np.allclose(out.numpy(), want, rtol=1e-12, atol=1e-12), subs
         ran += 1
+
+
+def test_a_large_batch_is_not_kept():
+    """The launch arguments that are kept between calls hold no entry per batch value."""
+    import tracemalloc
+    import torch
+    from pycc_gb300 import contract
+    a = torch.empty(1, dtype=torch.float64).expand(400, 500, 3)
+    tracemalloc.start()
+    call = contract._Call("xyk,xyk->xy", a, a, None)
+    kept = tracemalloc.get_traced_memory()[0]
+    tracemalloc.stop()
+    assert kept < 100_000
+    it = call.offsets()
+    assert [next(it) for _ in range(2)] == [(0, 0, 0), (0, 0, 8)]
+    assert sum(1 for _ in it) == 400 * 500 - 2
