@@ -16,6 +16,7 @@ Packed operands of static tensors (the integral blocks) are cached by the caller
 from __future__ import annotations
 
 import math
+import operator
 
 import torch
 
@@ -87,13 +88,19 @@ class Operand:
 
     def geometry(self):
         """What fixes this operand's gather besides its data: labels, extents and strides."""
-        if self._geometry is None:
-            self._geometry = tuple([None if s is None else (s[1], s[0].shape, s[0].stride())
-                                    for s in self.sources()])
-        return self._geometry
+        src = self.sources()
+        if self._geometry is None or any(map(operator.is_not, src, self._geometry[0])):
+            self._geometry = src, tuple([None if s is None else
+                                         (_key(s[1]), s[0].shape, s[0].stride()) for s in src])
+        return self._geometry[1]
 
     def device(self):
         return next(s for s in self.sources() if s is not None)[0].device
+
+
+def _key(labels):
+    """Labels, a string or a sequence of them, as part of a dictionary key."""
+    return labels if type(labels) is str else tuple(labels)
 
 
 def _merge_multi(groups):
@@ -219,7 +226,7 @@ _MAP_PLANS = {}
 
 def _output_map(out, row_labels, col_labels, out_labels, with_cols):
     """The output's row and column sub-indices as the library takes them."""
-    key = (out.shape, out.stride(), tuple(row_labels), tuple(col_labels), out_labels, with_cols)
+    key = (out.shape, out.stride(), tuple(row_labels), tuple(col_labels), _key(out_labels), with_cols)
     got = _MAP_PLANS.get(key)
     if got is None:
         ost = dict(zip(out_labels, out.stride()))
@@ -257,7 +264,7 @@ _CONTRACT_PLANS = {}
 def _contract_plan(subscripts, A, B, out):
     """(swap, rows, columns, K labels) of one contraction: which operand takes the 128-row tile
     side and in which order its indices run."""
-    key = (subscripts, A.labels, B.labels, A.geometry(), B.geometry(), A.key is None, out.shape,
+    key = (subscripts, _key(A.labels), _key(B.labels), A.geometry(), B.geometry(), A.key is None, out.shape,
            out.stride())
     got = _CONTRACT_PLANS.get(key)
     if got is not None:

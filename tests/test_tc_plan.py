@@ -244,3 +244,30 @@ def test_random_contractions_through_the_entry_point_model(monkeypatch):
         eng.contract(subs, A, B, out, alpha=2.0, beta=0.25, fmt=random.choice(fmts))
         assert np.allclose(out.numpy(), want, rtol=1e-11, atol=1e-11), subs
         ran += 1
+
+
+def test_labels_in_lists_and_exchanged_sources(monkeypatch):
+    """Labels may be sequences, and an operand whose source is replaced is gathered anew."""
+    import abi_model
+    abi_model.install(monkeypatch)
+    gen = torch.Generator().manual_seed(3)
+    rand = lambda *s: torch.randn(s, dtype=torch.float64, generator=gen)
+    a, b, wide = rand(5, 6), rand(4, 6), rand(9, 6)
+    status = torch.zeros(4, dtype=torch.int32)
+    B = tc.pack(Operand("ck", (b, "ck")), ["c"], ["k"], FMT_BF16)
+    for labels in (["r", "k"], ("r", "k"), "rk"):
+        for out_labels in (["r", "c"], ("r", "c"), "rc"):
+            out = torch.zeros(5, 4, dtype=torch.float64)
+            A = tc.pack(Operand(labels, (a, labels)), ["r"], ["k"], FMT_BF16)
+            tc.gemm(FMT_BF16, A, B, out, ["r"], ["c"], out_labels, status=status)
+            assert torch.allclose(out, a @ b.t(), rtol=1e-13)
+    op = Operand("rk", (a, "rk"))
+    tc.pack(op, ["r"], ["k"], FMT_BF16)
+    op.X = (wide.t()[:, ::2].t(), "rk")          # other rows, other strides
+    A = tc.pack(op, ["r"], ["k"], FMT_BF16)
+    out = torch.zeros(5, 4, dtype=torch.float64)
+    tc.gemm(FMT_BF16, A, B, out, ["r"], ["c"], "rc", status=status)
+    assert torch.allclose(out, wide[::2] @ b.t(), rtol=1e-13)
+    with pytest.raises(ValueError):
+        TCEngine.contract(TCEngine.__new__(TCEngine), "rk,ck->rc", Operand(["r", "k"], (a, "rk")),
+                          Operand("ck", (b, "ck")), out)
