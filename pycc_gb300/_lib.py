@@ -119,12 +119,12 @@ def exported_symbols():
 
 @functools.lru_cache(maxsize=8192)
 def _i64_array(vals):
-    return (C.c_longlong * max(1, len(vals)))(*[int(x) for x in vals])
+    return (C.c_longlong * max(1, len(vals)))(*vals)
 
 
 def i64s(vals):
     """A C array of long long for the library to read (shared between equal calls)."""
-    return _i64_array(tuple(vals))
+    return _i64_array(tuple([int(x) for x in vals]))
 
 
 def call(name, *args):

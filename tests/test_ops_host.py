@@ -22,3 +22,17 @@ def test_cpu_tensors_are_refused():
         torch.ops.gbcc.tau(t1, t2, 1.0, 1.0)
     with pytest.raises(NotImplementedError):
         torch.ops.gbcc.contract("ij,jk->ik", t1.T.contiguous(), t1)
+
+
+def test_integer_arrays_hold_values():
+    """Arrays handed to the library follow the values given, not the objects that hold them."""
+    import numpy as np
+    from pycc_gb300 import _lib
+    n = torch.tensor(3)
+    assert list(_lib.i64s([n, 5])) == [3, 5]
+    n += 4
+    assert list(_lib.i64s([n, 5])) == [7, 5]
+    m = np.array([2, 3])
+    assert list(_lib.i64s(m)) == [2, 3]
+    m[0] = 9
+    assert list(_lib.i64s(m)) == [9, 3]
