@@ -80,8 +80,8 @@ inline long long sub_total(const SubIdx& d) {
 }
 
 // Whether an output's row and column sub-indices (extents and strides) cover one contiguous run
-// of elements from its base pointer on.
-inline bool dense_output(int mn, const long long* me, const long long* ms, int nn,
+// of `total` elements from its base pointer on.
+inline bool dense_output(long long total, int mn, const long long* me, const long long* ms, int nn,
                          const long long* ne, const long long* ns) {
   long long e[2 * kMaxSub], s[2 * kMaxSub];
   int k = 0;
@@ -98,7 +98,7 @@ inline bool dense_output(int mn, const long long* me, const long long* ms, int n
     run *= e[at];
     e[at] = 0;
   }
-  return true;
+  return run == total;
 }
 
 // Status word for device-side bounded waits (0 = fine).

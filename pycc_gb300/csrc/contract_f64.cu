@@ -366,7 +366,7 @@ void sort_by_operand_stride(SubIdx& d) {
 int scale_output(const F64Args& p, const SubIdx& m, const SubIdx& n, long long M, long long N,
                  double beta, cudaStream_t st) {
   if (beta == 1.0) return 0;
-  if (beta == 0.0 && dense_output(m.n, m.ext, m.s1, n.n, n.ext, n.s1)) {
+  if (beta == 0.0 && dense_output(M * N, m.n, m.ext, m.s1, n.n, n.ext, n.s1)) {
     if (cudaMemsetAsync(p.C, 0, (size_t)(8 * M * N), st) == cudaSuccess) return 0;
     set_error("pcg_contract_f64: clearing the output failed");
     return -2;

@@ -1313,8 +1313,8 @@ extern "C" int pcg_tc_gemm(int fmt, const void* A_hi, const void* A_mid, const v
   // (the short-K terms are bound by that wait)
   a.red_out = (splits == 1 && nkb <= a.kb_chunk) ? 1 : 0;
   cudaStream_t st = (cudaStream_t)stream;
-  if (a.atomic_out && beta == 0.0 &&
-      dense_output(a.em.n, a.em.ext, a.em.s, a.en.n, a.en.ext, a.en.s) && !col_map) {
+  if (a.atomic_out && beta == 0.0 && !col_map &&
+      dense_output(M * N, a.em.n, a.em.ext, a.em.s, a.en.n, a.en.ext, a.en.s)) {
     if (cudaMemsetAsync(C, 0, (size_t)(8 * M * N), st) != cudaSuccess) {
       set_error("pcg_tc_gemm: clearing the output failed");
       return -2;
