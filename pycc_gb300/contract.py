@@ -187,7 +187,9 @@ def _launch(M, N, K, alpha, pa, pb, beta, pc, st, work=None):
     _launch_groups(_group_args(M, N, K), alpha, pa, pb, beta, pc, st, work)
 
 
-RNS_WORK_LIMIT = 8 << 30     # bytes of scratch of one contraction in residue arithmetic
+# Bytes of scratch of one contraction in residue arithmetic.  8.5 GiB hold 12000 x 12000 x 12000
+# (no = 40, nv = 300) in two panels of rows: 38.6 ms, in four panels (8 GiB) 44.2.
+RNS_WORK_LIMIT = 17 << 29
 
 
 @functools.lru_cache(maxsize=4096)
@@ -206,10 +208,11 @@ def _takes_rns(m, n, k):
     FP64 pipe: 6 us and 1.05 TFLOP/s.  Residues: 42 us of launches, 50 bytes moved per operand
     element at 5 TB/s, 0.3 ns per step of K (a row's norm), 17 BF16 products over whole 128 x 16 x
     64 tiles at 1.1 PFLOP/s and at least 2.5 us for 128 x 256 of them on an SM, and 13 ps per
-    output to rebuild it.  Measured on both sides of the line (us, FP64 pipe / residues): 2809 x 81
-    x 81 48 / 46, 53 x 53 x 4293 42 / 44, 60 x 60 x 8640 73 / 53, 110 x 21560 x 14 88 / 92, 11 x
-    75779 x 83 146 / 183, 14 x 169400 x 110 567 / 387, 20 x 20 x 648000 482 / 676, 180 x 72000 x
-    20 511 / 356, 477 x 477 x 477 205 / 52."""
+    output to rebuild it.  Measured (us, FP64 pipe / residues), where the rule takes the FP64 pipe:
+    53 x 53 x 4293 42 / 47, 110 x 21560 x 14 92 / 102, 11 x 75779 x 83 146 / 221, 20 x 20 x 648000
+    556 / 713, and on the wrong side by up to 1.4 2809 x 81 x 81 52 / 44, 128 x 128 x 1024 58 / 41;
+    where it takes the residues: 60 x 60 x 8640 76 / 56, 14 x 169400 x 110 486 / 458, 180 x 72000 x
+    20 518 / 393, 477 x 477 x 477 206 / 44."""
     if min(m, n) < 2 or m * n * k < 1 << 22:
         return False
     up = lambda x, t: -(-x // t) * t
