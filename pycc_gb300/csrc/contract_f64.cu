@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(256) contract_dot_kernel(const F64Args p, int 
   }
 }
 
-// Outputs with a degenerate free dimension (matrix-vector shapes such as 'nf,mnef->me', and
+// Outputs with a degenerate or short free dimension (matrix-vector shapes such as 'nf,mnef->me', and
 // full dot products): kw warps of a block share an output and a K slice (blockIdx.y), a lane holds
 // four products in flight and (I) 32-bit index arithmetic where the totals allow it.  With one
 // warp per output the index divisions of K / 32 products were a serial chain.  us: 'ijab,jb->ia'
@@ -503,6 +503,14 @@ F64Plan f64_plan(const F64Args& p, bool wide) {
   return e.q;
 }
 
+// Blocks of contract_gemv_kernel, and the warps kw that share an output: more while its 128-wide
+// steps of K suffice and fewer than `want` warps run.
+long long gemv_blocks(long long outputs, long long K, long long want, int& kw) {
+  const long long steps = (K + 127) / 128;
+  for (kw = 1; kw < 8 && 2 * kw <= steps && outputs * kw < want;) kw *= 2;
+  return std::min((outputs * kw + 7) / 8, 64LL * num_sms());
+}
+
 // the two operands exchanged
 F64Args swapped(F64Args p) {
   std::swap(p.m, p.n);
@@ -557,8 +565,7 @@ extern "C" int pcg_contract_f64(int m_n, const long long* m_ext, const long long
       if (blocks < want && p.K >= 128) splits = std::min((want + blocks - 1) / blocks, p.K / 64);
     } else {
       const long long steps = (p.K + 127) / 128, want = 20LL * num_sms();
-      while (kw < 8 && 2 * kw <= steps && p.N * kw < want) kw *= 2;
-      blocks = std::min((p.N * kw + 7) / 8, 64LL * num_sms());
+      blocks = gemv_blocks(p.N, p.K, want, kw);
       if (kw == 8) splits = std::min(want / 8 / blocks, steps / 8);
     }
     splits = std::max(1LL, std::min(splits, 65535LL));
@@ -577,6 +584,29 @@ extern "C" int pcg_contract_f64(int m_n, const long long* m_ext, const long long
     return 0;
   }
   if (p.M < p.N) p = swapped(p);
+  // A side below eight, and few outputs or rows of K contiguous in both operands: an output per
+  // warp, or per up to eight, without staged offsets or tiles.  A long K is cut over up to eight
+  // blocks where the outputs alone leave SMs idle.  us in a graph, here / by the kernels below: 5 x
+  // 2 x 52 3.4 / 6.5, 322 x 7 x 111 3.8 / 7.8, 1024 x 7 x 1000 21 / 25, 40 x 2 x 4000 6 / 12; but
+  // 4096 x 2 x 111 10.0 / 8.0 and, with K not contiguous, 1024 x 7 x 4000 128 / 75.
+  const bool k_rows = p.k.s0[p.k.n - 1] == 1 && p.k.s1[p.k.n - 1] == 1;
+  const long long outputs = p.M * p.N;
+  if (p.N < 8 && !wide &&
+      ((outputs <= 4096 && p.K <= 8192) ||
+       (k_rows && p.K >= 256 && (p.K <= 8192 || outputs >= 48)))) {
+    const long long want = (p.K >= 2048 ? 20LL : 8LL) * num_sms();
+    int kw = 1;
+    const long long blocks = gemv_blocks(outputs, p.K, want, kw);
+    const long long splits =
+        p.K > 8192 ? std::max(1LL, std::min({want / 8 / blocks, p.K / 4096, 8LL})) : 1;
+    p.k_per_split = (p.K + splits - 1) / splits;
+    p.atomic_out = splits > 1;
+    if (p.atomic_out)
+      if (const int rc = scale_output(p, p.m, p.n, p.M, p.N, beta, st)) return rc;
+    contract_gemv_kernel<unsigned><<<dim3((unsigned)blocks, (unsigned)splits), 256, 0, st>>>(p, kw);
+    PCG_CHECK_LAUNCH("pcg_contract_f64/gemv");
+    return 0;
+  }
   const F64Plan q = f64_plan(p, wide);
   if (q.swap) p = swapped(p);
   if (q.blocks > 0x7fffffffLL) {

@@ -55,3 +55,29 @@ def test_orders(cuda, m, n, k, order):
     want = 2 * (A @ B) - C
     tol = 2.0 ** -53 * ((k + 40) * 2 * (abs(A) @ abs(B)) + 4 * abs(C))
     assert (abs(got.t().cpu().numpy() - want) <= tol).all()
+
+
+@pytest.mark.parametrize("m,n,k", [(585, 7, 13), (586, 7, 13), (1365, 3, 255), (2049, 2, 256),
+                                   (300, 2, 8192), (24, 2, 8193), (23, 2, 8193), (50, 7, 20001),
+                                   (2, 2, 129), (7, 7, 1)])
+@pytest.mark.parametrize("order", ["mk,nk", "km,kn"])
+@pytest.mark.parametrize("beta", [0.0, 0.5])
+def test_short_sides(cuda, m, n, k, order, beta):
+    """A side below eight, on both sides of the line between an output per warp and tiles."""
+    gen = torch.Generator(device=cuda).manual_seed(m + n + k)
+    la, lb = order.split(",")
+    ext = {"m": m, "n": n, "k": k}
+    a, b = (torch.randn(ext[x[0]], ext[x[1]], dtype=torch.float64, device=cuda, generator=gen)
+            for x in (la, lb))
+    c = torch.randn(m, n, dtype=torch.float64, device=cuda, generator=gen)
+    got = c.clone() if beta else torch.full_like(c, float("nan"))
+    st = lambda t, lab, x: t.stride(lab.index(x))
+    contract._launch([(m, st(a, la, "m"), n)], [(n, st(b, lb, "n"), 1)],
+                     [(k, st(a, la, "k"), st(b, lb, "k"))], -1.5, a.data_ptr(), b.data_ptr(), beta,
+                     got.data_ptr(), _lib.stream_handle())
+    A = (a if la == "mk" else a.t()).cpu().numpy().astype(np.longdouble)
+    B = (b.t() if lb == "nk" else b).cpu().numpy().astype(np.longdouble)
+    C = c.cpu().numpy()
+    want = beta * C - 1.5 * (A @ B)
+    tol = 2.0 ** -53 * ((k + 40) * 1.5 * (abs(A) @ abs(B)) + 4 * abs(C))
+    assert (abs(got.cpu().numpy() - want) <= tol).all()
