@@ -215,8 +215,8 @@ int pcg_triples_energy(int fp32, const void* P1, const void* P2, const void* P3,
                        const double* fov, long long no, long long nv, double* part,
                        void* stream);
 /* pcg_triples_energy(fp32 = 1) for partials P[ntrip][3][nv][nv][pitch] and eoovv, t2 of
- * [no][no][nv][pitch], the pitch a multiple of four floats (16-byte aligned bases): tiles by TMA.  An expired device-side wait sets
- * *status (device int) and makes its partial NaN. */
+ * [no][no][nv][pitch], the pitch a multiple of four floats (16-byte aligned bases): tiles by TMA.
+ * An expired device-side wait sets *status (device int) and makes its partial NaN. */
 int pcg_triples_energy_pitched(const float* P, long long pitch, const int* ijk, int ntrip,
                                const double* eps, const float* eoovv, const double* t1,
                                const float* t2, const double* fov, long long no, long long nv,

@@ -17,18 +17,18 @@
 //    reduce every chunk modulo p and keep the running residue in registers.
 //    A seventeenth GEMM, of the integers' magnitudes in BF16, gives sum |a'||b'|, 2 % low at most.
 // 4. The integer sum is at most |a'_i| |b'_j| (Cauchy-Schwarz), below half the product of the
-//    moduli (2^125.4), so the residues determine it exactly.  It is rebuilt as a 96-bit
+//    moduli (2^123.95), so the residues determine it exactly.  It is rebuilt as a 96-bit
 //    fraction of that product, rounded to FP64, scaled back and added into C.
 //
-// Where large entries of a row meet small or zero ones of a column, the rounding of step 1 can
-// be as large as the sum.  Step 4 sees this from the sum of magnitudes (kDoubt in rns.cuh) and takes
-// such outputs from FP64 dot products, so every output's error is bounded in terms of sum |a||b|, as
-// that of FP64 multiply-adds.  So are the outputs of a row (or a column of B) with an infinity or a
-// NaN, and non-finite inputs give what FP64 arithmetic gives.
+// Where large entries of a row meet small or zero ones of a column, the rounding of step 1 can be
+// as large as the sum.  Step 4 sees this from the sum of magnitudes (kDoubt in rns.cuh) and takes
+// such outputs from FP64 dot products, so every output's error is bounded in terms of sum |a||b|,
+// as that of FP64 multiply-adds.  So are the outputs of a row (or a column of B) with an infinity
+// or a NaN, and non-finite inputs give what FP64 arithmetic gives.
 //
 // Measured on GB300 against the FP64 pipe at its peak rate, no = 20, nv = 180: the ladder
-// 'ijef,abef->ijab' 727 -> 21.9 ms (GEMM 12.8, packs 7.7), a ring 'imae,mbej->ijab' 81 -> 1.40 ms; at
-// no = 9, nv = 53 2.2 -> 0.16 ms for the ladder.
+// 'ijef,abef->ijab' 727 -> 21.9 ms (GEMM 12.8, packs 7.7), a ring 'imae,mbej->ijab' 81 -> 1.40 ms;
+// at no = 9, nv = 53 2.2 -> 0.16 ms for the ladder.
 //
 // The offsets of strided rows, columns and K indices are expanded into tables once per call;
 // operands larger than the workspace go through in panels of rows, columns or K.
@@ -55,8 +55,8 @@ struct JoinArgs {
 
 // This lane's part of the FP64 dot product of one output: K indices k0, k0 + step, ..., four in
 // flight.  A warp leaves when its sum is a NaN, which nothing changes any more.
-__device__ __forceinline__ double lane_dot(const JoinArgs& p, long long row, long long col, int part,
-                                           int step) {
+__device__ __forceinline__ double lane_dot(const JoinArgs& p, long long row, long long col,
+                                           int part, int step) {
   const int lane = threadIdx.x & 31;
   const double* x = p.a.X + p.a.off[row];
   const double* y = p.b.X + p.b.off[col];
@@ -157,12 +157,12 @@ __device__ __forceinline__ double item_sum(const JoinArgs& p, unsigned row, unsi
 }
 
 // The outputs of this block's items i0, i0 + 1, ... that their threads marked (bit e of `doubt`:
-// column e).  A few: a warp each with the lanes along K, or, along a long K, all eight warps.  That
-// takes up to four times an FP64 kernel's time for an output, so from a third of the block's outputs
-// on an item's four columns are computed together, by a thread or, where B is contiguous along K,
-// by a warp.  The whole call, with no output, one output of each row and every output marked: 1600 x
-// 1600 x 1600 0.20, 0.30 and 7.4 ms (FP64 kernel 6.7), 477 x 477 x 477 42, 46 and 274 us (201),
-// 53 x 53 x 4293 53, 57 and 89 us (36).
+// column e).  A few: a warp each with the lanes along K, or, along a long K, all eight warps.
+// That takes up to four times an FP64 kernel's time for an output, so from a third of the block's
+// outputs on an item's four columns are computed together, by a thread or, where B is contiguous
+// along K, by a warp.  The whole call, with no output, one output of each row and every output
+// marked: 1600 x 1600 x 1600 0.20, 0.30 and 7.4 ms (FP64 kernel 6.7), 477 x 477 x 477 42, 46 and
+// 274 us (201), 53 x 53 x 4293 53, 57 and 89 us (36).
 __device__ __noinline__ void redo_marked(const JoinArgs& p, Redo& s, unsigned i0, unsigned nc,
                                          unsigned doubt) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -225,11 +225,11 @@ __device__ __noinline__ void redo_marked(const JoinArgs& p, Redo& s, unsigned i0
 }
 
 // Four columns of one row per thread: for every modulus the residues times the three words of
-// floor(2^96 q / p) are summed in 64-bit accumulators (their integer part falls out modulo
-// 2^96), the signed fraction is rounded to FP64 and scaled.  About 200 integer instructions and
-// two FP64 ones per output; four resident blocks hide the loads' latency.  At 13.0e6 outputs
-// 134 us, against 175 at 66 registers with each column's scale computed where it is read; on another
-// day 121, and 131 with the sums of magnitudes, a seventeenth byte per output, and their check.
+// floor(2^96 q / p) are summed in 64-bit accumulators (their integer part falls out modulo 2^96),
+// the signed fraction is rounded to FP64 and scaled.  About 200 integer instructions and two FP64
+// ones per output; four resident blocks hide the loads' latency.  At 13.0e6 outputs 134 us,
+// against 175 at 66 registers with each column's scale computed where it is read; on another day
+// 121, and 131 with the sums of magnitudes, a seventeenth byte per output, and their check.
 __global__ void __launch_bounds__(256, 4) rns_join_kernel(const __grid_constant__ JoinArgs p) {
   __shared__ Redo redo;
   const unsigned nc = (unsigned)((p.N + 3) >> 2);

@@ -22,11 +22,11 @@ constexpr int NM = 16;
 constexpr int kModuli[NM] = {256, 253, 251, 247, 241, 239, 233, 229,
                              227, 223, 217, 211, 199, 197, 193, 191};
 // Planes of a packed operand and of a product: the residues, then magnitudes.  A row is rounded to
-// integers at one power of two, so an output's error is a fixed number of units: 0.29 sqrt(|a'|^2 +
-// |b'|^2) <= 2^60.6 of them (root mean square).  Where large entries of a row meet small or zero
-// ones, that can be all of a sum of small products.  So |a'| and |b'|, truncated to BF16, go through
-// the GEMM as well and give sum |a'||b'|; an output whose sum is not zero and below kDoubt units
-// is computed again in FP64.  Elsewhere the error is at most 2^-53.4 sum |a||b| (root mean
+// integers at one power of two, so an output's error is a fixed number of units: 0.29 sqrt(|a'|^2
+// + |b'|^2) <= 2^60.6 of them (root mean square).  Where large entries of a row meet small or zero
+// ones, that can be all of a sum of small products.  So |a'| and |b'|, truncated to BF16, go
+// through the GEMM as well and give sum |a'||b'|; an output whose sum is not zero and below kDoubt
+// units is computed again in FP64.  Elsewhere the error is at most 2^-53.4 sum |a||b| (root mean
 // square) and sqrt(K) 2^-52 sum |a||b| in the worst case, against K 2^-53 for FP64 multiply-adds.
 constexpr int NP = NM + 1;
 constexpr float kDoubt = 0x1p114f;
@@ -45,7 +45,9 @@ constexpr bool moduli_hold_sums() {
 static_assert(moduli_hold_sums(), "half the product of the moduli exceeds 2^(kSumBits + 0.9)");
 // first bit of the four digits of a scaled integer (16, 15, 15 and 16 bits): with residues of
 // the powers of at most 127, a digit sum stays below 2^16 + 127 * 2^17 < 2^24, exact in FP32
-__host__ __device__ constexpr int digit_bit(int q) { return q == 0 ? 0 : (q == 4 ? 62 : 1 + 15 * q); }
+__host__ __device__ constexpr int digit_bit(int q) {
+  return q == 0 ? 0 : (q == 4 ? 62 : 1 + 15 * q);
+}
 constexpr int kChunk = 15;          // 64-K blocks per exact FP32 accumulation: 960 K
 constexpr float kMagic = 12582912.f;  // 1.5 * 2^23: adding it rounds to an integer
 
@@ -242,10 +244,10 @@ struct RowNorm {
   }
 };
 
-// Norms of the rows over K indices [k0, k1): one read of the operand, bound by HBM.  Gathered along K
-// (KF: a warp per row) or along the rows (a thread per row, or, of few rows, one per row and slice
-// of K: the eight warps of a block then share 32 rows), eight loads in flight per lane.  Block by of
-// segs has K indices [k0 + by seg, ..).
+// Norms of the rows over K indices [k0, k1): one read of the operand, bound by HBM.  Gathered
+// along K (KF: a warp per row) or along the rows (a thread per row, or, of few rows, one per row
+// and slice of K: the eight warps of a block then share 32 rows), eight loads in flight per lane.
+// Block by of segs has K indices [k0 + by seg, ..).
 template <bool KF>
 __device__ __forceinline__ void norm_rows(const Operand& o, unsigned long long* part, long long k0,
                                           long long k1, bool slices, long long seg, long long segs,
@@ -323,7 +325,8 @@ struct NormArgs {
 };
 
 // Both operands in one launch: the first blocks take A, the others B.
-static __global__ void __launch_bounds__(256, 8) rns_norm_kernel(const __grid_constant__ NormArgs p) {
+static __global__ void __launch_bounds__(256, 8)
+    rns_norm_kernel(const __grid_constant__ NormArgs p) {
   const int side = blockIdx.x >= p.blocks[0];
   const long long b = (long long)blockIdx.x - (side ? p.blocks[0] : 0);
   const long long bx = b % p.gx[side], by = b / p.gx[side];
@@ -336,8 +339,8 @@ static __global__ void __launch_bounds__(256, 8) rns_norm_kernel(const __grid_co
 
 constexpr int kNotFinite = 1 << 20;
 
-// Power of two s of a row: |x| 2^s has a 2-norm of at most 2^61.9 (and of at least 2^60.3, where its
-// entries are normal numbers).  A zero row may take any.
+// Power of two s of a row: |x| 2^s has a 2-norm of at most 2^61.9 (and of at least 2^60.3, where
+// its entries are normal numbers).  A zero row may take any.
 __device__ __forceinline__ int row_shift(const Operand& o, long long row) {
   if (o.shift) return *o.shift;
   unsigned frac;
@@ -437,11 +440,10 @@ __device__ __forceinline__ void store_residues(const PackArgs& p, const PackSide
 
 // Operand -> residues: 8 bytes read and 2 NP written per element, about 95 instructions; bound by
 // the writes.  A quarter warp takes 64 K of a row, eight neighbouring K a lane.  Gathered along K
-// it loads them straight from global memory; otherwise a tile of 64 walked rows x 64 K goes through
-// shared memory, read along the rows.  One launch packs a panel of each operand: the first blocks
-// take A's, the others B's.  163e6 elements: 1.12 ms (6.1 TB/s), 1.07
-// before the plane of magnitudes, against 1.15 with one element to an instruction and 1.20 with four
-// K a lane as well.
+// it loads them straight from global memory; otherwise a tile of 64 walked rows x 64 K goes
+// through shared memory, read along the rows.  One launch packs a panel of each operand: the first
+// blocks take A's, the others B's.  163e6 elements: 1.12 ms (6.1 TB/s), 1.07 before the plane of
+// magnitudes, against 1.15 with one element to an instruction and 1.20 with four K a lane as well.
 static __global__ void __launch_bounds__(256, 4)
     rns_pack_kernel(const __grid_constant__ PackArgs p) {
   __shared__ double tile[64][65];
@@ -522,8 +524,8 @@ struct GemmArgs {
   const int* ijk;           // [triples][3]
   int kc;                   // K blocks of a product over e and m
   int blocks_a, pairs;      // blocks of v^2 rows of an A matrix, pairs (blocks of v rows) of B
-  int c, first[3], width[3];  // of i, j, k: slots of c occupied indices from first on, width of them
-                              // present; c = 0: one slot for all of them
+  int c, first[3], width[3];  // of i, j, k: slots of c occupied indices from first on, width of
+                              // them present; c = 0: one slot for all of them
 };
 
 struct GemmMaps {
@@ -569,8 +571,8 @@ __device__ __forceinline__ T3Product t3_product(int q, int s) {
 }
 
 // Unit u -> (plane, split or group, tile): neighbouring groups share row blocks of one plane (mod:
-// a modulus, or NM for the magnitudes).  The tile order within a plane is tc_gemm_kernel's raster (groups of gm M tiles, M fastest), so a wave shares the row blocks of
-// both operands in L2.
+// a modulus, or NM for the magnitudes).  The tile order within a plane is tc_gemm_kernel's raster
+// (groups of gm M tiles, M fastest), so a wave shares the row blocks of both operands in L2.
 template <bool TRIP, bool SEGS>
 __device__ __forceinline__ Unit decode_unit(const GemmArgs& p, unsigned u) {
   // 32-bit divisions: in 64 bits the chain took longer than the MMAs of a short-K unit
@@ -1010,7 +1012,8 @@ inline int run_gemm(const GemmMaps& maps, const GemmArgs& a, cudaStream_t st) {
     return -1;
   }
   rns_gemm_kernel<BN, TRIP>
-      <<<(unsigned)std::min<long long>(units, num_sms()), kGemmThreads, smem, st>>>(maps, a, (unsigned)units);
+      <<<(unsigned)std::min<long long>(units, num_sms()), kGemmThreads, smem, st>>>(
+          maps, a, (unsigned)units);
   PCG_CHECK_LAUNCH("rns gemm");
   return 0;
 }

@@ -354,14 +354,14 @@ long long tile_triples(long long nv) {
 }
 
 // ---- FP32 path, partials with a 16-byte pitch: tiles by TMA ------------------------------
-// One block per (triple, tile triple A >= B >= C) as above, but the six orderings of the tile
-// sets of each partial arrive as 8 x 8 x 8 boxes by TMA (18 boxes of 2 KB, zeros beyond nv) and W is
+// One block per (triple, tile triple A >= B >= C) as above, but the six orderings of the tile sets
+// of each partial arrive as 8 x 8 x 8 boxes by TMA (18 boxes of 2 KB, zeros beyond nv) and W is
 // summed where it is used.  The 8 x 8 blocks of integrals and amplitudes are the threads' own
 // loads: 36 more small copies by TMA, which takes 2.6 clocks for a 32-byte row, made the kernel
-// 15 % slower.  The staging of the kernel above cost about 500 instructions a thread and, at a
-// pitch that is no multiple of 32 bytes, two sectors for each 32-byte run; what bounds this one is shared-memory reads, so a warp takes 2 x 4 x 4 elements (a, b, c), which keeps the
-// boxes' 256-byte slices at two to four reads to a bank.
-// At nv = 121, 32 triples: 260 us against 400.
+// 15 % slower.  The staging of the kernel above cost about 500 instructions a thread and, at a pitch
+// that is no multiple of 32 bytes, two sectors for each 32-byte run; what bounds this one is
+// shared-memory reads, so a warp takes 2 x 4 x 4 elements (a, b, c), which keeps the boxes'
+// 256-byte slices at two to four reads to a bank.  At nv = 121, 32 triples: 260 us against 400.
 struct CubeArgs {
   const int* ijk;      // [ntrip][3]
   const double* eps;   // [nmo]
@@ -378,7 +378,9 @@ struct CubeArgs {
 
 // ordered pairs of the tile sets A, B, C (0, 1, 2): AB, AC, BA, BC, CA, CB
 __host__ __device__ constexpr int pair_first(int q) { return q >> 1; }
-__host__ __device__ constexpr int pair_second(int q) { return (q >> 1) == 0 ? 1 + (q & 1) : ((q & 1) ? 3 - (q >> 1) : 0); }
+__host__ __device__ constexpr int pair_second(int q) {
+  return (q >> 1) == 0 ? 1 + (q & 1) : ((q & 1) ? 3 - (q >> 1) : 0);
+}
 
 template <bool FOV>
 struct CubeStage {
@@ -463,7 +465,8 @@ __global__ void __launch_bounds__(TE2_THREADS, 4)
   }
   __syncthreads();
   if (!s.ok) {
-    if (tid == 0) p.part[(long long)t * p.ntt + blockIdx.x] = __longlong_as_double(0x7ff8000000000000ll);
+    if (tid == 0)
+      p.part[(long long)t * p.ntt + blockIdx.x] = __longlong_as_double(0x7ff8000000000000ll);
     return;
   }
   // the TMA's writes: every thread observes the completed phase itself
@@ -471,7 +474,6 @@ __global__ void __launch_bounds__(TE2_THREADS, 4)
   const int lane = tid & 31, warp = tid >> 5;
   const int bl = ((lane >> 2) & 3) | (((warp >> 1) & 1) << 2), cl = (lane & 3) | ((warp >> 2) << 2);
   const int b = org[1] + bl, c = org[2] + cl;
-  // of (b, c), shared by the thread's elements: <..|bc>, <..|cb>, t1, f and their products
   float acc = 0.f;
   const float eo = f64_to_f32(p.eps[i] + p.eps[j] + p.eps[k]);
   auto lin = [](int o, int la, int lb, int lc) {  // place of (la, lb, lc) in a box of ordering o
@@ -593,8 +595,9 @@ extern "C" int pcg_triples_energy(int fp32, const void* P1, const void* P2, cons
 }
 
 // The FP32 path with the partials P[triple][orientation][nv][nv][pitch] and eoovv, t2 of
-// [o][o][nv][pitch], pitch a multiple of four floats (16 bytes): the partials' tiles come by TMA.  *status: a device word that an expired wait sets (the
-// partial is NaN then).  Partials as pcg_triples_energy(fp32 = 1) writes them.
+// [o][o][nv][pitch], pitch a multiple of four floats (16 bytes): the partials' tiles come by TMA.
+// *status: a device word that an expired wait sets (the partial is NaN then).  Partials as
+// pcg_triples_energy(fp32 = 1) writes them.
 extern "C" int pcg_triples_energy_pitched(const float* P, long long pitch, const int* ijk, int ntrip,
                                           const double* eps, const float* eoovv, const double* t1,
                                           const float* t2, const double* fov, long long no,

@@ -34,8 +34,8 @@ struct T3MaxArgs {
   const unsigned long long* norm[2];
   long long R[2];
   int which[2];   // entry of `out`
-  unsigned* out;  // [4] largest log2 of a squared row norm, rounded up, + kT3Bias (0: no row is above
-                  // zero); [1] an Inf or a NaN
+  unsigned* out;  // [4] largest log2 of a squared row norm, rounded up, + kT3Bias (0: no row is
+                  // above zero); [1] an Inf or a NaN
 };
 constexpr int kT3Bias = 1 << 16;
 
@@ -111,7 +111,7 @@ __device__ __forceinline__ double t3_dot(const T3JoinArgs& p, int g, long long r
   return s;
 }
 
-// The partials that the lanes of a warp (rows row0, row0 + 1, ...) marked, bit e for column col + e.
+// The partials that the lanes of a warp (rows row0, row0 + 1, ...) marked: bit e, column col + e.
 __device__ __noinline__ void t3_redo(const T3JoinArgs& p, int g, long long row0, int col,
                                      unsigned doubt) {
   const long long M = (long long)p.nv * p.nv;
@@ -161,10 +161,10 @@ __global__ void __launch_bounds__(256, 5) t3_join_kernel(const __grid_constant__
 }
 
 // Workspace: status and shifts, the residues of the matrices, then each batch's products (while
-// operands are prepared, the rows' tables lie there instead).  The residues of all occupied orbitals
-// take 17 * 4 no nv^2 kc bytes (38 GB at no = 30, nv = 240), so a caller may go through the triples in
-// windows: i, j and k each in a slot of c orbitals, of which [VT | TM] holds i's and j's and
-// [VN | TMT] j's and k's.  c = no: one slot for all three.
+// operands are prepared, the rows' tables lie there instead).  The residues of all occupied
+// orbitals take 17 * 4 no nv^2 kc bytes (38 GB at no = 30, nv = 240), so a caller may go through
+// the triples in windows: i, j and k each in a slot of c orbitals, of which [VT | TM] holds i's
+// and j's and [VN | TMT] j's and k's.  c = no: one slot for all three.
 struct T3Plan {
   long long no, nv, c;
   bool windows;
@@ -301,7 +301,7 @@ int t3_scales(const T3Plan& p, const double* V, const double* O, const double* t
 // Occupied indices in the slot that starts at `first`.
 long long t3_width(const T3Plan& p, long long first) { return std::min(p.c, p.no - first); }
 
-// Residues of the slots in `changed` (bits 0, 1, 2: i, j, k) and of the pairs that one of them is in.
+// Residues of the slots in `changed` (bits 0, 1, 2: i, j, k) and of their pairs.
 int t3_pack(const T3Plan& p, const double* V, const double* O, const double* t2, const int* first,
             unsigned changed, unsigned char* w, cudaStream_t st) {
   struct Item {
@@ -342,8 +342,8 @@ int t3_pack(const T3Plan& p, const double* V, const double* O, const double* t2,
       Operand oa, ob;
       if (k.tables(a->rows, b ? &b->rows : nullptr, oa, ob)) return -2;
       auto side = [&](const Item& x, const Operand& op) {
-        return PackSide{op, 0, op.R, (__nv_bfloat16*)x.panel + x.row * p.kc + col, x.plane * p.kc / 8,
-                        x.rows.flip, 0};
+        return PackSide{op, 0, op.R, (__nv_bfloat16*)x.panel + x.row * p.kc + col,
+                        x.plane * p.kc / 8, x.rows.flip, 0};
       };
       PackArgs args{{side(*a, oa), b ? side(*b, ob) : PackSide{}}, 0, q ? o : v,
                     q ? p.kc - p.c0 : p.c0, p.kc, tables().pairs};
@@ -410,7 +410,8 @@ bool t3_batch(const int* ijk, int ntrip, const double* P, const char* who) {
 bool t3_first(const T3Plan& p, const int* first, const char* who) {
   bool ok = first != nullptr;
   for (int r = 0; ok && r < 3; ++r)
-    ok = first[r] >= 0 && first[r] < p.no && first[r] % p.c == 0 && (r == 0 || first[r] <= first[r - 1]);
+    ok = first[r] >= 0 && first[r] < p.no && first[r] % p.c == 0 &&
+         (r == 0 || first[r] <= first[r - 1]);
   if (!ok) set_error("%s: bad first indices of the window's slots", who);
   return ok;
 }
@@ -498,11 +499,11 @@ extern "C" int pcg_t3_rns_pack(const double* V, const double* O, const double* t
   return rc ? rc : t3_pack(p, V, O, t2, kNoFirst, 7, w, (cudaStream_t)stream);
 }
 
-extern "C" int pcg_t3_rns_partials_of(const double* V, const double* O, const double* t2, long long no,
-                                      long long nv, const int* ijk, int ntrip, double* P, void* work,
-                                      long long work_len, void* stream) {
-  return partials_entry("pcg_t3_rns_partials_of", V, O, t2, no, nv, no, kNoFirst, ijk, ntrip, P, work,
-                        work_len, stream);
+extern "C" int pcg_t3_rns_partials_of(const double* V, const double* O, const double* t2,
+                                      long long no, long long nv, const int* ijk, int ntrip,
+                                      double* P, void* work, long long work_len, void* stream) {
+  return partials_entry("pcg_t3_rns_partials_of", V, O, t2, no, nv, no, kNoFirst, ijk, ntrip, P,
+                        work, work_len, stream);
 }
 
 extern "C" int pcg_t3_rns_partials(long long no, long long nv, const int* ijk, int ntrip, double* P,
